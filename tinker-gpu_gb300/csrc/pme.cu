@@ -223,11 +223,51 @@ __device__ __forceinline__ bool grid_word_big(long long w, int packed)
    return a >= (1 << 30) || a <= -(1 << 30) || b >= (1 << 30) || b <= -(1 << 30);
 }
 
-// Spreading, one warp per atom: lane (jy, kz) < 25 owns one row of five x
-// points.  MODE 0 spreads fractional multipoles into the real part; MODE 1
-// spreads fractional d dipoles into the real and p dipoles into the
-// imaginary part.  rp rows are 12 floats (q, d, quadrupole, ...), u rows 8.
-// DIR (MODE 1): the dipoles are the CG search direction p = z + b p_old
+// One piece of the order-5 cardinal B-spline and its derivatives as
+// polynomials in t, for a lane that owns one of the five points along an
+// axis.  The pieces mirror each other (M5 is even about its centre), so the
+// first two are the last two at t = 1 - w with the odd derivatives' sign
+// flipped, and there is no cancellation at either end.  Coefficients x 24:
+// centre 11 + 12 t - 6 t^2 - 12 t^3 + 6 t^4, next 1 + 4 t + 6 t^2 + 4 t^3 -
+// 4 t^4, edge t^4 (the closed form of the recursion in bspline5).
+struct SplinePiece {
+   float c0, c1, c2, c3, c4;
+   bool mirror;
+   __device__ __forceinline__ explicit SplinePiece(int j)
+   {
+      mirror = j < 2;
+      const bool mid = j == 2, edge = j == 0 || j == 4;
+      constexpr float q = 1.f / 24.f;
+      c0 = mid ? 11.f * q : edge ? 0.f : q;
+      c1 = mid ? 12.f * q : edge ? 0.f : 4.f * q;
+      c2 = mid ? -6.f * q : edge ? 0.f : 6.f * q;
+      c3 = mid ? -12.f * q : edge ? 0.f : 4.f * q;
+      c4 = mid ? 6.f * q : edge ? q : -4.f * q;
+   }
+   template <int LEVEL>
+   __device__ __forceinline__ void eval(float w, float* th) const
+   {
+      const float t = mirror ? 1.f - w : w;
+      th[0] = __fmaf_rn(__fmaf_rn(__fmaf_rn(__fmaf_rn(c4, t, c3), t, c2), t, c1), t, c0);
+      if (LEVEL > 1) {
+         const float d = __fmaf_rn(__fmaf_rn(__fmaf_rn(4.f * c4, t, 3.f * c3), t, 2.f * c2), t, c1);
+         th[1] = mirror ? -d : d;
+      }
+      if (LEVEL > 2)
+         th[2] = __fmaf_rn(__fmaf_rn(12.f * c4, t, 6.f * c3), t, 2.f * c2);
+      if (LEVEL > 3) {
+         const float d = __fmaf_rn(24.f * c4, t, 6.f * c3);
+         th[3] = mirror ? -d : d;
+      }
+   }
+};
+
+// Spreading, one warp per atom: lane (ix, jy) < 25 owns one column of five z
+// points, so that each of a warp's five reductions covers five rows of five
+// consecutive words.  MODE 0 spreads fractional multipoles into the real
+// part; MODE 1 spreads fractional d dipoles into the real and p dipoles into
+// the imaginary part.  rp rows are 12 floats (q, d, quadrupole, ...), u rows
+// 8.  DIR (MODE 1): the dipoles are the CG search direction p = z + b p_old
 // (src = p_old, z8 = z, b from scal), formed as each row is read.
 template <int MODE, bool DIR = false>
 __global__ void __launch_bounds__(256) k_spread(int n, GridParams G, const float4* __restrict__ spos,
@@ -244,20 +284,20 @@ __global__ void __launch_bounds__(256) k_spread(int n, GridParams G, const float
    float w1, w2, w3;
    site(G, spos[s], i1, i2, i3, w1, w2, w3);
    constexpr int L = MODE == 0 ? 3 : 2;
-   float t1[5][L], t2[5][L], t3[5][L];
-   bspline5<L>(w1, t1);
-   bspline5<L>(w2, t2);
+   const int ix = lane % 5, jy = lane / 5;
+   float tx[L], ty[L], t3[5][L];
+   SplinePiece(ix).eval<L>(w1, tx);
+   SplinePiece(jy).eval<L>(w2, ty);
    bspline5<L>(w3, t3);
-   pdl_wait();
-   pdl_trigger();
-   const int jy = lane % 5, kz = lane / 5;
-   int zb = i3 + kz;
-   zb -= (zb >= G.n3 ? G.n3 : 0);
+   int xb = i1 + ix;
+   xb -= (xb >= G.n1 ? G.n1 : 0);
    int yb = i2 + jy;
    yb -= (yb >= G.n2 ? G.n2 : 0);
-   const size_t row = ((size_t)zb * G.n2 + yb) * G.n1;
-   const float v0 = t3[kz][0], v1 = t3[kz][1];
-   const float u0 = t2[jy][0], u1 = t2[jy][1];
+   const size_t plane = (size_t)G.n2 * G.n1;
+   unsigned long long* col = q + ((size_t)yb * G.n1 + xb);
+   pdl_wait();
+   pdl_trigger();
+   const float xy = tx[0] * ty[0], x1y = tx[1] * ty[0], xy1 = tx[0] * ty[1];
    if (MODE == 0) {
       const float* m = src + 12 * s;
       // Cartesian -> fractional (orthogonal box; quadrupole off-diagonals doubled)
@@ -265,15 +305,15 @@ __global__ void __launch_bounds__(256) k_spread(int n, GridParams G, const float
       const float fx = G.a1 * m[1], fy = G.a2 * m[2], fz = G.a3 * m[3];
       const float fxx = G.a1 * G.a1 * m[4], fyy = G.a2 * G.a2 * m[5], fzz = G.a3 * G.a3 * m[6];
       const float fxy = 2.f * G.a1 * G.a2 * m[7], fxz = 2.f * G.a1 * G.a3 * m[8], fyz = 2.f * G.a2 * G.a3 * m[9];
-      const float v2 = t3[kz][L - 1], u2 = t2[jy][L - 1];
-      const float term0 = f0 * u0 * v0 + fy * u1 * v0 + fz * u0 * v1 + fyy * u2 * v0 + fzz * u0 * v2 + fyz * u1 * v1;
-      const float term1 = fx * u0 * v0 + fxy * u1 * v0 + fxz * u0 * v1;
-      const float term2 = fxx * u0 * v0;
+      const float x2y = tx[L - 1] * ty[0], xy2 = tx[0] * ty[L - 1], x1y1 = tx[1] * ty[1];
+      const float c0 = f0 * xy + fx * x1y + fy * xy1 + fxx * x2y + fyy * xy2 + fxy * x1y1;
+      const float c1 = fz * xy + fxz * x1y + fyz * xy1;
+      const float c2 = fzz * xy;
 #pragma unroll
-      for (int ix = 0; ix < 5; ++ix) {
-         int xb = i1 + ix;
-         xb -= (xb >= G.n1 ? G.n1 : 0);
-         grid_add(q, row + xb, term0 * t1[ix][0] + term1 * t1[ix][1] + term2 * t1[ix][L - 1]);
+      for (int kz = 0; kz < 5; ++kz) {
+         int zb = i3 + kz;
+         zb -= (zb >= G.n3 ? G.n3 : 0);
+         grid_add(col, zb * plane, c0 * t3[kz][0] + c1 * t3[kz][1] + c2 * t3[kz][L - 1]);
       }
    } else {
       float u[8];
@@ -283,15 +323,13 @@ __global__ void __launch_bounds__(256) k_spread(int n, GridParams G, const float
 #pragma unroll
          for (int c = 0; c < 6; ++c)
             u[c] = src[8 * s + c];
-      const float dx = G.a1 * u[0], dy = G.a2 * u[1], dz = G.a3 * u[2];
-      const float px = G.a1 * u[3], py = G.a2 * u[4], pz = G.a3 * u[5];
-      const float d01 = dy * u1 * v0 + dz * u0 * v1, d11 = dx * u0 * v0;
-      const float p01 = py * u1 * v0 + pz * u0 * v1, p11 = px * u0 * v0;
+      const float d0 = G.a1 * u[0] * x1y + G.a2 * u[1] * xy1, d1 = G.a3 * u[2] * xy;
+      const float p0 = G.a1 * u[3] * x1y + G.a2 * u[4] * xy1, p1 = G.a3 * u[5] * xy;
 #pragma unroll
-      for (int ix = 0; ix < 5; ++ix) {
-         int xb = i1 + ix;
-         xb -= (xb >= G.n1 ? G.n1 : 0);
-         grid_add2(q, row + xb, d01 * t1[ix][0] + d11 * t1[ix][1], p01 * t1[ix][0] + p11 * t1[ix][1], G);
+      for (int kz = 0; kz < 5; ++kz) {
+         int zb = i3 + kz;
+         zb -= (zb >= G.n3 ? G.n3 : 0);
+         grid_add2(col, zb * plane, d0 * t3[kz][0] + d1 * t3[kz][1], p0 * t3[kz][0] + p1 * t3[kz][1], G);
       }
    }
 }
@@ -321,16 +359,62 @@ __global__ void k_conv(size_t ng, const float* __restrict__ infl, float2* __rest
    }
 }
 
+// Sums of N values over the 32 lanes of a warp, value k ending in the lanes
+// where sum_slot<N>(lane) == k: each step halves the values a lane carries
+// (it sends the half it does not keep), so N values take about N + 3
+// shuffles where N separate trees take 5 N.  The order of the additions is
+// fixed.  Lanes with sum_slot < 0 hold nothing.
+template <int N, int O = 16>
+__device__ __forceinline__ float warp_sums(float* v, int lane)
+{
+   constexpr int H = (N + 1) / 2;
+   const bool up = lane & O;
+   if constexpr (N > 1) {
+#pragma unroll
+      for (int k = 0; k < H; ++k) {
+         const float hi = k + H < N ? v[k + H] : 0.f;
+         const float keep = up ? hi : v[k], send = up ? v[k] : hi;
+         v[k] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+      }
+   } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+   }
+   if constexpr (O > 1)
+      return warp_sums<H, O / 2>(v, lane);
+   else
+      return v[0];
+}
+
+template <int N, int O = 16>
+__device__ __forceinline__ int sum_slot(int lane)
+{
+   if constexpr (N <= 1) {
+      return (lane & (2 * O - 1)) == 0 ? 0 : -1;  // the other lanes hold copies
+   } else {
+      constexpr int H = (N + 1) / 2;
+      const bool up = lane & O;
+      int r;
+      if constexpr (O > 1)
+         r = sum_slot<H, O / 2>(lane);
+      else
+         r = 0;
+      return r < 0 || (up && r + H >= N) ? -1 : r + (up ? H : 0);
+   }
+}
+
 // Gather of the first potential derivatives fused with the recip + self
-// field, one warp per atom: lane (jy, kz) < 25 reads one row of five points,
-// a fixed xor tree combines the rows.  MODE 0: real part -> d and p field,
-// self term with the permanent dipole.  MODE 1: real -> d, imaginary -> p,
-// self term with the induced dipoles.  Plain stores, rows of 8 floats.
+// field, one warp per atom: lane (ix, jy) < 25 reads one column of five z
+// points, so that each of a warp's five loads covers five rows of five
+// consecutive points (about six 128-byte lines; one lane per row touched 25
+// lines in each load), and the columns are combined by warp_sums.  MODE 0:
+// real part -> d and p field, self term with the permanent dipole.  MODE 1:
+// real -> d, imaginary -> p, self term with the induced dipoles.  Plain
+// stores, rows of 8 floats.
 // AP (MODE 1, ACC): the dipoles are the CG search direction p = z + b p_old
-// (P.conj = p_old, P.zrsd = z); instead of the field, lane 0 stores
-// p and Ap = p/alpha - field, and the block partials of p.Ap give, in the
-// last block, the step length a = s / p.Ap.  Atoms are visited warp-strided
-// over at most RED_MAX blocks.
+// (P.conj = p_old, P.zrsd = z); instead of the field, the lanes that hold
+// the components store p and Ap = p/alpha - field, and the block partials of
+// p.Ap give, in the last block, the step length a = s / p.Ap.  Atoms are
+// visited warp-strided over at most RED_MAX blocks.
 // LATE: the kernel has not waited for its programmatic predecessor yet; the
 // site and the B-splines (positions only) are formed first, then the wait,
 // then the grid and dipole reads, so the prologue overlaps the predecessor.
@@ -342,97 +426,85 @@ __device__ __forceinline__ void gather_atom(int s, int lane, const GridParams& G
    int i1, i2, i3;
    float w1, w2, w3;
    site(G, spos[s], i1, i2, i3, w1, w2, w3);
-   float acc[6] = {0, 0, 0, 0, 0, 0};
-   float t1[5][2], t2[5][2], t3[5][2];
-   bspline5<2>(w1, t1);
-   bspline5<2>(w2, t2);
+   constexpr int NC = MODE == 1 ? 6 : 3;
+   float acc[NC];
+#pragma unroll
+   for (int c = 0; c < NC; ++c)
+      acc[c] = 0.f;
+   float t3[5][2];
    bspline5<2>(w3, t3);
+   const int ix = lane % 5, jy = lane / 5;
+   float tx[2], ty[2];
+   SplinePiece(ix).eval<2>(w1, tx);
+   SplinePiece(jy).eval<2>(w2, ty);
    if (LATE)
       pdl_wait();
    if (lane < 25) {
-      const int jy = lane % 5, kz = lane / 5;
-      int zb = i3 + kz;
-      zb -= (zb >= G.n3 ? G.n3 : 0);
+      int xb = i1 + ix;
+      xb -= (xb >= G.n1 ? G.n1 : 0);
       int yb = i2 + jy;
       yb -= (yb >= G.n2 ? G.n2 : 0);
-      const size_t row = ((size_t)zb * G.n2 + yb) * G.n1;
-      float rt0 = 0.f, rt1 = 0.f, it0 = 0.f, it1 = 0.f;
+      const size_t plane = (size_t)G.n2 * G.n1;
+      const float2* col = g + ((size_t)yb * G.n1 + xb);
+      float2 q[5];
 #pragma unroll
-      for (int ix = 0; ix < 5; ++ix) {
-         int xb = i1 + ix;
-         xb -= (xb >= G.n1 ? G.n1 : 0);
-         const float2 qv = g[row + xb];
-         rt0 += qv.x * t1[ix][0];
-         rt1 += qv.x * t1[ix][1];
+      for (int kz = 0; kz < 5; ++kz) {
+         int zb = i3 + kz;
+         zb -= (zb >= G.n3 ? G.n3 : 0);
+         if (MODE == 1)
+            q[kz] = col[zb * plane];
+         else
+            q[kz].x = col[zb * plane].x;
+      }
+      float r0 = 0.f, r1 = 0.f, m0 = 0.f, m1 = 0.f;
+#pragma unroll
+      for (int kz = 0; kz < 5; ++kz) {
+         r0 += q[kz].x * t3[kz][0];
+         r1 += q[kz].x * t3[kz][1];
          if (MODE == 1) {
-            it0 += qv.y * t1[ix][0];
-            it1 += qv.y * t1[ix][1];
+            m0 += q[kz].y * t3[kz][0];
+            m1 += q[kz].y * t3[kz][1];
          }
       }
-      const float u0 = t2[jy][0], u1 = t2[jy][1], v0 = t3[kz][0], v1 = t3[kz][1];
-      acc[0] = rt1 * u0 * v0;
-      acc[1] = rt0 * u1 * v0;
-      acc[2] = rt0 * u0 * v1;
+      const float x1y = tx[1] * ty[0], xy1 = tx[0] * ty[1], xy = tx[0] * ty[0];
+      acc[0] = r0 * x1y;
+      acc[1] = r0 * xy1;
+      acc[2] = r1 * xy;
       if (MODE == 1) {
-         acc[3] = it1 * u0 * v0;
-         acc[4] = it0 * u1 * v0;
-         acc[5] = it0 * u0 * v1;
+         acc[NC - 3] = m0 * x1y;
+         acc[NC - 2] = m0 * xy1;
+         acc[NC - 1] = m1 * xy;
       }
    }
-#pragma unroll
-   for (int c = 0; c < (MODE == 1 ? 6 : 3); ++c)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-         acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+   const float sum = warp_sums<NC>(acc, lane);
+   const int c = sum_slot<NC>(lane);
+   if (c < 0)
+      return;
+   // the lane that holds component c finishes it
+   const int d = c < 3 ? c : c - 3, x = 8 * s + c;
+   const float gc = d == 0 ? G.a1 : (d == 1 ? G.a2 : G.a3);
    if (AP) {
-      // lane c < 6 finishes component c: p, its recip + self field added to
-      // the real-space field, Ap = p/alpha - field, and p.Ap
-      if (lane < 6) {
-         float ac = acc[0];
-#pragma unroll
-         for (int k = 1; k < 6; ++k)
-            if (lane == k)
-               ac = acc[k];
-         const int c = lane, x = 8 * s + c;
-         const float gc = c % 3 == 0 ? G.a1 : (c % 3 == 1 ? G.a2 : G.a3);
-         const float p = __fmaf_rn(c < 3 ? bd : bp, P.conj[x], P.zrsd[x]);
-         const float fld = out[x] + (G.selfterm * p - gc * ac);
-         const float v = P.polinv[s] * p - fld;
-         P.vec[x] = v;
-         P.conj[x] = p;
-         pap[c < 3 ? 0 : 1] += p * v;
-      }
+      // p, its recip + self field added to the real-space field, Ap =
+      // p/alpha - field, and p.Ap
+      const float p = __fmaf_rn(c < 3 ? bd : bp, P.conj[x], P.zrsd[x]);
+      const float fld = out[x] + (G.selfterm * p - gc * sum);
+      const float v = P.polinv[s] * p - fld;
+      P.vec[x] = v;
+      P.conj[x] = p;
+      pap[c < 3 ? 0 : 1] += p * v;
       return;
    }
-   if (lane != 0)
-      return;
-   float* a = out + 8 * s;
-   float r[6];
    if (MODE == 0) {
-      const float* m = rp + 12 * s;
-      r[0] = r[3] = -G.a1 * acc[0] + G.selfterm * m[1];
-      r[1] = r[4] = -G.a2 * acc[1] + G.selfterm * m[2];
-      r[2] = r[5] = -G.a3 * acc[2] + G.selfterm * m[3];
-   } else {
-      float u[8];
-      if (DIR)
-         dir_row(P.conj, P.zrsd, s, bd, bp, u);
-      else
-#pragma unroll
-         for (int c = 0; c < 6; ++c)
-            u[c] = u8[8 * s + c];
-      r[0] = G.selfterm * u[0] - G.a1 * acc[0];
-      r[1] = G.selfterm * u[1] - G.a2 * acc[1];
-      r[2] = G.selfterm * u[2] - G.a3 * acc[2];
-      r[3] = G.selfterm * u[3] - G.a1 * acc[3];
-      r[4] = G.selfterm * u[4] - G.a2 * acc[4];
-      r[5] = G.selfterm * u[5] - G.a3 * acc[5];
+      const float r = -gc * sum + G.selfterm * rp[12 * s + 1 + d];
+      out[x] = ACC ? out[x] + r : r;
+      out[x + 3] = ACC ? out[x + 3] + r : r;
+      return;
    }
+   const float u = DIR ? __fmaf_rn(c < 3 ? bd : bp, P.conj[x], P.zrsd[x]) : u8[x];
+   const float r = G.selfterm * u - gc * sum;
    // ACC: add to the real-space field already stored (the same two-operand
    // sum the real-space kernel forms when it adds this result as its base)
-#pragma unroll
-   for (int c = 0; c < 6; ++c)
-      a[c] = ACC ? a[c] + r[c] : r[c];
+   out[x] = ACC ? out[x] + r : r;
 }
 
 template <int MODE, bool ACC, bool AP = false, bool DIR = false>
