@@ -59,6 +59,21 @@ __device__ __forceinline__ float erfc_hastings(float x, float expmx2)
 
 __device__ __forceinline__ float image1(float d, float l, float linv) { return d - l * rintf(d * linv); }
 
+// one 32-byte row: d xyz, p xyz, thole, polarizability
+__device__ __forceinline__ void load8(const float* __restrict__ a, int s, float* v)
+{
+   const float4* p = reinterpret_cast<const float4*>(a + 8 * s);
+   const float4 x = p[0], y = p[1];
+   v[0] = x.x;
+   v[1] = x.y;
+   v[2] = x.z;
+   v[3] = x.w;
+   v[4] = y.x;
+   v[5] = y.y;
+   v[6] = y.z;
+   v[7] = y.w;
+}
+
 struct PmeGrid {
    int n1 = 0, n2 = 0, n3 = 0;
    bool own_fft = false;      // power-of-two grid: the library's fused FFT path
@@ -69,6 +84,9 @@ struct PmeGrid {
    float2* qgrid2 = nullptr;  // the second grid pair (induced-dipole reciprocal forces)
    long long* qfx2 = nullptr;
    float* infl = nullptr;     // influence function [n3][n2][n1]
+   int4* org = nullptr;       // [npad] grid origin of each slot's spline support (x, y, z)
+   float* spl_lo = nullptr;   // [npad][SPL_ROW] spline values and first derivatives (spline.cuh)
+   float* spl_hi = nullptr;   // [npad][SPL_ROW] second and third derivatives
    float2* qstash = nullptr;  // transformed permanent grid kept for the virial cross terms
    bool packed = false;       // the fixed-point grid holds packed d / p dipole values
    int pack_shift = 24;       // their 32-bit fixed-point scale 2^pack_shift (16 after a range fallback)

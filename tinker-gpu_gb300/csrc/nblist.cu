@@ -21,6 +21,7 @@
 #include <map>
 
 #include "common.cuh"
+#include "spline.cuh"
 
 namespace t9gb {
 
@@ -602,23 +603,56 @@ int list_update(Context* ctx)
 // ---------------------------------------------------------------------------
 // positions and permutations
 
-// sorted positions, w = pdamp (read with the position by every pair kernel)
+// Sorted positions, w = pdamp (read with the position by every pair kernel),
+// and with PME every slot's grid origin and B-spline weights.  Three threads
+// per slot, one per axis.  The weights depend on the positions only and are
+// read by every spread and gather until the next update (12 of them in a
+// five-iteration solve).
+struct SplineParams {
+   float r[3];         // 1 / box
+   int nfft[3];        // 0: no PME
+   int4* org;          // [npad] grid origins
+   float *lo, *hi;     // [npad][SPL_ROW]
+};
+
 __global__ void k_scatter_pos(int npad, const int* __restrict__ perm, const float* __restrict__ xyz,
-   const float2* __restrict__ sdamp, float4* __restrict__ spos)
+   const float2* __restrict__ sdamp, float4* __restrict__ spos, SplineParams S)
 {
-   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < npad; s += gridDim.x * blockDim.x) {
-      int a = perm[s];
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (a >= 0)
-         v = make_float4(xyz[3 * a], xyz[3 * a + 1], xyz[3 * a + 2], sdamp[s].x);
-      spos[s] = v;
+   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 3 * npad; e += gridDim.x * blockDim.x) {
+      const int s = e / 3, d = e - 3 * s;
+      const int a = perm[s];
+      if (a < 0) {
+         if (d == 0)
+            spos[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+         continue;
+      }
+      const float x = xyz[3 * a + d];
+      if (d == 0)
+         spos[s] = make_float4(x, xyz[3 * a + 1], xyz[3 * a + 2], sdamp[s].x);
+      if (S.nfft[0]) {
+         const float rb = d == 0 ? S.r[0] : d == 1 ? S.r[1] : S.r[2];
+         const int nf = d == 0 ? S.nfft[0] : d == 1 ? S.nfft[1] : S.nfft[2];
+         reinterpret_cast<int*>(S.org)[4 * s + d] =
+            spline_axis(x, rb, nf, d, S.lo + (size_t)SPL_ROW * s, S.hi + (size_t)SPL_ROW * s);
+      }
    }
 }
 
 int scatter_positions(Context* ctx)
 {
-   k_scatter_pos<<<grid_for(ctx->npad, 256), 256, 0, ctx->stream>>>(ctx->npad, ctx->perm, ctx->xyz, ctx->sdamp,
-      ctx->spos);
+   const t9gb_config& c = ctx->cfg;
+   SplineParams S = {};
+   if (c.use_ewald) {
+      for (int d = 0; d < 3; ++d) {
+         S.r[d] = (float)(1.0 / c.box[d]);
+         S.nfft[d] = c.nfft[d];
+      }
+      S.org = ctx->pme.org;
+      S.lo = ctx->pme.spl_lo;
+      S.hi = ctx->pme.spl_hi;
+   }
+   k_scatter_pos<<<grid_for(3 * (long long)ctx->npad, 256), 256, 0, ctx->stream>>>(ctx->npad, ctx->perm, ctx->xyz,
+      ctx->sdamp, ctx->spos, S);
    T9_CUDA(cudaGetLastError());
    ctx->list_stale = true;
    return T9GB_OK;

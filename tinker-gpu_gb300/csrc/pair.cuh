@@ -46,21 +46,6 @@ __device__ __forceinline__ void group_reduce(float* v)
    }
 }
 
-// one 32-byte row: d xyz, p xyz, thole, polarizability
-__device__ __forceinline__ void load8(const float* __restrict__ a, int s, float* v)
-{
-   const float4* p = reinterpret_cast<const float4*>(a + 8 * s);
-   const float4 x = p[0], y = p[1];
-   v[0] = x.x;
-   v[1] = x.y;
-   v[2] = x.z;
-   v[3] = x.w;
-   v[4] = y.x;
-   v[5] = y.y;
-   v[6] = y.z;
-   v[7] = y.w;
-}
-
 static inline PairParams make_params(const Context* ctx, double cutoff)
 {
    PairParams P;

@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "reduce.cuh"
+#include "spline.cuh"
 
 namespace t9gb {
 
@@ -185,18 +186,15 @@ __device__ __forceinline__ void grid_add(unsigned long long* q, size_t idx, floa
       red_u64(q, idx, (unsigned long long)to_fx(v));
 }
 
-// d and p values of one point into one word; a value at or above pk_lim in
-// magnitude (1/32 of the half's range) raises the range flag
-__device__ __forceinline__ void grid_add2(unsigned long long* q, size_t idx, float vd, float vp, const GridParams& G)
+// d and p values of one point into one word; false when a value is at or
+// above pk_lim in magnitude (1/32 of the half's range) or not a number: the
+// caller raises the range flag, and the grid's user solves again
+__device__ __forceinline__ bool grid_add2(unsigned long long* q, float vd, float vp, const GridParams& G)
 {
-   if (vd == 0.f && vp == 0.f)
-      return;
-   if (!(fabsf(vd) < G.pk_lim && fabsf(vp) < G.pk_lim)) {
-      atomicOr(G.range, 1);
-      return;
-   }
+   const bool ok = (fabsf(vd) < G.pk_lim) & (fabsf(vp) < G.pk_lim);
    const long long a = __float2int_rn(vd * G.pk_s), b = __float2int_rn(vp * G.pk_s);
-   red_u64(q, idx, (unsigned long long)(a * 4294967296ll + b));
+   red_u64(q, 0, (unsigned long long)(a * 4294967296ll + b));
+   return ok;
 }
 
 // one word of the fixed-point grid as a complex value
@@ -223,44 +221,25 @@ __device__ __forceinline__ bool grid_word_big(long long w, int packed)
    return a >= (1 << 30) || a <= -(1 << 30) || b >= (1 << 30) || b <= -(1 << 30);
 }
 
-// One piece of the order-5 cardinal B-spline and its derivatives as
-// polynomials in t, for a lane that owns one of the five points along an
-// axis.  The pieces mirror each other (M5 is even about its centre), so the
-// first two are the last two at t = 1 - w with the odd derivatives' sign
-// flipped, and there is no cancellation at either end.  Coefficients x 24:
-// centre 11 + 12 t - 6 t^2 - 12 t^3 + 6 t^4, next 1 + 4 t + 6 t^2 + 4 t^3 -
-// 4 t^4, edge t^4 (the closed form of the recursion in bspline5).
-struct SplinePiece {
-   float c0, c1, c2, c3, c4;
-   bool mirror;
-   __device__ __forceinline__ explicit SplinePiece(int j)
-   {
-      mirror = j < 2;
-      const bool mid = j == 2, edge = j == 0 || j == 4;
-      constexpr float q = 1.f / 24.f;
-      c0 = mid ? 11.f * q : edge ? 0.f : q;
-      c1 = mid ? 12.f * q : edge ? 0.f : 4.f * q;
-      c2 = mid ? -6.f * q : edge ? 0.f : 6.f * q;
-      c3 = mid ? -12.f * q : edge ? 0.f : 4.f * q;
-      c4 = mid ? 6.f * q : edge ? q : -4.f * q;
-   }
-   template <int LEVEL>
-   __device__ __forceinline__ void eval(float w, float* th) const
-   {
-      const float t = mirror ? 1.f - w : w;
-      th[0] = __fmaf_rn(__fmaf_rn(__fmaf_rn(__fmaf_rn(c4, t, c3), t, c2), t, c1), t, c0);
-      if (LEVEL > 1) {
-         const float d = __fmaf_rn(__fmaf_rn(__fmaf_rn(4.f * c4, t, 3.f * c3), t, 2.f * c2), t, c1);
-         th[1] = mirror ? -d : d;
-      }
-      if (LEVEL > 2)
-         th[2] = __fmaf_rn(__fmaf_rn(12.f * c4, t, 6.f * c3), t, 2.f * c2);
-      if (LEVEL > 3) {
-         const float d = __fmaf_rn(24.f * c4, t, 6.f * c3);
-         th[3] = mirror ? -d : d;
-      }
-   }
+// The sites' spline tables and grid origins (spline.cuh) as the kernels take
+// them.
+struct Sites {
+   const int4* org;
+   const float *lo, *hi;
 };
+
+// Byte stride between z planes of a grid of 8-byte points.
+__device__ __forceinline__ unsigned plane_bytes(const GridParams& G) { return 8u * (unsigned)G.n1 * (unsigned)G.n2; }
+
+// Byte offset within a plane of point (ix, jy) of a site's support.
+__device__ __forceinline__ unsigned column_bytes(const GridParams& G, int4 o, int ix, int jy)
+{
+   int xb = o.x + ix;
+   xb -= (xb >= G.n1 ? G.n1 : 0);
+   int yb = o.y + jy;
+   yb -= (yb >= G.n2 ? G.n2 : 0);
+   return 8u * ((unsigned)yb * (unsigned)G.n1 + (unsigned)xb);
+}
 
 // Spreading, one warp per atom: lane (ix, jy) < 25 owns one column of five z
 // points, so that each of a warp's five reductions covers five rows of five
@@ -270,67 +249,71 @@ struct SplinePiece {
 // 8.  DIR (MODE 1): the dipoles are the CG search direction p = z + b p_old
 // (src = p_old, z8 = z, b from scal), formed as each row is read.
 template <int MODE, bool DIR = false>
-__global__ void __launch_bounds__(256) k_spread(int n, GridParams G, const float4* __restrict__ spos,
-   const float* __restrict__ src, const float* __restrict__ z8, const double* __restrict__ scal,
-   unsigned long long* __restrict__ q)
+__global__ void __launch_bounds__(256) k_spread(int n, GridParams G, Sites S, const float* __restrict__ src,
+   const float* __restrict__ z8, const double* __restrict__ scal, unsigned long long* __restrict__ q)
 {
-   // the site and the B-splines need the positions only: they are formed
-   // before the wait for the programmatic predecessor (no-op otherwise)
+   // the sites do not depend on the programmatic predecessor: they are read
+   // before the wait for it (no-op otherwise)
    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
    const int lane = threadIdx.x & 31;
    if (s >= n || lane >= 25)
       return;
-   int i1, i2, i3;
-   float w1, w2, w3;
-   site(G, spos[s], i1, i2, i3, w1, w2, w3);
-   constexpr int L = MODE == 0 ? 3 : 2;
    const int ix = lane % 5, jy = lane / 5;
-   float tx[L], ty[L], t3[5][L];
-   SplinePiece(ix).eval<L>(w1, tx);
-   SplinePiece(jy).eval<L>(w2, ty);
-   bspline5<L>(w3, t3);
-   int xb = i1 + ix;
-   xb -= (xb >= G.n1 ? G.n1 : 0);
-   int yb = i2 + jy;
-   yb -= (yb >= G.n2 ? G.n2 : 0);
-   const size_t plane = (size_t)G.n2 * G.n1;
-   unsigned long long* col = q + ((size_t)yb * G.n1 + xb);
-   pdl_wait();
-   pdl_trigger();
-   const float xy = tx[0] * ty[0], x1y = tx[1] * ty[0], xy1 = tx[0] * ty[1];
+   const int4 o = S.org[s];
+   const float* lo = S.lo + (size_t)SPL_ROW * s;
+   const float* hi = S.hi + (size_t)SPL_ROW * s;
+   const float2 tx = spl(lo, 0, ix), ty = spl(lo, 1, jy);
+   float2 tz[5];
+#pragma unroll
+   for (int k = 0; k < 5; ++k)
+      tz[k] = spl(lo, 2, k);
+   char* col = reinterpret_cast<char*>(q) + column_bytes(G, o, ix, jy);
+   const unsigned plane = plane_bytes(G);
+   const float xy = tx.x * ty.x, x1y = tx.y * ty.x, xy1 = tx.x * ty.y;
    if (MODE == 0) {
+      const float x2 = spl(hi, 0, ix).x, y2 = spl(hi, 1, jy).x;
+      float z2[5];
+#pragma unroll
+      for (int k = 0; k < 5; ++k)
+         z2[k] = spl(hi, 2, k).x;
+      pdl_wait();
+      pdl_trigger();
       const float* m = src + 12 * s;
       // Cartesian -> fractional (orthogonal box; quadrupole off-diagonals doubled)
       const float f0 = m[0];
       const float fx = G.a1 * m[1], fy = G.a2 * m[2], fz = G.a3 * m[3];
       const float fxx = G.a1 * G.a1 * m[4], fyy = G.a2 * G.a2 * m[5], fzz = G.a3 * G.a3 * m[6];
       const float fxy = 2.f * G.a1 * G.a2 * m[7], fxz = 2.f * G.a1 * G.a3 * m[8], fyz = 2.f * G.a2 * G.a3 * m[9];
-      const float x2y = tx[L - 1] * ty[0], xy2 = tx[0] * ty[L - 1], x1y1 = tx[1] * ty[1];
-      const float c0 = f0 * xy + fx * x1y + fy * xy1 + fxx * x2y + fyy * xy2 + fxy * x1y1;
+      const float c0 = f0 * xy + fx * x1y + fy * xy1 + fxx * x2 * ty.x + fyy * tx.x * y2 + fxy * tx.y * ty.y;
       const float c1 = fz * xy + fxz * x1y + fyz * xy1;
       const float c2 = fzz * xy;
 #pragma unroll
       for (int kz = 0; kz < 5; ++kz) {
-         int zb = i3 + kz;
+         int zb = o.z + kz;
          zb -= (zb >= G.n3 ? G.n3 : 0);
-         grid_add(col, zb * plane, c0 * t3[kz][0] + c1 * t3[kz][1] + c2 * t3[kz][L - 1]);
+         grid_add(reinterpret_cast<unsigned long long*>(col + (size_t)(unsigned)zb * plane), 0,
+            c0 * tz[kz].x + c1 * tz[kz].y + c2 * z2[kz]);
       }
    } else {
+      pdl_wait();
+      pdl_trigger();
       float u[8];
       if (DIR)
          dir_row(src, z8, s, (float)scal[S_B_D], (float)scal[S_B_P], u);
       else
-#pragma unroll
-         for (int c = 0; c < 6; ++c)
-            u[c] = src[8 * s + c];
+         load8(src, s, u);
       const float d0 = G.a1 * u[0] * x1y + G.a2 * u[1] * xy1, d1 = G.a3 * u[2] * xy;
       const float p0 = G.a1 * u[3] * x1y + G.a2 * u[4] * xy1, p1 = G.a3 * u[5] * xy;
+      bool ok = true;
 #pragma unroll
       for (int kz = 0; kz < 5; ++kz) {
-         int zb = i3 + kz;
+         int zb = o.z + kz;
          zb -= (zb >= G.n3 ? G.n3 : 0);
-         grid_add2(col, zb * plane, d0 * t3[kz][0] + d1 * t3[kz][1], p0 * t3[kz][0] + p1 * t3[kz][1], G);
+         ok &= grid_add2(reinterpret_cast<unsigned long long*>(col + (size_t)(unsigned)zb * plane),
+            d0 * tz[kz].x + d1 * tz[kz].y, p0 * tz[kz].x + p1 * tz[kz].y, G);
       }
+      if (!ok)
+         atomicOr(G.range, 1);
    }
 }
 
@@ -416,57 +399,56 @@ __device__ __forceinline__ int sum_slot(int lane)
 // p.Ap give, in the last block, the step length a = s / p.Ap.  Atoms are
 // visited warp-strided over at most RED_MAX blocks.
 // LATE: the kernel has not waited for its programmatic predecessor yet; the
-// site and the B-splines (positions only) are formed first, then the wait,
-// then the grid and dipole reads, so the prologue overlaps the predecessor.
+// site's splines are read first, then the wait, then the grid and dipole
+// reads, so the prologue overlaps the predecessor.
 template <int MODE, bool ACC, bool AP, bool DIR, bool LATE = false>
-__device__ __forceinline__ void gather_atom(int s, int lane, const GridParams& G, const float4* __restrict__ spos,
+__device__ __forceinline__ void gather_atom(int s, int lane, const GridParams& G, const Sites& S,
    const float2* __restrict__ g, const float* __restrict__ rp, const float* __restrict__ u8, float* __restrict__ out,
    const PcgAp& P, float bd, float bp, float* pap)
 {
-   int i1, i2, i3;
-   float w1, w2, w3;
-   site(G, spos[s], i1, i2, i3, w1, w2, w3);
    constexpr int NC = MODE == 1 ? 6 : 3;
    float acc[NC];
 #pragma unroll
    for (int c = 0; c < NC; ++c)
       acc[c] = 0.f;
-   float t3[5][2];
-   bspline5<2>(w3, t3);
+   const int4 o = S.org[s];
+   const float* lo = S.lo + (size_t)SPL_ROW * s;
    const int ix = lane % 5, jy = lane / 5;
-   float tx[2], ty[2];
-   SplinePiece(ix).eval<2>(w1, tx);
-   SplinePiece(jy).eval<2>(w2, ty);
+   float2 tx, ty, t3[5];
+   if (lane < 25) {
+      tx = spl(lo, 0, ix);
+      ty = spl(lo, 1, jy);
+#pragma unroll
+      for (int k = 0; k < 5; ++k)
+         t3[k] = spl(lo, 2, k);
+   }
    if (LATE)
       pdl_wait();
    if (lane < 25) {
-      int xb = i1 + ix;
-      xb -= (xb >= G.n1 ? G.n1 : 0);
-      int yb = i2 + jy;
-      yb -= (yb >= G.n2 ? G.n2 : 0);
-      const size_t plane = (size_t)G.n2 * G.n1;
-      const float2* col = g + ((size_t)yb * G.n1 + xb);
+      const unsigned plane = plane_bytes(G);
+      const char* col = reinterpret_cast<const char*>(g) + column_bytes(G, o, ix, jy);
       float2 q[5];
 #pragma unroll
       for (int kz = 0; kz < 5; ++kz) {
-         int zb = i3 + kz;
+         int zb = o.z + kz;
          zb -= (zb >= G.n3 ? G.n3 : 0);
+         const float2* p = reinterpret_cast<const float2*>(col + (size_t)(unsigned)zb * plane);
          if (MODE == 1)
-            q[kz] = col[zb * plane];
+            q[kz] = *p;
          else
-            q[kz].x = col[zb * plane].x;
+            q[kz].x = p->x;
       }
       float r0 = 0.f, r1 = 0.f, m0 = 0.f, m1 = 0.f;
 #pragma unroll
       for (int kz = 0; kz < 5; ++kz) {
-         r0 += q[kz].x * t3[kz][0];
-         r1 += q[kz].x * t3[kz][1];
+         r0 += q[kz].x * t3[kz].x;
+         r1 += q[kz].x * t3[kz].y;
          if (MODE == 1) {
-            m0 += q[kz].y * t3[kz][0];
-            m1 += q[kz].y * t3[kz][1];
+            m0 += q[kz].y * t3[kz].x;
+            m1 += q[kz].y * t3[kz].y;
          }
       }
-      const float x1y = tx[1] * ty[0], xy1 = tx[0] * ty[1], xy = tx[0] * ty[0];
+      const float x1y = tx.y * ty.x, xy1 = tx.x * ty.y, xy = tx.x * ty.x;
       acc[0] = r0 * x1y;
       acc[1] = r0 * xy1;
       acc[2] = r1 * xy;
@@ -508,7 +490,7 @@ __device__ __forceinline__ void gather_atom(int s, int lane, const GridParams& G
 }
 
 template <int MODE, bool ACC, bool AP = false, bool DIR = false>
-__global__ void __launch_bounds__(256, 6) k_gather_field(int n, GridParams G, const float4* __restrict__ spos,
+__global__ void __launch_bounds__(256, 6) k_gather_field(int n, GridParams G, Sites S,
    const float2* __restrict__ g, const float* __restrict__ rp, const float* __restrict__ u8, float* __restrict__ out,
    PcgAp P)
 {
@@ -525,7 +507,7 @@ __global__ void __launch_bounds__(256, 6) k_gather_field(int n, GridParams G, co
          bp = (float)P.scal[S_B_P];
       }
       if (s < n)
-         gather_atom<MODE, ACC, false, DIR, LATE>(s, lane, G, spos, g, rp, u8, out, P, bd, bp, nullptr);
+         gather_atom<MODE, ACC, false, DIR, LATE>(s, lane, G, S, g, rp, u8, out, P, bd, bp, nullptr);
       else if (LATE)
          pdl_wait();
       return;
@@ -535,7 +517,7 @@ __global__ void __launch_bounds__(256, 6) k_gather_field(int n, GridParams G, co
    float pap[2] = {0.f, 0.f};
    const int nw = (gridDim.x * blockDim.x) >> 5;
    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < n; s += nw)
-      gather_atom<MODE, ACC, true, false>(s, lane, G, spos, g, rp, u8, out, P, bd, bp, pap);
+      gather_atom<MODE, ACC, true, false>(s, lane, G, S, g, rp, u8, out, P, bd, bp, pap);
    store_partials_f<2>(P.red, R_PAP_D, pap, sh);
    if (!last_block(P.state + ST_TICKET1))
       return;
@@ -1555,6 +1537,9 @@ int pme_setup(Context* ctx)
                e = std::exp(term) / (hsq * pi * vol * m1[k1] * m2[k2] * m3[k3]);
             infl[i] = (float)e;
          }
+   T9_CUDA(cudaMalloc(&P.org, sizeof(int4) * ctx->npad));
+   T9_CUDA(cudaMalloc(&P.spl_lo, sizeof(float) * SPL_ROW * (size_t)ctx->npad));
+   T9_CUDA(cudaMalloc(&P.spl_hi, sizeof(float) * SPL_ROW * (size_t)ctx->npad));
    float* d_infl = nullptr;
    T9_CUDA(cudaMalloc(&d_infl, sizeof(float) * ng));
    T9_CUDA(cudaMemcpy(d_infl, infl.data(), sizeof(float) * ng, cudaMemcpyHostToDevice));
@@ -1599,10 +1584,15 @@ void pme_free(Context* ctx)
    cudaFree(P.qgrid);
    cudaFree(P.qfx);
    cudaFree(P.infl);
+   cudaFree(P.org);
+   cudaFree(P.spl_lo);
+   cudaFree(P.spl_hi);
    cudaFree(P.qstash);
    cudaFree(P.fft_err);
    P = PmeGrid();
 }
+
+static Sites sites(const Context* ctx) { return Sites{ctx->pme.org, ctx->pme.spl_lo, ctx->pme.spl_hi}; }
 
 static GridParams grid_params(const Context* ctx)
 {
@@ -1707,7 +1697,7 @@ int launch_dfield_recip_grid(Context* ctx)
    GridParams G = grid_params(ctx);
    prof_begin(ctx, P_SPREAD_MPOLE);
    ctx->pme.packed = false;
-   k_spread<0><<<grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream>>>(ctx->n, G, ctx->spos, ctx->srpole,
+   k_spread<0><<<grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->srpole,
       nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx));
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
@@ -1722,10 +1712,10 @@ int launch_dfield_recip_gather(Context* ctx, float* out6, bool acc)
    const int nb = grid_for((long long)ctx->n * 32, 256);
    prof_begin(ctx, P_GATHER_MPOLE);
    if (acc)
-      k_gather_field<0, true><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, ctx->spos, ctx->pme.qgrid, ctx->srpole, nullptr,
+      k_gather_field<0, true><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->pme.qgrid, ctx->srpole, nullptr,
          out6, PcgAp{});
    else
-      k_gather_field<0, false><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, ctx->spos, ctx->pme.qgrid, ctx->srpole,
+      k_gather_field<0, false><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->pme.qgrid, ctx->srpole,
          nullptr, out6, PcgAp{});
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
@@ -1746,7 +1736,7 @@ int launch_ufield_recip_grid(Context* ctx, const float* u6)
    prof_begin(ctx, P_SPREAD_UIND);
    ctx->pme.packed = true;
    T9_CUDA(launch_k(use_pdl(ctx), k_spread<1, false>, grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream,
-      ctx->n, G, ctx->spos, u6, nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx)));
+      ctx->n, G, sites(ctx), u6, nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx)));
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return fft_conv(ctx);
@@ -1760,7 +1750,7 @@ int launch_ufield_recip_gather(Context* ctx, const float* u6, float* out6, bool 
    const int nb = grid_for((long long)ctx->n * 32, 256);
    prof_begin(ctx, P_GATHER_UIND);
    T9_CUDA(launch_k(use_pdl(ctx), acc ? k_gather_field<1, true> : k_gather_field<1, false>, nb, 256, 0, ctx->stream,
-      ctx->n, G, ctx->spos, ctx->pme.qgrid, nullptr, u6, out6, PcgAp{}));
+      ctx->n, G, sites(ctx), ctx->pme.qgrid, nullptr, u6, out6, PcgAp{}));
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
@@ -1804,7 +1794,7 @@ int launch_ufield_recip_grid_dir(Context* ctx, const float* p6, const float* z6,
    prof_begin(ctx, P_SPREAD_UIND);
    ctx->pme.packed = true;
    T9_CUDA(launch_k(use_pdl(ctx), k_spread<1, true>, grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream,
-      ctx->n, G, ctx->spos, p6, z6, scal, reinterpret_cast<unsigned long long*>(ctx->pme.qfx)));
+      ctx->n, G, sites(ctx), p6, z6, scal, reinterpret_cast<unsigned long long*>(ctx->pme.qfx)));
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return fft_conv(ctx);
@@ -1817,7 +1807,7 @@ int launch_ufield_recip_gather_dir(Context* ctx, float* out6, const PcgAp& P)
    GridParams G = grid_params(ctx);
    const int nb = grid_for((long long)ctx->n * 32, 256);
    prof_begin(ctx, P_GATHER_UIND);
-   k_gather_field<1, true, false, true><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, ctx->spos, ctx->pme.qgrid, nullptr,
+   k_gather_field<1, true, false, true><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->pme.qgrid, nullptr,
       nullptr, out6, P);
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
@@ -1831,7 +1821,7 @@ int launch_ufield_recip_gather_ap(Context* ctx, float* out6, const PcgAp& P)
    GridParams G = grid_params(ctx);
    const int nb = std::min(RED_MAX, grid_for((long long)ctx->n * 32, 256));
    prof_begin(ctx, P_GATHER_UIND);
-   k_gather_field<1, true, true><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, ctx->spos, ctx->pme.qgrid, nullptr, nullptr,
+   k_gather_field<1, true, true><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->pme.qgrid, nullptr, nullptr,
       out6, P);
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
@@ -1847,7 +1837,7 @@ int launch_empole_recip(Context* ctx, double* e_atom)
       return T9GB_OK;
    GridParams G = grid_params(ctx);
    ctx->pme.packed = false;
-   k_spread<0><<<grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream>>>(ctx->n, G, ctx->spos, ctx->srpole,
+   k_spread<0><<<grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->srpole,
       nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx));
    T9_CUDA(cudaGetLastError());
    T9_CHECK(fft_conv(ctx));
@@ -1878,7 +1868,7 @@ int launch_force_recip_perm(Context* ctx, bool mpole, bool polar, float* wrec)
       T9_CUDA(cudaMemsetAsync(ctx->scal + 40, 0, sizeof(double) * 12, ctx->stream));
    }
    ctx->pme.packed = false;
-   k_spread<0><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, ctx->spos, ctx->srpole,
+   k_spread<0><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->srpole,
       nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx));
    T9_CUDA(cudaGetLastError());
    T9_CHECK(fft_conv(ctx, vir ? 1 : 0, mpole ? 0.5f * f : 0.f, 0.f, vir && polar, ctx->scal + 40));
@@ -1912,7 +1902,7 @@ int launch_force_recip_uind(Context* ctx, float* wrec, bool alt)
    const float f = (float)ctx->cfg.electric;
    const bool vir = wrec != nullptr;
    P.packed = true;
-   k_spread<1><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, ctx->spos, ctx->uind,
+   k_spread<1><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->uind,
       nullptr, nullptr, reinterpret_cast<unsigned long long*>(P.qfx));
    int rc = cudaGetLastError() == cudaSuccess ? T9GB_OK : T9GB_CUDA_ERR;
    if (rc == T9GB_OK)
