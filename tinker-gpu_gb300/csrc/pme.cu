@@ -88,49 +88,6 @@ static void bspline_moduli(int nfft, int order, std::vector<double>& mod)
    }
 }
 
-// ---------------------------------------------------------------------------
-// per-site B-spline weights (include/seq/bsplgen.h:27-116), order 5
-
-template <int LEVEL>
-__device__ __forceinline__ void bspline5(float w, float th[5][LEVEL])
-{
-   float b[6][6];  // b[order][i], 1-based
-   b[2][2] = w;
-   b[2][1] = 1.f - w;
-   b[3][3] = 0.5f * w * b[2][2];
-   b[3][2] = 0.5f * ((1.f + w) * b[2][1] + (2.f - w) * b[2][2]);
-   b[3][1] = 0.5f * (1.f - w) * b[2][1];
-#pragma unroll
-   for (int i = 4; i <= 5; ++i) {
-      const int k = i - 1;
-      const float denom = 1.f / k;
-      b[i][i] = denom * w * b[k][k];
-#pragma unroll
-      for (int j = 1; j <= i - 2; ++j)
-         b[i][i - j] = denom * ((w + j) * b[k][i - j - 1] + (i - j - w) * b[k][i - j]);
-      b[i][1] = denom * (1.f - w) * b[k][1];
-   }
-   // derivative rows by repeated differencing of the lower-order rows
-#pragma unroll
-   for (int lv = 2; lv <= LEVEL; ++lv) {
-      const int k = 5 - lv + 1;
-#pragma unroll
-      for (int pass = 0; pass < lv - 1; ++pass) {
-         const int top = 5 - (lv - 2) + pass;
-         b[k][top] = b[k][top - 1];
-#pragma unroll
-         for (int i = top - 1; i >= 2; --i)
-            b[k][i] = b[k][i - 1] - b[k][i];
-         b[k][1] = -b[k][1];
-      }
-   }
-#pragma unroll
-   for (int i = 1; i <= 5; ++i)
-#pragma unroll
-      for (int j = 1; j <= LEVEL; ++j)
-         th[i - 1][j - 1] = b[5 - j + 1][i];
-}
-
 struct GridParams {
    int n1, n2, n3;
    float r1, r2, r3;  // 1/box
@@ -241,6 +198,13 @@ __device__ __forceinline__ unsigned column_bytes(const GridParams& G, int4 o, in
    return 8u * ((unsigned)yb * (unsigned)G.n1 + (unsigned)xb);
 }
 
+// a b + c d with the product c d rounded: the roundings of a grid value are
+// written out, so that they do not depend on how a kernel is laid out
+__device__ __forceinline__ float dot2(float a, float b, float c, float d)
+{
+   return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+
 // Spreading, one warp per atom: lane (ix, jy) < 25 owns one column of five z
 // points, so that each of a warp's five reductions covers five rows of five
 // consecutive words.  MODE 0 spreads fractional multipoles into the real
@@ -269,9 +233,9 @@ __global__ void __launch_bounds__(256) k_spread(int n, GridParams G, Sites S, co
       tz[k] = spl(lo, 2, k);
    char* col = reinterpret_cast<char*>(q) + column_bytes(G, o, ix, jy);
    const unsigned plane = plane_bytes(G);
-   const float xy = tx.x * ty.x, x1y = tx.y * ty.x, xy1 = tx.x * ty.y;
+   const float u0 = ty.x, u1 = ty.y;
    if (MODE == 0) {
-      const float x2 = spl(hi, 0, ix).x, y2 = spl(hi, 1, jy).x;
+      const float x2 = spl(hi, 0, ix).x, u2 = spl(hi, 1, jy).x;
       float z2[5];
 #pragma unroll
       for (int k = 0; k < 5; ++k)
@@ -284,15 +248,20 @@ __global__ void __launch_bounds__(256) k_spread(int n, GridParams G, Sites S, co
       const float fx = G.a1 * m[1], fy = G.a2 * m[2], fz = G.a3 * m[3];
       const float fxx = G.a1 * G.a1 * m[4], fyy = G.a2 * G.a2 * m[5], fzz = G.a3 * G.a3 * m[6];
       const float fxy = 2.f * G.a1 * G.a2 * m[7], fxz = 2.f * G.a1 * G.a3 * m[8], fyz = 2.f * G.a2 * G.a3 * m[9];
-      const float c0 = f0 * xy + fx * x1y + fy * xy1 + fxx * x2 * ty.x + fyy * tx.x * y2 + fxy * tx.y * ty.y;
-      const float c1 = fz * xy + fxz * x1y + fyz * xy1;
-      const float c2 = fzz * xy;
 #pragma unroll
       for (int kz = 0; kz < 5; ++kz) {
          int zb = o.z + kz;
          zb -= (zb >= G.n3 ? G.n3 : 0);
+         const float v0 = tz[kz].x, v1 = tz[kz].y, v2 = z2[kz];
+         float term0 = dot2(f0 * u0, v0, fy * u1, v0);
+         term0 = __fmaf_rn(fz * u0, v1, term0);
+         term0 = __fmaf_rn(fyy * u2, v0, term0);
+         term0 = __fmaf_rn(fzz * u0, v2, term0);
+         term0 = __fmaf_rn(fyz * u1, v1, term0);
+         const float term1 = __fmaf_rn(fxz * u0, v1, dot2(fx * u0, v0, fxy * u1, v0));
+         const float term2 = fxx * u0 * v0;
          grid_add(reinterpret_cast<unsigned long long*>(col + (size_t)(unsigned)zb * plane), 0,
-            c0 * tz[kz].x + c1 * tz[kz].y + c2 * z2[kz]);
+            __fmaf_rn(term2, x2, dot2(term0, tx.x, term1, tx.y)));
       }
    } else {
       pdl_wait();
@@ -302,15 +271,18 @@ __global__ void __launch_bounds__(256) k_spread(int n, GridParams G, Sites S, co
          dir_row(src, z8, s, (float)scal[S_B_D], (float)scal[S_B_P], u);
       else
          load8(src, s, u);
-      const float d0 = G.a1 * u[0] * x1y + G.a2 * u[1] * xy1, d1 = G.a3 * u[2] * xy;
-      const float p0 = G.a1 * u[3] * x1y + G.a2 * u[4] * xy1, p1 = G.a3 * u[5] * xy;
+      const float dx = G.a1 * u[0], dy = G.a2 * u[1], dz = G.a3 * u[2];
+      const float px = G.a1 * u[3], py = G.a2 * u[4], pz = G.a3 * u[5];
       bool ok = true;
 #pragma unroll
       for (int kz = 0; kz < 5; ++kz) {
          int zb = o.z + kz;
          zb -= (zb >= G.n3 ? G.n3 : 0);
+         const float v0 = tz[kz].x, v1 = tz[kz].y;
+         const float d01 = dot2(dy * u1, v0, dz * u0, v1), d11 = dx * u0 * v0;
+         const float p01 = dot2(py * u1, v0, pz * u0, v1), p11 = px * u0 * v0;
          ok &= grid_add2(reinterpret_cast<unsigned long long*>(col + (size_t)(unsigned)zb * plane),
-            d0 * tz[kz].x + d1 * tz[kz].y, p0 * tz[kz].x + p1 * tz[kz].y, G);
+            dot2(d01, tx.x, d11, tx.y), dot2(p01, tx.x, p11, tx.y), G);
       }
       if (!ok)
          atomicOr(G.range, 1);
@@ -386,10 +358,12 @@ __device__ __forceinline__ int sum_slot(int lane)
 }
 
 // Gather of the first potential derivatives fused with the recip + self
-// field, one warp per atom: lane (ix, jy) < 25 reads one column of five z
-// points, so that each of a warp's five loads covers five rows of five
-// consecutive points (about six 128-byte lines; one lane per row touched 25
-// lines in each load), and the columns are combined by warp_sums.  MODE 0:
+// field, one warp per atom.  The points are loaded as lane (ix, jy) < 25
+// taking a column of five z points, so that each of a warp's five loads
+// covers five rows of five consecutive points (about six 128-byte lines; a
+// lane per row touches 25 lines in each load and was bound by them), then
+// exchanged through shared memory: lane (jy, kz) sums one row of five x
+// points, and a fixed xor tree combines the rows (warp_sums).  MODE 0:
 // real part -> d and p field, self term with the permanent dipole.  MODE 1:
 // real -> d, imaginary -> p, self term with the induced dipoles.  Plain
 // stores, rows of 8 floats.
@@ -404,7 +378,7 @@ __device__ __forceinline__ int sum_slot(int lane)
 template <int MODE, bool ACC, bool AP, bool DIR, bool LATE = false>
 __device__ __forceinline__ void gather_atom(int s, int lane, const GridParams& G, const Sites& S,
    const float2* __restrict__ g, const float* __restrict__ rp, const float* __restrict__ u8, float* __restrict__ out,
-   const PcgAp& P, float bd, float bp, float* pap)
+   const PcgAp& P, float bd, float bp, float* pap, float2* xch)
 {
    constexpr int NC = MODE == 1 ? 6 : 3;
    float acc[NC];
@@ -413,20 +387,21 @@ __device__ __forceinline__ void gather_atom(int s, int lane, const GridParams& G
       acc[c] = 0.f;
    const int4 o = S.org[s];
    const float* lo = S.lo + (size_t)SPL_ROW * s;
-   const int ix = lane % 5, jy = lane / 5;
-   float2 tx, ty, t3[5];
+   const int q5 = lane % 5, d5 = lane / 5;  // (ix, jy) loading, (jy, kz) summing
+   float2 tx[5], ty, tz;
    if (lane < 25) {
-      tx = spl(lo, 0, ix);
-      ty = spl(lo, 1, jy);
 #pragma unroll
       for (int k = 0; k < 5; ++k)
-         t3[k] = spl(lo, 2, k);
+         tx[k] = spl(lo, 0, k);
+      ty = spl(lo, 1, q5);
+      tz = spl(lo, 2, d5);
    }
    if (LATE)
       pdl_wait();
+   float* xr = reinterpret_cast<float*>(xch);
    if (lane < 25) {
       const unsigned plane = plane_bytes(G);
-      const char* col = reinterpret_cast<const char*>(g) + column_bytes(G, o, ix, jy);
+      const char* col = reinterpret_cast<const char*>(g) + column_bytes(G, o, q5, d5);
       float2 q[5];
 #pragma unroll
       for (int kz = 0; kz < 5; ++kz) {
@@ -438,26 +413,42 @@ __device__ __forceinline__ void gather_atom(int s, int lane, const GridParams& G
          else
             q[kz].x = p->x;
       }
-      float r0 = 0.f, r1 = 0.f, m0 = 0.f, m1 = 0.f;
 #pragma unroll
-      for (int kz = 0; kz < 5; ++kz) {
-         r0 += q[kz].x * t3[kz].x;
-         r1 += q[kz].x * t3[kz].y;
+      for (int kz = 0; kz < 5; ++kz)
+         if (MODE == 1)
+            xch[25 * kz + lane] = q[kz];
+         else
+            xr[25 * kz + lane] = q[kz].x;
+   }
+   __syncwarp();
+   if (lane < 25) {
+      // row (jy, kz) = 5 lane .. 5 lane + 4 of the exchanged points
+      float rt0 = 0.f, rt1 = 0.f, it0 = 0.f, it1 = 0.f;
+#pragma unroll
+      for (int ix = 0; ix < 5; ++ix) {
+         float2 qv;
+         if (MODE == 1)
+            qv = xch[5 * lane + ix];
+         else
+            qv.x = xr[5 * lane + ix];
+         rt0 += qv.x * tx[ix].x;
+         rt1 += qv.x * tx[ix].y;
          if (MODE == 1) {
-            m0 += q[kz].y * t3[kz].x;
-            m1 += q[kz].y * t3[kz].y;
+            it0 += qv.y * tx[ix].x;
+            it1 += qv.y * tx[ix].y;
          }
       }
-      const float x1y = tx.y * ty.x, xy1 = tx.x * ty.y, xy = tx.x * ty.x;
-      acc[0] = r0 * x1y;
-      acc[1] = r0 * xy1;
-      acc[2] = r1 * xy;
+      const float u0 = ty.x, u1 = ty.y, v0 = tz.x, v1 = tz.y;
+      acc[0] = rt1 * u0 * v0;
+      acc[1] = rt0 * u1 * v0;
+      acc[2] = rt0 * u0 * v1;
       if (MODE == 1) {
-         acc[NC - 3] = m0 * x1y;
-         acc[NC - 2] = m0 * xy1;
-         acc[NC - 1] = m1 * xy;
+         acc[NC - 3] = it1 * u0 * v0;
+         acc[NC - 2] = it0 * u1 * v0;
+         acc[NC - 1] = it0 * u0 * v1;
       }
    }
+   __syncwarp();  // the exchange buffer is free for the warp's next atom
    const float sum = warp_sums<NC>(acc, lane);
    const int c = sum_slot<NC>(lane);
    if (c < 0)
@@ -496,6 +487,7 @@ __global__ void __launch_bounds__(256, 6) k_gather_field(int n, GridParams G, Si
 {
    // the plain gather waits inside gather_atom, after its position-only prologue
    constexpr bool LATE = !AP && !DIR;
+   __shared__ float2 xch[8][125];
    if (!LATE)
       pdl_wait();
    const int lane = threadIdx.x & 31;
@@ -507,7 +499,7 @@ __global__ void __launch_bounds__(256, 6) k_gather_field(int n, GridParams G, Si
          bp = (float)P.scal[S_B_P];
       }
       if (s < n)
-         gather_atom<MODE, ACC, false, DIR, LATE>(s, lane, G, S, g, rp, u8, out, P, bd, bp, nullptr);
+         gather_atom<MODE, ACC, false, DIR, LATE>(s, lane, G, S, g, rp, u8, out, P, bd, bp, nullptr, xch[threadIdx.x >> 5]);
       else if (LATE)
          pdl_wait();
       return;
@@ -517,7 +509,7 @@ __global__ void __launch_bounds__(256, 6) k_gather_field(int n, GridParams G, Si
    float pap[2] = {0.f, 0.f};
    const int nw = (gridDim.x * blockDim.x) >> 5;
    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < n; s += nw)
-      gather_atom<MODE, ACC, true, false>(s, lane, G, S, g, rp, u8, out, P, bd, bp, pap);
+      gather_atom<MODE, ACC, true, false>(s, lane, G, S, g, rp, u8, out, P, bd, bp, pap, xch[threadIdx.x >> 5]);
    store_partials_f<2>(P.red, R_PAP_D, pap, sh);
    if (!last_block(P.state + ST_TICKET1))
       return;

@@ -8,29 +8,45 @@
 
 namespace t9gb {
 
-// Piece j of the cardinal B-spline M5 and its first three derivatives at
-// the site's fraction w, as polynomials.  M5 is even about its centre: the
-// first two pieces are the last two at t = 1 - w with the odd derivatives'
-// sign flipped, so there is no cancellation at either end.  Coefficients
-// x 24: centre 11 + 12 t - 6 t^2 - 12 t^3 + 6 t^4, next 1 + 4 t + 6 t^2 +
-// 4 t^3 - 4 t^4, edge t^4.
-template <int J>
-__device__ __forceinline__ void spline_piece(float w, float* th)
+// weights and derivatives of the five points of one axis at fraction w
+template <int LEVEL>
+__device__ __forceinline__ void bspline5(float w, float th[5][LEVEL])
 {
-   constexpr bool mid = J == 2, edge = J == 0 || J == 4, mirror = J < 2;
-   constexpr float q = 1.f / 24.f;
-   constexpr float c0 = mid ? 11.f * q : edge ? 0.f : q;
-   constexpr float c1 = mid ? 12.f * q : edge ? 0.f : 4.f * q;
-   constexpr float c2 = mid ? -6.f * q : edge ? 0.f : 6.f * q;
-   constexpr float c3 = mid ? -12.f * q : edge ? 0.f : 4.f * q;
-   constexpr float c4 = mid ? 6.f * q : edge ? q : -4.f * q;
-   const float t = mirror ? 1.f - w : w;
-   th[0] = __fmaf_rn(__fmaf_rn(__fmaf_rn(__fmaf_rn(c4, t, c3), t, c2), t, c1), t, c0);
-   const float d1 = __fmaf_rn(__fmaf_rn(__fmaf_rn(4.f * c4, t, 3.f * c3), t, 2.f * c2), t, c1);
-   th[1] = mirror ? -d1 : d1;
-   th[2] = __fmaf_rn(__fmaf_rn(12.f * c4, t, 6.f * c3), t, 2.f * c2);
-   const float d3 = __fmaf_rn(24.f * c4, t, 6.f * c3);
-   th[3] = mirror ? -d3 : d3;
+   float b[6][6];  // b[order][i], 1-based
+   b[2][2] = w;
+   b[2][1] = 1.f - w;
+   b[3][3] = 0.5f * w * b[2][2];
+   b[3][2] = 0.5f * ((1.f + w) * b[2][1] + (2.f - w) * b[2][2]);
+   b[3][1] = 0.5f * (1.f - w) * b[2][1];
+#pragma unroll
+   for (int i = 4; i <= 5; ++i) {
+      const int k = i - 1;
+      const float denom = 1.f / k;
+      b[i][i] = denom * w * b[k][k];
+#pragma unroll
+      for (int j = 1; j <= i - 2; ++j)
+         b[i][i - j] = denom * ((w + j) * b[k][i - j - 1] + (i - j - w) * b[k][i - j]);
+      b[i][1] = denom * (1.f - w) * b[k][1];
+   }
+   // derivative rows by repeated differencing of the lower-order rows
+#pragma unroll
+   for (int lv = 2; lv <= LEVEL; ++lv) {
+      const int k = 5 - lv + 1;
+#pragma unroll
+      for (int pass = 0; pass < lv - 1; ++pass) {
+         const int top = 5 - (lv - 2) + pass;
+         b[k][top] = b[k][top - 1];
+#pragma unroll
+         for (int i = top - 1; i >= 2; --i)
+            b[k][i] = b[k][i - 1] - b[k][i];
+         b[k][1] = -b[k][1];
+      }
+   }
+#pragma unroll
+   for (int i = 1; i <= 5; ++i)
+#pragma unroll
+      for (int j = 1; j <= LEVEL; ++j)
+         th[i - 1][j - 1] = b[5 - j + 1][i];
 }
 
 // Rows of the tables, 32 floats (128 bytes) per slot: point j of axis a at
@@ -55,11 +71,7 @@ __device__ __forceinline__ int spline_axis(float x, float rbox, int nfft, int ax
    i -= BSORDER - 1;
    i += (i < 0 ? nfft : 0);
    float th[5][4];
-   spline_piece<0>(w, th[0]);
-   spline_piece<1>(w, th[1]);
-   spline_piece<2>(w, th[2]);
-   spline_piece<3>(w, th[3]);
-   spline_piece<4>(w, th[4]);
+   bspline5<4>(w, th);
    float2* l = reinterpret_cast<float2*>(lo) + 5 * axis;
    float2* h = reinterpret_cast<float2*>(hi) + 5 * axis;
 #pragma unroll
