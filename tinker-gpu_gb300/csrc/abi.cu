@@ -36,6 +36,7 @@ static int alloc_all(Context* ctx)
    T9_CUDA(cudaMalloc(&ctx->spolar, sizeof(float) * npad));
    T9_CUDA(cudaMalloc(&ctx->spolinv, sizeof(float) * npad));
    T9_CUDA(cudaMalloc(&ctx->sdamp, sizeof(float2) * npad));
+   T9_CUDA(cudaMalloc(&ctx->stag, sizeof(float2) * npad));
    T9_CUDA(cudaMalloc(&ctx->srpole, sizeof(float) * 12 * npad));
    T9_CUDA(cudaMemset(ctx->srpole, 0, sizeof(float) * 12 * npad));
    T9_CUDA(cudaMalloc(&ctx->exfld, sizeof(float) * 4));
@@ -101,6 +102,7 @@ static void free_all(Context* ctx)
 {
    void* dev[] = {ctx->frames, ctx->pole, ctx->xyz, ctx->perm, ctx->iperm, ctx->spos, ctx->spolar, ctx->spolinv,
       ctx->sdamp, ctx->srpole, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->nbr, ctx->nnbr, ctx->nbr_over, ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp,
+      ctx->stag, ctx->cfu, ctx->cfd, ctx->cfp, ctx->spu, ctx->spp,
       ctx->jbl, ctx->jbn, ctx->nbrc_l, ctx->nbrp_l, ctx->copy_err,
       ctx->cell_count, ctx->cell_start, ctx->cell_atoms, ctx->atom_cell, ctx->rcp6, ctx->fld6, ctx->udir,
       ctx->efield, ctx->uind, ctx->rsd, ctx->zrsd, ctx->conj, ctx->vec, ctx->tmp6, ctx->e_atom, ctx->sframe, ctx->hout,
@@ -600,8 +602,10 @@ int t9gb_pair_lanes(t9gb_context* h, int lanes)
 {
    if (!h || (lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32))
       return T9GB_BAD_ARG;
-   if (lanes != h->c.pair_lanes)
+   if (lanes != h->c.pair_lanes) {
       drop_graphs(&h->c);
+      h->c.list_stale = true;  // the sub-lists are tiled for the lane count
+   }
    h->c.pair_lanes = lanes;
    return T9GB_OK;
 }

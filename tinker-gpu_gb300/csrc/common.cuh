@@ -74,6 +74,32 @@ __device__ __forceinline__ void load8(const float* __restrict__ a, int s, float*
    v[7] = y.w;
 }
 
+// the same row in one 256-bit load (one L1 access per row where two 16-byte
+// loads make two); not before the wait for the kernel that wrote it
+__device__ __forceinline__ void load8_wide(const float* a, int s, float* v)
+{
+   asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                : "l"(a + 8 * (size_t)s));
+}
+
+// A per-slot list of up to cap entries (a multiple of 32), stored by tiles of
+// 32 / G atoms, G = 2^sg lanes per atom: entry k of slot i lies where lane
+// k % G of the atom, in a warp that walks the tile's atoms together, reads
+// it on trip k / G, so each trip of the warp is 32 consecutive entries.
+// sg = 5 is one row after the other.
+struct ListView {
+   const int* p;
+   int cap, sg;
+   __host__ __device__ __forceinline__ size_t at(int i, int k) const
+   {
+      const int sw = 5 - sg;
+      return (((size_t)(i >> sw) * cap) << sw) + ((size_t)(k >> sg) << 5) + ((i & ((1 << sw) - 1)) << sg) +
+         (k & ((1 << sg) - 1));
+   }
+   __device__ __forceinline__ int operator()(int i, int k) const { return p[at(i, k)]; }
+};
+
 struct PmeGrid {
    int n1 = 0, n2 = 0, n3 = 0;
    bool own_fft = false;      // power-of-two grid: the library's fused FFT path
@@ -249,6 +275,7 @@ struct Context {
    float* spolar = nullptr;  // [npad] polarizability (0 on padding)
    float* spolinv = nullptr; // [npad] 1/max(alpha, 1e-16)
    float2* sdamp = nullptr;  // [npad] pdamp, thole
+   float2* stag = nullptr;   // [npad] thole (or type), polarizability
    float* srpole = nullptr;  // [npad][12] global-frame multipoles, thole, polarizability
    float* sframe = nullptr;  // [npad][9] local multipole frame (rows: x, y, z axes)
 
@@ -269,6 +296,15 @@ struct Context {
    int* nnbrc = nullptr;
    int* nbrp = nullptr;
    int* nnbrp = nullptr;
+   int list_lanes = 32;      // lanes per atom the sub-lists were tiled for (ListView)
+   // radial factors of every sub-list entry, formed by the filter: (b1, b2)
+   // of the mutual field and (b2, b3) of the permanent one (nbrc), (c1, c2)
+   // of the preconditioner (nbrp); and those of the scaled partners
+   float2* cfu = nullptr;    // [npad][nbr_cap], tiled
+   float2* cfd = nullptr;
+   float2* cfp = nullptr;
+   float2* spu = nullptr;    // [nsp] mutual field
+   float2* spp = nullptr;    // [nsp] preconditioner
    // staged field / preconditioner kernels (t9gb_pair_staging): per 32-slot
    // block the j-blocks its sub-list entries fall in (ascending, at most
    // STAGE_JB_CAP; jbn > cap means the block reads rows from global memory),
@@ -533,6 +569,14 @@ inline void prof_collect(Context* ctx)
    }
    p.used = 0;
 }
+
+// the cutoff sub-list, and the stored list, as views
+inline ListView nbrc_view(const Context* ctx)
+{
+   const int g = ctx->list_lanes;
+   return {ctx->nbrc, ctx->nbr_cap, g == 4 ? 2 : g == 8 ? 3 : g == 16 ? 4 : 5};
+}
+inline ListView nbr_view(const Context* ctx) { return {ctx->nbr, ctx->nbr_cap, 5}; }
 
 // ---- entry points implemented across the translation units ----
 int order_build(Context* ctx);  // host: spatial order, scaled partners

@@ -330,7 +330,7 @@ __device__ __forceinline__ void elec_pair(const PairParams& P, float3 Rv, float 
 // the scaled partners.  f: electric; outputs per slot: force [npad][3],
 // torque field [npad][10], empole real energy (MPOLE).
 template <int G, bool MPOLE, bool POLAR, bool VIR>
-__global__ void __launch_bounds__(128) k_elec_real(PairParams P, int npad, float f, const int* __restrict__ nbr,
+__global__ void __launch_bounds__(128) k_elec_real(PairParams P, int npad, float f, ListView nbr,
    const int* __restrict__ nnbr, const int* __restrict__ sp_start, const int* __restrict__ sp_j,
    const float4* __restrict__ sp_sc, const float4* __restrict__ spos, const float* __restrict__ rp,
    const float* __restrict__ u8, float* __restrict__ fout, float* __restrict__ tout, double* __restrict__ e_atom,
@@ -357,10 +357,9 @@ __global__ void __launch_bounds__(128) k_elec_real(PairParams P, int npad, float
       if (POLAR)
          load8(u8, i, ui);
       const float pti = rp[12 * i + 10];
-      const int* row = nbr + (size_t)i * P.cap;
       const int cnt = nnbr[i];
       for (int k = g; k < cnt; k += G) {
-         const int j = row[k];
+         const int j = nbr(i, k);
          const float4 pk = spos[j];
          const float3 d = sep(P, pi, pk);
          const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
@@ -719,7 +718,7 @@ template <int G, bool MPOLE, bool POLAR, bool VIR>
 static void launch_real_g(Context* ctx, const PairParams& P, float f)
 {
    const int grid = grid_for((long long)ctx->npad * G, 128);
-   k_elec_real<G, MPOLE, POLAR, VIR><<<grid, 128, 0, ctx->stream>>>(P, ctx->npad, f, ctx->nbrc, ctx->nnbrc,
+   k_elec_real<G, MPOLE, POLAR, VIR><<<grid, 128, 0, ctx->stream>>>(P, ctx->npad, f, nbrc_view(ctx), ctx->nnbrc,
       ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos, ctx->srpole, ctx->uind, ctx->freal, ctx->treal,
       MPOLE ? ctx->e_atom : nullptr, ctx->wvir);
 }

@@ -63,6 +63,11 @@ int alloc_lists(Context* ctx, int cap)
       *p = nullptr;
       T9_CUDA(cudaMalloc(p, sizeof(int) * (size_t)ctx->npad * cap));
    }
+   for (float2** p : {&ctx->cfu, &ctx->cfd, &ctx->cfp}) {
+      cudaFree(*p);
+      *p = nullptr;
+      T9_CUDA(cudaMalloc(p, sizeof(float2) * (size_t)ctx->npad * cap));
+   }
    for (unsigned short** p : {&ctx->nbrc_l, &ctx->nbrp_l}) {
       cudaFree(*p);
       *p = nullptr;
@@ -227,7 +232,10 @@ int order_build(Context* ctx)
    cudaFree(ctx->sp_j);
    cudaFree(ctx->sp_sc);
    cudaFree(ctx->sp_v);
+   cudaFree(ctx->spu);
+   cudaFree(ctx->spp);
    ctx->sp_v = nullptr;
+   ctx->spu = ctx->spp = nullptr;
    cudaFree(ctx->cell_count);
    cudaFree(ctx->cell_start);
    ctx->perm = ctx->iperm = ctx->sp_start = ctx->sp_j = ctx->cell_count = ctx->cell_start = nullptr;
@@ -238,6 +246,8 @@ int order_build(Context* ctx)
    T9_CUDA(cudaMalloc(&ctx->sp_j, sizeof(int) * std::max(1, ctx->nsp)));
    T9_CUDA(cudaMalloc(&ctx->sp_sc, sizeof(float4) * std::max(1, ctx->nsp)));
    T9_CUDA(cudaMalloc(&ctx->sp_v, sizeof(float) * std::max(1, ctx->nsp)));
+   T9_CUDA(cudaMalloc(&ctx->spu, sizeof(float2) * std::max(1, ctx->nsp)));
+   T9_CUDA(cudaMalloc(&ctx->spp, sizeof(float2) * std::max(1, ctx->nsp)));
    T9_CUDA(cudaMemcpy(ctx->perm, ctx->h_perm.data(), sizeof(int) * npad, cudaMemcpyHostToDevice));
    T9_CUDA(cudaMemcpy(ctx->iperm, ctx->h_iperm.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
    T9_CUDA(cudaMemcpy(ctx->sp_start, sp_start.data(), sizeof(int) * (npad + 1), cudaMemcpyHostToDevice));
@@ -249,6 +259,9 @@ int order_build(Context* ctx)
    T9_CUDA(cudaMemcpy(ctx->spolar, pol.data(), sizeof(float) * npad, cudaMemcpyHostToDevice));
    T9_CUDA(cudaMemcpy(ctx->spolinv, pinv.data(), sizeof(float) * npad, cudaMemcpyHostToDevice));
    T9_CUDA(cudaMemcpy(ctx->sdamp, dmp.data(), sizeof(float2) * npad, cudaMemcpyHostToDevice));
+   for (int s = 0; s < npad; ++s)
+      dmp[s] = make_float2(dmp[s].y, pol[s]);
+   T9_CUDA(cudaMemcpy(ctx->stag, dmp.data(), sizeof(float2) * npad, cudaMemcpyHostToDevice));
    if (ctx->use_cells) {
       T9_CUDA(cudaMalloc(&ctx->cell_count, sizeof(int) * ctx->ncell));
       T9_CUDA(cudaMalloc(&ctx->cell_start, sizeof(int) * (ctx->ncell + 1)));

@@ -59,135 +59,197 @@ __device__ __forceinline__ float pick6(const float* f, int g)
    return v;
 }
 
-// lane g of a group of G stores components g, g + G, ... < 6: out = base + f
-template <int G>
-__device__ __forceinline__ void store6(float* __restrict__ out, const float* __restrict__ base, int s, int g,
-   const float* f)
+// The six sums of a group of G lanes: fn(c, sum) for the components c = g,
+// g + G, ... < 6 that lane g of the group finishes.  Sums in the order of an
+// xor tree, farthest lanes first; for G = 8 by the halving tree (the same
+// additions in 7 shuffles where six trees take 18).
+template <int G, class F>
+__device__ __forceinline__ void for_own6(float* f, F&& fn)
 {
+   const int lane = threadIdx.x & 31, g = lane & (G - 1);
+   if constexpr (G == 8) {
+      const float v = warp_sums<6, 4>(f, lane);
+      // components 0-2 sit in lanes 0-2 of the group, 3-5 in lanes 4-6
+      const float w = __shfl_sync(0xffffffffu, v, (lane & 24) | (g < 3 ? g : (g + 1) & 7));
+      if (g < 6)
+         fn(g, w);
+   } else {
+      group_reduce<G, 6>(f);
 #pragma unroll
-   for (int c0 = 0; c0 < 6; c0 += G) {
-      const int c = c0 + g;
-      if (c < 6) {
-         float v = pick6(f, c);
-         if (base)
-            v += base[8 * s + c];
-         out[8 * s + c] = v;
+      for (int c0 = 0; c0 < 6; c0 += G) {
+         const int c = c0 + g;
+         if (c < 6)
+            fn(c, pick6(f, c));
       }
    }
 }
 
 // ---------------------------------------------------------------------------
-// mutual field -T u, i side (pair_ufield_v2)
+// Dipole tensor rows.  The mutual field -T u (pair_ufield_v2) and the sparse
+// preconditioner's off-diagonal part have one form,
+//   f_i = sum_k [ c2 (d . v_k) d - c1 v_k ],  d = r_k - r_i,
+// and their radial factors (c1, c2) depend on the positions only: the filter
+// forms them once per position update for every listed pair, and a solve of
+// m iterations reads them 2 m + 2 times.  A pair then costs an index, 8 bytes
+// of factors, one position and one row, and about 40 instructions (the
+// kernels that formed the factors in place spent 168 per pair and waited on
+// the transcendental chain).  The sub-lists and factors are stored by tiles of
+// 32 / G atoms (ListView), so that a warp's index load is one 128-byte line
+// and its factor load two; the neighbour's row is one 32-byte load.  What
+// bounds the rows is the L1's rate of one line per cycle (83% of it at 98,304
+// atoms, 4 lanes: 1 + 2 + 11 + 14 lines for 32 pairs, 47 before).  GB300, ncu,
+// 12,288 / 98,304 atoms: mutual field 20.6 -> 16.0 / 97 -> 76 us,
+// preconditioner 20.5 -> 15.8 / 82 -> 63, permanent field 26.3 -> 18.9 /
+// 120 -> 94, filter 23 -> 33 / 118 -> 211 (once per position update).
 
-__device__ __forceinline__ void ufield_i(const PairParams& P, float r2, float3 d, float uscale, float pdi, float pti,
-   float pdk, float ptk, const float* uk, float* f)
+// a sub-list with its factors, tiled (ListView) for the kernels' lane count:
+// counts per slot, indices, factors, and the factors of the scaled partners
+struct TensorList {
+   const int *nbr, *cnt;
+   const float2 *coef, *spc;
+};
+
+// scaled partners of every slot (CSR)
+struct Partners {
+   const int *start, *j;
+};
+
+// slot i's first entry in a tiled list of G lanes per atom
+template <int G>
+__device__ __forceinline__ size_t tile_at(int cap, int i)
 {
-   float invr = rsqrtf(r2);
-   float r = r2 * invr;
-   float rr2 = invr * invr;
-   float rr3 = invr * rr2;
-   float rr5 = 3.f * rr3 * rr2;
-   float s3, s5, s7;
-   thole_damp(r, pdi, pair_gamma(P, pti, ptk), pdk, s3, s5, s7);
-   float b1, b2;
-   if (P.ewald) {
-      float e1, e2, e3;
-      ewald_bn(P, r, invr, rr2, e1, e2, e3);
-      b1 = e1 - (1.f - uscale * s3) * rr3;
-      b2 = e2 - (1.f - uscale * s5) * rr5;
-   } else {
-      b1 = uscale * s3 * rr3;
-      b2 = uscale * s5 * rr5;
+   constexpr int W = 32 / G;
+   return (size_t)(i / W) * W * cap + (i % W) * G;
+}
+
+__device__ __forceinline__ void tensor_add(float3 d, float2 c, const float* v, float* f)
+{
+   float q = c.y * (d.x * v[0] + d.y * v[1] + d.z * v[2]);
+   f[0] += q * d.x - c.x * v[0];
+   f[1] += q * d.y - c.x * v[1];
+   f[2] += q * d.z - c.x * v[2];
+   q = c.y * (d.x * v[3] + d.y * v[4] + d.z * v[5]);
+   f[3] += q * d.x - c.x * v[3];
+   f[4] += q * d.y - c.x * v[4];
+   f[5] += q * d.z - c.x * v[5];
+}
+
+// list entries and factors: read once per application, kept out of L1 so
+// that the neighbours' positions and rows stay there
+__device__ __forceinline__ int stream_index(const int* p)
+{
+   int v;
+   asm volatile("ld.global.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+   return v;
+}
+
+__device__ __forceinline__ int stream_index(const unsigned short* p) { return *p; }
+
+__device__ __forceinline__ float2 stream_coef(const float2* p)
+{
+   float2 v;
+   asm volatile("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+   return v;
+}
+
+// neighbour j's position and row from global memory; DIR: the row is the CG
+// search direction p = z + b p_old, formed as it is read
+template <bool DIR>
+struct GlobalRows {
+   const float4* spos;
+   const float *u8, *z8;
+   float bd, bp;
+   __device__ __forceinline__ void get(int j, float4& p, float* v) const
+   {
+      p = spos[j];
+      if (DIR)
+         dir_row(u8, z8, j, bd, bp, v);
+      else
+         load8_wide(u8, j, v);
    }
-   float c = b2 * (d.x * uk[0] + d.y * uk[1] + d.z * uk[2]);
-   f[0] += c * d.x - b1 * uk[0];
-   f[1] += c * d.y - b1 * uk[1];
-   f[2] += c * d.z - b1 * uk[2];
-   c = b2 * (d.x * uk[3] + d.y * uk[4] + d.z * uk[5]);
-   f[3] += c * d.x - b1 * uk[3];
-   f[4] += c * d.y - b1 * uk[4];
-   f[5] += c * d.z - b1 * uk[5];
+};
+
+// the row sum of one atom's lane g of G: two entries per trip, both sets of
+// loads in flight together, the next trip's indices loaded ahead.  ip, cp:
+// the lane's first index and factors; is: index stride from one entry of the
+// lane to the next (factors: 32)
+template <int G, class IDX, class R>
+__device__ __forceinline__ void tensor_row(const PairParams& P, const IDX* __restrict__ ip, int is,
+   const float2* __restrict__ cp, int cnt, int g, float4 pi, const R& rows, float* f)
+{
+   int k = g;
+   int j0 = k < cnt ? stream_index(ip) : 0;
+   int j1 = k + G < cnt ? stream_index(ip + is) : 0;
+   while (k + G < cnt) {
+      const float2 c0 = stream_coef(cp), c1 = stream_coef(cp + 32);
+      float4 p0, p1;
+      float u0[8], u1[8];
+      rows.get(j0, p0, u0);
+      rows.get(j1, p1, u1);
+      k += 2 * G;
+      ip += 2 * is;
+      cp += 64;
+      j0 = k < cnt ? stream_index(ip) : 0;
+      j1 = k + G < cnt ? stream_index(ip + is) : 0;
+      tensor_add(sep(P, pi, p0), c0, u0, f);
+      tensor_add(sep(P, pi, p1), c1, u1, f);
+   }
+   if (k < cnt) {
+      const float2 c0 = stream_coef(cp);
+      float4 p0;
+      float u0[8];
+      rows.get(j0, p0, u0);
+      tensor_add(sep(P, pi, p0), c0, u0, f);
+   }
 }
 
-// DIR: the dipoles are the CG search direction p = z + b p_old, formed
-// from u8 = p_old, z8 and b (scal) as each row is read
-template <int G, bool DIR>
-__device__ __forceinline__ void urow(const float* __restrict__ u8, const float* __restrict__ z8, int j, float bd,
-   float bp, float* v)
+// the scaled partners of slot i (their factors are zero beyond the cutoff)
+template <int G, class R>
+__device__ __forceinline__ void tensor_partners(const PairParams& P, const Partners& S, const float2* __restrict__ spc,
+   int i, int g, float4 pi, const R& rows, float* f)
 {
-   if (DIR)
-      dir_row(u8, z8, j, bd, bp, v);
-   else
-      load8(u8, j, v);
+   const int pa = S.start[i], pb = S.start[i + 1];
+   for (int q = pa + g; q < pb; q += G) {
+      const float2 c = spc[q];
+      float4 p;
+      float u[8];
+      rows.get(S.j[q], p, u);
+      tensor_add(sep(P, pi, p), c, u, f);
+   }
+}
+
+// both, from global memory
+template <int G, class R>
+__device__ __forceinline__ void tensor_sum(const PairParams& P, const TensorList& T, const Partners& S, int i, int g,
+   const float4* __restrict__ spos, const R& rows, float* f)
+{
+   const float4 pi = spos[i];
+   const size_t at = tile_at<G>(P.cap, i) + g;
+   tensor_row<G>(P, T.nbr + at, 32, T.coef + at, T.cnt[i], g, pi, rows, f);
+   tensor_partners<G>(P, S, T.spc, i, g, pi, rows, f);
 }
 
 template <int G, bool DIR>
-__global__ void __launch_bounds__(256) k_ufield_real(PairParams P, int npad, const int* __restrict__ nbr,
-   const int* __restrict__ nnbr, const int* __restrict__ sp_start, const int* __restrict__ sp_j,
-   const float4* __restrict__ sp_sc, const float4* __restrict__ spos, const float* __restrict__ u8,
-   const float* __restrict__ z8, const double* __restrict__ scal, const float* __restrict__ base8,
-   float* __restrict__ out8)
+__global__ void __launch_bounds__(256) k_ufield_real(PairParams P, int npad, TensorList T, Partners S,
+   const float4* __restrict__ spos, const float* __restrict__ u8, const float* __restrict__ z8,
+   const double* __restrict__ scal, const float* __restrict__ base8, float* __restrict__ out8)
 {
-   pdl_wait();
    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
    const int i = tid / G, g = tid % G;
    if (i >= npad)
       return;
-   float bd = 0.f, bp = 0.f;
-   if (DIR) {
-      bd = (float)scal[S_B_D];
-      bp = (float)scal[S_B_P];
-   }
+   pdl_wait();
    float f[6] = {0, 0, 0, 0, 0, 0};
    if (i < P.n) {
-      const float4 pi = spos[i];  // w = pdamp
-      const float pti = u8[8 * i + 6];
-      const int* row = nbr + (size_t)i * P.cap;
-      const int cnt = nnbr[i];
-      int k = g;
-      // two neighbours per trip: both sets of loads are in flight together;
-      // each neighbour is one 16-byte position and one 32-byte row
-      for (; k + G < cnt; k += 2 * G) {
-         const int j0 = row[k], j1 = row[k + G];
-         const float4 p0 = spos[j0], p1 = spos[j1];
-         float u0[8], u1[8];
-         urow<G, DIR>(u8, z8, j0, bd, bp, u0);
-         urow<G, DIR>(u8, z8, j1, bd, bp, u1);
-         const float3 s0 = sep(P, pi, p0), s1 = sep(P, pi, p1);
-         const float r0 = s0.x * s0.x + s0.y * s0.y + s0.z * s0.z;
-         const float r1 = s1.x * s1.x + s1.y * s1.y + s1.z * s1.z;
-         if (r0 <= P.cut2)
-            ufield_i(P, r0, s0, 1.f, pi.w, pti, p0.w, u0[6], u0, f);
-         if (r1 <= P.cut2)
-            ufield_i(P, r1, s1, 1.f, pi.w, pti, p1.w, u1[6], u1, f);
+      GlobalRows<DIR> rows{spos, u8, z8, 0.f, 0.f};
+      if (DIR) {
+         rows.bd = (float)scal[S_B_D];
+         rows.bp = (float)scal[S_B_P];
       }
-      if (k < cnt) {
-         const int j = row[k];
-         const float4 pk = spos[j];
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         if (r2 <= P.cut2) {
-            float uk[8];
-            urow<G, DIR>(u8, z8, j, bd, bp, uk);
-            ufield_i(P, r2, d, 1.f, pi.w, pti, pk.w, uk[6], uk, f);
-         }
-      }
-      const int pa = sp_start[i], pb = sp_start[i + 1];
-      for (int q = pa + g; q < pb; q += G) {
-         const int j = sp_j[q];
-         const float4 pk = spos[j];
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         if (r2 <= P.cut2) {
-            float uk[8];
-            urow<G, DIR>(u8, z8, j, bd, bp, uk);
-            ufield_i(P, r2, d, sp_sc[q].w, pi.w, pti, pk.w, uk[6], uk, f);
-         }
-      }
+      tensor_sum<G>(P, T, S, i, g, spos, rows, f);
    }
    pdl_trigger();
-   group_reduce<G, 6>(f);
-   store6<G>(out8, i < P.n ? base8 : nullptr, i, g, f);
+   for_own6<G>(f, [&](int c, float v) { out8[8 * i + c] = base8 && i < P.n ? v + base8[8 * i + c] : v; });
 }
 
 // ---------------------------------------------------------------------------
@@ -264,9 +326,26 @@ __device__ __forceinline__ void load12(const float* __restrict__ rp, int s, floa
    }
 }
 
+// the field of multipole row mk at separation d with radial factors b1-b3
+__device__ __forceinline__ void mpole_field(float3 d, float b1, float b2, float b3, const float* mk, float* f)
+{
+   const float dkr = mk[1] * d.x + mk[2] * d.y + mk[3] * d.z;
+   const float qkx = mk[4] * d.x + mk[7] * d.y + mk[8] * d.z;
+   const float qky = mk[7] * d.x + mk[5] * d.y + mk[9] * d.z;
+   const float qkz = mk[8] * d.x + mk[9] * d.y + mk[6] * d.z;
+   const float qkr = qkx * d.x + qky * d.y + qkz * d.z;
+   const float c1 = -(b1 * mk[0] - b2 * dkr + b3 * qkr);
+   f[0] += c1 * d.x - b1 * mk[1] + 2.f * b2 * qkx;
+   f[1] += c1 * d.y - b1 * mk[2] + 2.f * b2 * qky;
+   f[2] += c1 * d.z - b1 * mk[3] + 2.f * b2 * qkz;
+}
+
+// the unscaled pairs, whose field is the same for both sets, with the
+// filter's radial factors (T.coef: b1; coefd: b2, b3), then the scaled
+// partners
 template <int G>
-__global__ void __launch_bounds__(256) k_dfield_real(PairParams P, int npad, const int* __restrict__ nbr,
-   const int* __restrict__ nnbr, const int* __restrict__ sp_start, const int* __restrict__ sp_j,
+__global__ void __launch_bounds__(256) k_dfield_real(PairParams P, int npad, TensorList T,
+   const float2* __restrict__ coefd, const int* __restrict__ sp_start, const int* __restrict__ sp_j,
    const float4* __restrict__ sp_sc, const float4* __restrict__ spos, const float* __restrict__ rp,
    const float* __restrict__ base8, const float* __restrict__ exfld, float* __restrict__ out8)
 {
@@ -278,151 +357,87 @@ __global__ void __launch_bounds__(256) k_dfield_real(PairParams P, int npad, con
    if (i < P.n) {
       const float4 pi = spos[i];
       const float pti = rp[12 * i + 10];
-      const int* row = nbr + (size_t)i * P.cap;
-      const int cnt = nnbr[i];
+      size_t at = tile_at<G>(P.cap, i) + g;
+      const int cnt = T.cnt[i];
+      int j = g < cnt ? stream_index(T.nbr + at) : 0;
       for (int k = g; k < cnt; k += G) {
-         const int j = row[k];
+         const float b1 = stream_coef(T.coef + at).x;
+         const float2 c = stream_coef(coefd + at);
          const float4 pk = spos[j];
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         if (r2 <= P.cut2) {
-            float mk[12];
-            load12(rp, j, mk);
-            dfield_i(P, r2, d, 1.f, 1.f, pi.w, pti, pk.w, mk[10], mk, f);
-         }
+         float mk[12];
+         load12(rp, j, mk);
+         at += 32;
+         j = k + G < cnt ? stream_index(T.nbr + at) : 0;
+         mpole_field(sep(P, pi, pk), b1, c.x, c.y, mk, f);
       }
+      f[3] = f[0];
+      f[4] = f[1];
+      f[5] = f[2];
       const int pa = sp_start[i], pb = sp_start[i + 1];
       for (int q = pa + g; q < pb; q += G) {
-         const int j = sp_j[q];
-         const float4 pk = spos[j];
+         const int jq = sp_j[q];
+         const float4 pk = spos[jq];
          const float3 d = sep(P, pi, pk);
          const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
          if (r2 <= P.cut2) {
             float mk[12];
-            load12(rp, j, mk);
+            load12(rp, jq, mk);
             const float4 sc = sp_sc[q];
             dfield_i(P, r2, d, sc.y, sc.z, pi.w, pti, pk.w, mk[10], mk, f);
          }
       }
    }
-   group_reduce<G, 6>(f);
-   if (i < P.n) {
-      // uniform external field on both sets (extfieldModifyDField_cu1,
-      // src/cu/amoeba/empole.cu:139-159); zero when none is set
-      const float e0 = exfld[0], e1 = exfld[1], e2 = exfld[2];
-      f[0] += e0;
-      f[1] += e1;
-      f[2] += e2;
-      f[3] += e0;
-      f[4] += e1;
-      f[5] += e2;
-   }
-   store6<G>(out8, i < P.n ? base8 : nullptr, i, g, f);
+   for_own6<G>(f, [&](int c, float v) {
+      if (i < P.n) {
+         // uniform external field on both sets (extfieldModifyDField_cu1,
+         // src/cu/amoeba/empole.cu:139-159); zero when none is set
+         v += exfld[c < 3 ? c : c - 3];
+         if (base8)
+            v += base8[8 * i + c];
+      }
+      out8[8 * i + c] = v;
+   });
 }
 
 // ---------------------------------------------------------------------------
-// sparse preconditioner: z_i = udiag alpha_i r_i + sum_k alpha_i alpha_k T_ik r_k
-
-__device__ __forceinline__ void precond_i(const PairParams& P, float r2, float3 d, float us, float poli, float pdi, float pti, float pdk,
-   const float* rk, float* f)
-{
-   const float polk = rk[7];
-   float invr = rsqrtf(r2);
-   float r = r2 * invr;
-   float s3, s5, s7;
-   thole_damp(r, pdi, pair_gamma(P, pti, rk[6]), pdk, s3, s5, s7);
-   const float polik = poli * polk;
-   const float ir3 = invr * invr * invr;
-   const float rr3 = us * s3 * polik * ir3;
-   const float rr5 = 3.f * us * s5 * polik * ir3 * invr * invr;
-   float c = rr5 * (d.x * rk[0] + d.y * rk[1] + d.z * rk[2]);
-   f[0] += c * d.x - rr3 * rk[0];
-   f[1] += c * d.y - rr3 * rk[1];
-   f[2] += c * d.z - rr3 * rk[2];
-   c = rr5 * (d.x * rk[3] + d.y * rk[4] + d.z * rk[5]);
-   f[3] += c * d.x - rr3 * rk[3];
-   f[4] += c * d.y - rr3 * rk[4];
-   f[5] += c * d.z - rr3 * rk[5];
-}
-
-// the preconditioner row of slot i: the off-diagonal sums f[6] (reduced
-// over the group); z_c = udiag alpha_i r_c + f_c
-template <int G>
-__device__ __forceinline__ void precond_row(const PairParams& P, int i, int g, float* f,
-   const int* __restrict__ nbr, const int* __restrict__ nnbr, const int* __restrict__ sp_start,
-   const int* __restrict__ sp_j, const float4* __restrict__ sp_sc, const float4* __restrict__ spos,
-   const float* __restrict__ r8)
-{
-#pragma unroll
-   for (int c = 0; c < 6; ++c)
-      f[c] = 0.f;
-   const float poli = r8[8 * i + 7];
-   if (i < P.n) {
-      const float4 pi = spos[i];
-      const float pti = r8[8 * i + 6];
-      const int* row = nbr + (size_t)i * P.cap;
-      const int cnt = nnbr[i];
-      int k = g;
-      for (; k + G < cnt; k += 2 * G) {
-         const int j0 = row[k], j1 = row[k + G];
-         const float4 p0 = spos[j0], p1 = spos[j1];
-         float r0v[8], r1v[8];
-         load8(r8, j0, r0v);
-         load8(r8, j1, r1v);
-         const float3 s0 = sep(P, pi, p0), s1 = sep(P, pi, p1);
-         const float q0 = s0.x * s0.x + s0.y * s0.y + s0.z * s0.z;
-         const float q1 = s1.x * s1.x + s1.y * s1.y + s1.z * s1.z;
-         if (q0 <= P.cut2)
-            precond_i(P, q0, s0, 1.f, poli, pi.w, pti, p0.w, r0v, f);
-         if (q1 <= P.cut2)
-            precond_i(P, q1, s1, 1.f, poli, pi.w, pti, p1.w, r1v, f);
-      }
-      if (k < cnt) {
-         const int j = row[k];
-         const float4 pk = spos[j];
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         if (r2 <= P.cut2) {
-            float rk[8];
-            load8(r8, j, rk);
-            precond_i(P, r2, d, 1.f, poli, pi.w, pti, pk.w, rk, f);
-         }
-      }
-      const int pa = sp_start[i], pb = sp_start[i + 1];
-      for (int q = pa + g; q < pb; q += G) {
-         const int j = sp_j[q];
-         const float4 pk = spos[j];
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         if (r2 <= P.cut2) {
-            float rk[8];
-            load8(r8, j, rk);
-            precond_i(P, r2, d, sp_sc[q].w, poli, pi.w, pti, pk.w, rk, f);
-         }
-      }
-   }
-   group_reduce<G, 6>(f);
-}
+// sparse preconditioner: z_i = udiag alpha_i r_i + sum_k alpha_i alpha_k T_ik r_k,
+// the filter's factors holding alpha_i alpha_k and the Thole damping
 
 template <int G>
 __global__ void __launch_bounds__(256) k_precond_sparse(PairParams P, int npad, float udiag,
-   const int* __restrict__ nbr, const int* __restrict__ nnbr, const int* __restrict__ sp_start,
-   const int* __restrict__ sp_j, const float4* __restrict__ sp_sc, const float4* __restrict__ spos,
-   const float* __restrict__ r8, float* __restrict__ z8)
+   TensorList T, Partners S, const float4* __restrict__ spos, const float* __restrict__ r8, float* __restrict__ z8)
 {
    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
    const int i = tid / G, g = tid % G;
    if (i >= npad)
       return;
-   float f[6];
-   precond_row<G>(P, i, g, f, nbr, nnbr, sp_start, sp_j, sp_sc, spos, r8);
+   float f[6] = {0, 0, 0, 0, 0, 0};
+   if (i < P.n)
+      tensor_sum<G>(P, T, S, i, g, spos, GlobalRows<false>{spos, r8, nullptr, 0.f, 0.f}, f);
    const float poli = r8[8 * i + 7];
-#pragma unroll
-   for (int c0 = 0; c0 < 6; c0 += G) {
-      const int c = c0 + g;
-      if (c < 6)
-         z8[8 * i + c] = udiag * poli * r8[8 * i + c] + pick6(f, c);
-   }
+   for_own6<G>(f, [&](int c, float v) { z8[8 * i + c] = udiag * poli * r8[8 * i + c] + v; });
+}
+
+// z = M r of slot i from its row sums: stored, with the r.z and r.r sums
+template <int G>
+__device__ __forceinline__ void precond_store(int i, float udiag, float* f, const float* __restrict__ r8,
+   float* __restrict__ z8, const PcgDots& D, float* dots)
+{
+   const float poli = r8[8 * i + 7];
+   for_own6<G>(f, [&](int c, float v) {
+      const float r = r8[8 * i + c];
+      const float z = udiag * poli * r + v;
+      z8[8 * i + c] = z;
+      if (D.init)
+         D.conj[8 * i + c] = z;
+      if (c < 3) {
+         dots[0] += r * z;
+         dots[2] += r * r;
+      } else {
+         dots[1] += r * z;
+         dots[3] += r * r;
+      }
+   });
 }
 
 // z = M r fused with the partial sums r.z, r.r (d and p) and, in the last
@@ -431,41 +446,23 @@ __global__ void __launch_bounds__(256) k_precond_sparse(PairParams P, int npad, 
 // the same trips); at most RED_MAX blocks.
 template <int G>
 __global__ void __launch_bounds__(256, 4) k_precond_sparse_dots(PairParams P, int npad, float udiag,
-   const int* __restrict__ nbr, const int* __restrict__ nnbr, const int* __restrict__ sp_start,
-   const int* __restrict__ sp_j, const float4* __restrict__ sp_sc, const float4* __restrict__ spos,
-   const float* __restrict__ r8, float* __restrict__ z8, PcgDots D)
+   TensorList T, Partners S, const float4* __restrict__ spos, const float* __restrict__ r8, float* __restrict__ z8,
+   PcgDots D)
 {
    pdl_wait();
    __shared__ double sh[64];
    constexpr int PER = 256 / G;
    const int g = threadIdx.x % G;
-   float rz_d = 0.f, rz_p = 0.f, rr_d = 0.f, rr_p = 0.f;
+   float dots[4] = {0.f, 0.f, 0.f, 0.f};
+   const GlobalRows<false> rows{spos, r8, nullptr, 0.f, 0.f};
    for (int i = blockIdx.x * PER + threadIdx.x / G; i < npad; i += gridDim.x * PER) {
-      float f[6];
-      precond_row<G>(P, i, g, f, nbr, nnbr, sp_start, sp_j, sp_sc, spos, r8);
-      const float poli = r8[8 * i + 7];
-#pragma unroll
-      for (int c0 = 0; c0 < 6; c0 += G) {
-         const int c = c0 + g;
-         if (c < 6) {
-            const float r = r8[8 * i + c];
-            const float z = udiag * poli * r + pick6(f, c);
-            z8[8 * i + c] = z;
-            if (D.init)
-               D.conj[8 * i + c] = z;
-            if (c < 3) {
-               rz_d += r * z;
-               rr_d += r * r;
-            } else {
-               rz_p += r * z;
-               rr_p += r * r;
-            }
-         }
-      }
+      float f[6] = {0, 0, 0, 0, 0, 0};
+      if (i < P.n)
+         tensor_sum<G>(P, T, S, i, g, spos, rows, f);
+      precond_store<G>(i, udiag, f, r8, z8, D, dots);
    }
-   const float pv[4] = {rz_d, rz_p, rr_d, rr_p};
    pdl_trigger();
-   store_partials_f<4>(D.red, R_RZ_D, pv, sh);
+   store_partials_f<4>(D.red, R_RZ_D, dots, sh);
    if (!last_block(D.state + ST_TICKET0))
       return;
    double tot[4];
@@ -518,28 +515,41 @@ __device__ __forceinline__ void stage_rows(unsigned char* stg, unsigned bar, uns
    mbar_wait_bounded(bar, phase);  // the copies in flight, before the buffers are reused
 }
 
-// neighbour row L from the staged buffers
-__device__ __forceinline__ void staged_row(const unsigned char* stg, int L, float4& p, float* v)
+// neighbour rows from the staged buffers, by local index
+struct StagedRows {
+   const unsigned char* stg;
+   __device__ __forceinline__ void get(int L, float4& p, float* v) const
+   {
+      p = reinterpret_cast<const float4*>(stg)[L];
+      const float4* r = reinterpret_cast<const float4*>(stg + STAGE_JB_CAP * STAGE_POS_BYTES) + 2 * L;
+      const float4 x = r[0], y = r[1];
+      v[0] = x.x;
+      v[1] = x.y;
+      v[2] = x.z;
+      v[3] = x.w;
+      v[4] = y.x;
+      v[5] = y.y;
+      v[6] = y.z;
+      v[7] = y.w;
+   }
+};
+
+// the list from the staged rows (nbr_l: the row's local indices), the scaled
+// partners from global memory
+template <int G>
+__device__ __forceinline__ void staged_sum(const PairParams& P, const TensorList& T, const Partners& S,
+   const unsigned short* __restrict__ nbr_l, int i, int g, const float4* __restrict__ spos, const StagedRows& stg,
+   const GlobalRows<false>& rows, float* f)
 {
-   p = reinterpret_cast<const float4*>(stg)[L];
-   const float4* r = reinterpret_cast<const float4*>(stg + STAGE_JB_CAP * STAGE_POS_BYTES) + 2 * L;
-   const float4 x = r[0], y = r[1];
-   v[0] = x.x;
-   v[1] = x.y;
-   v[2] = x.z;
-   v[3] = x.w;
-   v[4] = y.x;
-   v[5] = y.y;
-   v[6] = y.z;
-   v[7] = y.w;
+   const float4 pi = spos[i];
+   tensor_row<G>(P, nbr_l + (size_t)i * P.cap + g, G, T.coef + tile_at<G>(P.cap, i) + g, T.cnt[i], g, pi, stg, f);
+   tensor_partners<G>(P, S, T.spc, i, g, pi, rows, f);
 }
 
 template <int G>
-__global__ void __launch_bounds__(32 * G) k_ufield_stg(PairParams P, const int* __restrict__ nbr,
-   const unsigned short* __restrict__ nbr_l, const int* __restrict__ nnbr, const int* __restrict__ jbl,
-   const int* __restrict__ jbn, const int* __restrict__ sp_start, const int* __restrict__ sp_j,
-   const float4* __restrict__ sp_sc, const float4* __restrict__ spos, const float* __restrict__ u8,
-   const float* __restrict__ base8, float* __restrict__ out8, int* __restrict__ err)
+__global__ void __launch_bounds__(32 * G) k_ufield_stg(PairParams P, TensorList T, Partners S,
+   const unsigned short* __restrict__ nbr_l, const int* __restrict__ jbl, const int* __restrict__ jbn,
+   const float4* __restrict__ spos, const float* __restrict__ u8, const float* __restrict__ base8, float* __restrict__ out8, int* __restrict__ err)
 {
    pdl_wait();
    extern __shared__ __align__(128) unsigned char stg[];
@@ -556,134 +566,13 @@ __global__ void __launch_bounds__(32 * G) k_ufield_stg(PairParams P, const int* 
       stage_rows(stg, bar_s, 0, jbl + (size_t)blk * STAGE_JB_CAP, nj, spos, u8, err);
    }
    float f[6] = {0, 0, 0, 0, 0, 0};
-   if (i < P.n) {
-      const float4 pi = spos[i];
-      const float pti = u8[8 * i + 6];
-      const int cnt = nnbr[i];
-      int k = g;
-      if (staged) {
-         const unsigned short* row = nbr_l + (size_t)i * P.cap;
-         for (; k + G < cnt; k += 2 * G) {
-            float4 p0, p1;
-            float u0[8], u1[8];
-            staged_row(stg, row[k], p0, u0);
-            staged_row(stg, row[k + G], p1, u1);
-            const float3 s0 = sep(P, pi, p0), s1 = sep(P, pi, p1);
-            const float r0 = s0.x * s0.x + s0.y * s0.y + s0.z * s0.z;
-            const float r1 = s1.x * s1.x + s1.y * s1.y + s1.z * s1.z;
-            if (r0 <= P.cut2)
-               ufield_i(P, r0, s0, 1.f, pi.w, pti, p0.w, u0[6], u0, f);
-            if (r1 <= P.cut2)
-               ufield_i(P, r1, s1, 1.f, pi.w, pti, p1.w, u1[6], u1, f);
-         }
-         if (k < cnt) {
-            float4 pk;
-            float uk[8];
-            staged_row(stg, row[k], pk, uk);
-            const float3 d = sep(P, pi, pk);
-            const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-            if (r2 <= P.cut2)
-               ufield_i(P, r2, d, 1.f, pi.w, pti, pk.w, uk[6], uk, f);
-         }
-      } else {
-         const int* row = nbr + (size_t)i * P.cap;
-         for (; k + G < cnt; k += 2 * G) {
-            const int j0 = row[k], j1 = row[k + G];
-            const float4 p0 = spos[j0], p1 = spos[j1];
-            float u0[8], u1[8];
-            load8(u8, j0, u0);
-            load8(u8, j1, u1);
-            const float3 s0 = sep(P, pi, p0), s1 = sep(P, pi, p1);
-            const float r0 = s0.x * s0.x + s0.y * s0.y + s0.z * s0.z;
-            const float r1 = s1.x * s1.x + s1.y * s1.y + s1.z * s1.z;
-            if (r0 <= P.cut2)
-               ufield_i(P, r0, s0, 1.f, pi.w, pti, p0.w, u0[6], u0, f);
-            if (r1 <= P.cut2)
-               ufield_i(P, r1, s1, 1.f, pi.w, pti, p1.w, u1[6], u1, f);
-         }
-         if (k < cnt) {
-            const int j = row[k];
-            const float4 pk = spos[j];
-            const float3 d = sep(P, pi, pk);
-            const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-            if (r2 <= P.cut2) {
-               float uk[8];
-               load8(u8, j, uk);
-               ufield_i(P, r2, d, 1.f, pi.w, pti, pk.w, uk[6], uk, f);
-            }
-         }
-      }
-      const int pa = sp_start[i], pb = sp_start[i + 1];
-      for (int q = pa + g; q < pb; q += G) {
-         const int j = sp_j[q];
-         const float4 pk = spos[j];
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         if (r2 <= P.cut2) {
-            float uk[8];
-            load8(u8, j, uk);
-            ufield_i(P, r2, d, sp_sc[q].w, pi.w, pti, pk.w, uk[6], uk, f);
-         }
-      }
-   }
+   const GlobalRows<false> rows{spos, u8, nullptr, 0.f, 0.f};
+   if (i < P.n && staged)
+      staged_sum<G>(P, T, S, nbr_l, i, g, spos, StagedRows{stg}, rows, f);
+   else if (i < P.n)
+      tensor_sum<G>(P, T, S, i, g, spos, rows, f);
    pdl_trigger();
-   group_reduce<G, 6>(f);
-   store6<G>(out8, i < P.n ? base8 : nullptr, i, g, f);
-}
-
-// the preconditioner row of slot i, rows from the staged buffers
-template <int G>
-__device__ __forceinline__ void precond_row_stg(const PairParams& P, int i, int g, const unsigned char* stg, float* f,
-   const unsigned short* __restrict__ nbr_l, const int* __restrict__ nnbr, const int* __restrict__ sp_start,
-   const int* __restrict__ sp_j, const float4* __restrict__ sp_sc, const float4* __restrict__ spos,
-   const float* __restrict__ r8)
-{
-#pragma unroll
-   for (int c = 0; c < 6; ++c)
-      f[c] = 0.f;
-   const float poli = r8[8 * i + 7];
-   if (i < P.n) {
-      const float4 pi = spos[i];
-      const float pti = r8[8 * i + 6];
-      const unsigned short* row = nbr_l + (size_t)i * P.cap;
-      const int cnt = nnbr[i];
-      int k = g;
-      for (; k + G < cnt; k += 2 * G) {
-         float4 p0, p1;
-         float r0v[8], r1v[8];
-         staged_row(stg, row[k], p0, r0v);
-         staged_row(stg, row[k + G], p1, r1v);
-         const float3 s0 = sep(P, pi, p0), s1 = sep(P, pi, p1);
-         const float q0 = s0.x * s0.x + s0.y * s0.y + s0.z * s0.z;
-         const float q1 = s1.x * s1.x + s1.y * s1.y + s1.z * s1.z;
-         if (q0 <= P.cut2)
-            precond_i(P, q0, s0, 1.f, poli, pi.w, pti, p0.w, r0v, f);
-         if (q1 <= P.cut2)
-            precond_i(P, q1, s1, 1.f, poli, pi.w, pti, p1.w, r1v, f);
-      }
-      if (k < cnt) {
-         float4 pk;
-         float rk[8];
-         staged_row(stg, row[k], pk, rk);
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         if (r2 <= P.cut2)
-            precond_i(P, r2, d, 1.f, poli, pi.w, pti, pk.w, rk, f);
-      }
-      const int pa = sp_start[i], pb = sp_start[i + 1];
-      for (int q = pa + g; q < pb; q += G) {
-         const int j = sp_j[q];
-         const float4 pk = spos[j];
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         if (r2 <= P.cut2) {
-            float rk[8];
-            load8(r8, j, rk);
-            precond_i(P, r2, d, sp_sc[q].w, poli, pi.w, pti, pk.w, rk, f);
-         }
-      }
-   }
-   group_reduce<G, 6>(f);
+   for_own6<G>(f, [&](int c, float v) { out8[8 * i + c] = base8 && i < P.n ? base8[8 * i + c] + v : v; });
 }
 
 // z = M r with the r.z / r.r partial sums and, in the last block, the CG
@@ -692,10 +581,9 @@ __device__ __forceinline__ void precond_row_stg(const PairParams& P, int i, int 
 // staging mbarrier's phase flipping with each staged pass.
 template <int G>
 __global__ void __launch_bounds__(32 * G) k_precond_dots_stg(PairParams P, int nblk, float udiag,
-   const int* __restrict__ nbr, const unsigned short* __restrict__ nbr_l, const int* __restrict__ nnbr,
-   const int* __restrict__ jbl, const int* __restrict__ jbn, const int* __restrict__ sp_start,
-   const int* __restrict__ sp_j, const float4* __restrict__ sp_sc, const float4* __restrict__ spos,
-   const float* __restrict__ r8, float* __restrict__ z8, PcgDots D, int* __restrict__ err)
+   TensorList T, Partners S, const unsigned short* __restrict__ nbr_l, const int* __restrict__ jbl,
+   const int* __restrict__ jbn, const float4* __restrict__ spos, const float* __restrict__ r8, float* __restrict__ z8, PcgDots D,
+   int* __restrict__ err)
 {
    pdl_wait();
    extern __shared__ __align__(128) unsigned char stg[];
@@ -706,43 +594,27 @@ __global__ void __launch_bounds__(32 * G) k_precond_dots_stg(PairParams P, int n
       mbar_init(bar_s, 1);
    __syncthreads();
    const int g = threadIdx.x % G;
-   float rz_d = 0.f, rz_p = 0.f, rr_d = 0.f, rr_p = 0.f;
+   float dots[4] = {0.f, 0.f, 0.f, 0.f};
    unsigned phase = 0;
    for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
       const int i = blk * 32 + threadIdx.x / G;
       const int nj = jbn[blk];
-      float f[6];
-      if (nj <= STAGE_JB_CAP) {
+      const bool staged = nj <= STAGE_JB_CAP;
+      if (staged) {
          __syncthreads();  // the previous pass has read the buffers
          stage_rows(stg, bar_s, phase, jbl + (size_t)blk * STAGE_JB_CAP, nj, spos, r8, err);
          phase ^= 1u;
-         precond_row_stg<G>(P, i, g, stg, f, nbr_l, nnbr, sp_start, sp_j, sp_sc, spos, r8);
-      } else {
-         precond_row<G>(P, i, g, f, nbr, nnbr, sp_start, sp_j, sp_sc, spos, r8);
       }
-      const float poli = r8[8 * i + 7];
-#pragma unroll
-      for (int c0 = 0; c0 < 6; c0 += G) {
-         const int c = c0 + g;
-         if (c < 6) {
-            const float r = r8[8 * i + c];
-            const float z = udiag * poli * r + pick6(f, c);
-            z8[8 * i + c] = z;
-            if (D.init)
-               D.conj[8 * i + c] = z;
-            if (c < 3) {
-               rz_d += r * z;
-               rr_d += r * r;
-            } else {
-               rz_p += r * z;
-               rr_p += r * r;
-            }
-         }
-      }
+      float f[6] = {0, 0, 0, 0, 0, 0};
+      const GlobalRows<false> rows{spos, r8, nullptr, 0.f, 0.f};
+      if (i < P.n && staged)
+         staged_sum<G>(P, T, S, nbr_l, i, g, spos, StagedRows{stg}, rows, f);
+      else if (i < P.n)
+         tensor_sum<G>(P, T, S, i, g, spos, rows, f);
+      precond_store<G>(i, udiag, f, r8, z8, D, dots);
    }
-   const float pv[4] = {rz_d, rz_p, rr_d, rr_p};
    pdl_trigger();
-   store_partials_f<4>(D.red, R_RZ_D, pv, sh);
+   store_partials_f<4>(D.red, R_RZ_D, dots, sh);
    if (!last_block(D.state + ST_TICKET0))
       return;
    double tot[4];
@@ -813,7 +685,7 @@ __device__ __forceinline__ void ewald_bn5(const PairParams& P, float f, float r,
 // e_atom[i] = 1/2 sum over i's list and scaled partners (every pair is seen
 // from both atoms); FP64 accumulation of FP32 pair energies
 template <int G>
-__global__ void __launch_bounds__(256) k_empole_real(PairParams P, int npad, float f, const int* __restrict__ nbr,
+__global__ void __launch_bounds__(256) k_empole_real(PairParams P, int npad, float f, ListView nbr,
    const int* __restrict__ nnbr, const int* __restrict__ sp_start, const int* __restrict__ sp_j,
    const float4* __restrict__ sp_sc, const float4* __restrict__ spos, const float* __restrict__ rp,
    double* __restrict__ e_atom)
@@ -827,10 +699,9 @@ __global__ void __launch_bounds__(256) k_empole_real(PairParams P, int npad, flo
       const float4 pi = spos[i];
       float mi[12];
       load12(rp, i, mi);
-      const int* row = nbr + (size_t)i * P.cap;
       const int cnt = nnbr[i];
       for (int k = g; k < cnt; k += G) {
-         const int j = row[k];
+         const int j = nbr(i, k);
          const float3 d = sep(P, pi, spos[j]);
          const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
          if (r2 <= P.cut2) {
@@ -879,24 +750,83 @@ __global__ void __launch_bounds__(256) k_empole_real(PairParams P, int npad, flo
 static constexpr int PAIR_THREADS = 256;
 
 // ---------------------------------------------------------------------------
-// Per-step sub-lists: one CTA per 32-slot block, warp w filtering the row of
-// slot 32 b + w.  Each row of the (reused, buffered) list is filtered into
-// the pairs within the cutoff and those within the preconditioner cutoff, in
-// the row's order (ballot compaction), so the field and preconditioner
-// kernels visit only pairs they use; the kernels repeat the same r^2 test
-// with the same arithmetic.  STAGE: the block also records which 32-slot
+// Per-step sub-lists, one warp per row.  Each row of the (reused, buffered)
+// list is filtered into the pairs within the cutoff and those within the
+// preconditioner cutoff, in the row's order (ballot compaction), so the field
+// and preconditioner kernels visit only pairs they use, and every entry's
+// radial factors are formed here, once per position update: (b1, b2) of the
+// mutual field, (b2, b3) of the permanent one and the preconditioner's
+// (c1, c2); the same for the scaled partners, by their place in the partner
+// table.  Entries within either cutoff queue up in shared memory until a
+// warp's worth is there, so the factors (about 130 instructions a pair) are
+// formed by full warps although only a quarter to a half of the stored list
+// passes.
+// STAGE (one CTA per 32-slot block): the block also records which 32-slot
 // j-blocks its entries fall in (a bitmap over all blocks in shared memory),
 // lists them in ascending order, and rewrites every entry as a local index
 // into that list (position x 32 + slot within the j-block), which is where
 // the staged kernels find the row in shared memory.
+struct FilterOut {
+   int lanes_log2;  // of the tiled layout (ListView)
+   int *nbrc, *nnbrc, *nbrp, *nnbrp;
+   float2* cu;  // mutual field
+   float2* cd;  // permanent field (b2, b3)
+   float2* cp;  // preconditioner
+   float2 *spu, *spp;  // scaled partners: mutual field, preconditioner
+   int *jbl, *jbn;
+   unsigned short *nbrc_l, *nbrp_l;
+};
+
+// radial factors of one pair at squared distance r2 and mutual scale us: the
+// mutual field's b1, b2 (u), the permanent field's b2, b3 (d; its b1 is the
+// mutual one's), the preconditioner's c.  The roundings are written out as
+// the kernels that formed the factors in place had them; the two b2 round at
+// different points.
+__device__ __forceinline__ void pair_factors(const PairParams& P, float r2, float us, float pdi, float pdk,
+   float gamma, float polik, float2& u, float2& d, float2& c)
+{
+   const float invr = rsqrtf(r2);
+   const float r = r2 * invr;
+   const float rr2 = invr * invr;
+   const float rr3 = invr * rr2;
+   const float rr5 = 3.f * rr3 * rr2;
+   const float rr7 = 5.f * rr5 * rr2;
+   float s3, s5, s7;
+   thole_damp(r, pdi, gamma, pdk, s3, s5, s7);
+   if (P.ewald) {
+      const float ralpha = P.aewald * r;
+      const float exp2a = __expf(-ralpha * ralpha);
+      const float b0 = __fmul_rn(erfc_hastings(ralpha, exp2a), invr);
+      const float e1 = __fmul_rn(__fmaf_rn(P.ec1, exp2a, b0), rr2);
+      const float y2 = __fmaf_rn(P.ec2, exp2a, __fmul_rn(3.f, e1));
+      const float e2 = __fmul_rn(y2, rr2);
+      const float y3 = __fmaf_rn(P.ec3, exp2a, __fmul_rn(5.f, e2));
+      const float t5 = __fmaf_rn(-us, s5, 1.f);
+      u.x = __fmaf_rn(-__fmaf_rn(-us, s3, 1.f), rr3, e1);
+      u.y = __fmaf_rn(y2, rr2, -__fmul_rn(t5, rr5));
+      d.x = __fmaf_rn(-t5, rr5, e2);
+      d.y = __fmaf_rn(-__fmaf_rn(-us, s7, 1.f), rr7, __fmul_rn(y3, rr2));
+   } else {
+      u.x = us * s3 * rr3;
+      u.y = us * s5 * rr5;
+      d.x = u.y;
+      d.y = us * s7 * rr7;
+   }
+   const float ir3 = invr * invr * invr;
+   c = make_float2(us * s3 * polik * ir3, 3.f * us * s5 * polik * ir3 * invr * invr);
+}
+
 template <bool STAGE>
-__global__ void __launch_bounds__(1024) k_list_filter(PairParams P, float cutp2, int npad, const int* __restrict__ nbr,
-   const int* __restrict__ nnbr, const float4* __restrict__ spos, int* __restrict__ nbrc, int* __restrict__ nnbrc,
-   int* __restrict__ nbrp, int* __restrict__ nnbrp, int* __restrict__ jbl, int* __restrict__ jbn,
-   unsigned short* __restrict__ nbrc_l, unsigned short* __restrict__ nbrp_l)
+__global__ void __launch_bounds__(STAGE ? 1024 : 256) k_list_filter(PairParams P, float cutp2, int npad,
+   const int* __restrict__ nbr, const int* __restrict__ nnbr, const int* __restrict__ sp_start,
+   const int* __restrict__ sp_j, const float4* __restrict__ sp_sc, const float4* __restrict__ spos,
+   const float2* __restrict__ stag, FilterOut O)
 {
    extern __shared__ unsigned bits_sm[];
    __shared__ int total_sm;
+   constexpr int NW = STAGE ? 32 : 8;
+   __shared__ float4 q_d[NW][64];  // separation, partner's pdamp
+   __shared__ int q_j[NW][64];
    const int words = (npad / 32 + 31) / 32;
    unsigned* bm = bits_sm;
    int* pre = reinterpret_cast<int*>(bits_sm + words);
@@ -907,40 +837,90 @@ __global__ void __launch_bounds__(1024) k_list_filter(PairParams P, float cutp2,
    }
    const int blk = blockIdx.x;
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   const int i = blk * 32 + warp;
+   const int i = blk * NW + warp;
+   const ListView V{nullptr, P.cap, O.lanes_log2};
    int oc = 0, op = 0;
    if (i < P.n) {
       const float4 pi = spos[i];
+      const float2 ti = stag[i];  // thole or type, polarizability
       const int* row = nbr + (size_t)i * P.cap;
-      int* rc = nbrc + (size_t)i * P.cap;
-      int* rp = nbrp + (size_t)i * P.cap;
       const int cnt = nnbr[i];
+      const float rmax2 = fmaxf(P.cut2, cutp2);
       const unsigned lt = (1u << lane) - 1u;
-      for (int k0 = 0; k0 < cnt; k0 += 32) {
-         const int k = k0 + lane;
-         bool inc = false, inp = false;
-         int j = 0;
-         if (k < cnt) {
-            j = row[k];
-            const float3 d = sep(P, pi, spos[j]);
-            const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-            inc = r2 <= P.cut2;
-            inp = r2 <= cutp2;
-         }
+      int qn = 0;
+      // the first m (<= 32) queued entries into the sub-lists
+      const auto drain = [&](int m) {
+         const bool valid = lane < m;
+         const int j = valid ? q_j[warp][lane] : i;
+         const float4 dk = valid ? q_d[warp][lane] : make_float4(1.f, 0.f, 0.f, 1.f);
+         const float r2 = dk.x * dk.x + dk.y * dk.y + dk.z * dk.z;
+         const bool inc = valid && r2 <= P.cut2, inp = valid && r2 <= cutp2;
          const unsigned mc = __ballot_sync(0xffffffffu, inc), mp = __ballot_sync(0xffffffffu, inp);
-         if (inc)
-            rc[oc + __popc(mc & lt)] = j;
-         if (inp)
-            rp[op + __popc(mp & lt)] = j;
+         const float2 tk = stag[j];
+         float2 u, f, c;
+         pair_factors(P, r2, 1.f, pi.w, dk.w, pair_gamma(P, ti.x, tk.x), ti.y * tk.y, u, f, c);
+         if (inc) {
+            const size_t at = V.at(i, oc + __popc(mc & lt));
+            O.nbrc[at] = j;
+            O.cu[at] = u;
+            O.cd[at] = f;
+         }
+         if (inp) {
+            const size_t at = V.at(i, op + __popc(mp & lt));
+            O.nbrp[at] = j;
+            O.cp[at] = c;
+         }
          if (STAGE && (inc || inp))
             atomicOr(&bm[j >> 10], 1u << ((j >> 5) & 31));
          oc += __popc(mc);
          op += __popc(mp);
+      };
+      int j = lane < cnt ? row[lane] : i;
+      for (int k0 = 0; k0 < cnt; k0 += 32) {
+         const bool in = k0 + lane < cnt;
+         const float4 pk = spos[j];
+         const int jn = k0 + 32 + lane < cnt ? row[k0 + 32 + lane] : i;
+         const float3 d = sep(P, pi, pk);
+         const bool acc = in && d.x * d.x + d.y * d.y + d.z * d.z <= rmax2;
+         const unsigned m = __ballot_sync(0xffffffffu, acc);
+         if (acc) {
+            const int p = qn + __popc(m & lt);
+            q_d[warp][p] = make_float4(d.x, d.y, d.z, pk.w);
+            q_j[warp][p] = j;
+         }
+         qn += __popc(m);
+         j = jn;
+         __syncwarp();
+         if (qn >= 32) {
+            drain(32);
+            qn -= 32;
+            __syncwarp();
+            if (lane < qn) {
+               q_d[warp][lane] = q_d[warp][32 + lane];
+               q_j[warp][lane] = q_j[warp][32 + lane];
+            }
+            __syncwarp();
+         }
+      }
+      if (qn > 0)
+         drain(qn);
+      // scaled partners: zero factors beyond the cutoff
+      const int pb = sp_start[i + 1];
+      for (int q = sp_start[i] + lane; q < pb; q += 32) {
+         const int js = sp_j[q];
+         const float4 pk = spos[js];
+         const float3 d = sep(P, pi, pk);
+         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+         const float2 tk = stag[js];
+         float2 u, f, c;
+         pair_factors(P, r2, sp_sc[q].w, pi.w, pk.w, pair_gamma(P, ti.x, tk.x), ti.y * tk.y, u, f, c);
+         O.spu[q] = r2 <= P.cut2 ? u : make_float2(0.f, 0.f);
+         O.spp[q] = r2 <= cutp2 ? c : make_float2(0.f, 0.f);
       }
    }
    if (lane == 0) {
-      nnbrc[i] = oc;
-      nnbrp[i] = op;
+      O.nnbrc[i] = oc;
+      O.nnbrp[i] = op;
    }
    if (!STAGE)
       return;
@@ -964,7 +944,7 @@ __global__ void __launch_bounds__(1024) k_list_filter(PairParams P, float cutp2,
       }
       if (lane == 0) {
          total_sm = run;
-         jbn[blk] = run;
+         O.jbn[blk] = run;
       }
    }
    __syncthreads();
@@ -976,23 +956,21 @@ __global__ void __launch_bounds__(1024) k_list_filter(PairParams P, float cutp2,
       int q = pre[w];
       while (m) {
          const int b = __ffs(m) - 1;
-         jbl[(size_t)blk * STAGE_JB_CAP + q] = w * 32 + b;
+         O.jbl[(size_t)blk * STAGE_JB_CAP + q] = w * 32 + b;
          ++q;
          m &= m - 1u;
       }
    }
    if (i < P.n) {
-      const int* rc = nbrc + (size_t)i * P.cap;
-      const int* rp = nbrp + (size_t)i * P.cap;
-      unsigned short* lc = nbrc_l + (size_t)i * P.cap;
-      unsigned short* lp = nbrp_l + (size_t)i * P.cap;
+      unsigned short* lc = O.nbrc_l + (size_t)i * P.cap;
+      unsigned short* lp = O.nbrp_l + (size_t)i * P.cap;
       for (int k = lane; k < oc; k += 32) {
-         const int j = rc[k], jb = j >> 5;
+         const int j = O.nbrc[V.at(i, k)], jb = j >> 5;
          const int q = pre[jb >> 5] + __popc(bm[jb >> 5] & ((1u << (jb & 31)) - 1u));
          lc[k] = (unsigned short)(q * 32 + (j & 31));
       }
       for (int k = lane; k < op; k += 32) {
-         const int j = rp[k], jb = j >> 5;
+         const int j = O.nbrp[V.at(i, k)], jb = j >> 5;
          const int q = pre[jb >> 5] + __popc(bm[jb >> 5] & ((1u << (jb & 31)) - 1u));
          lp[k] = (unsigned short)(q * 32 + (j & 31));
       }
@@ -1007,17 +985,24 @@ int launch_list_filter(Context* ctx)
    const int nblk = ctx->npad / 32;
    const int words = (nblk + 31) / 32;
    const size_t smem = sizeof(unsigned) * 2 * (size_t)words;
+   ctx->list_lanes = ctx->pair_lanes;
+   FilterOut O{nbrc_view(ctx).sg, ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp, ctx->cfu, ctx->cfd, ctx->cfp, ctx->spu,
+      ctx->spp, ctx->jbl, ctx->jbn, ctx->nbrc_l, ctx->nbrp_l};
    if (ctx->pair_staged)
-      k_list_filter<true><<<nblk, 1024, smem, ctx->stream>>>(P, cutp2, ctx->npad, ctx->nbr, ctx->nnbr, ctx->spos,
-         ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp, ctx->jbl, ctx->jbn, ctx->nbrc_l, ctx->nbrp_l);
+      k_list_filter<true><<<nblk, 1024, smem, ctx->stream>>>(P, cutp2, ctx->npad, ctx->nbr, ctx->nnbr, ctx->sp_start,
+         ctx->sp_j, ctx->sp_sc, ctx->spos, ctx->stag, O);
    else
-      k_list_filter<false><<<nblk, 1024, 0, ctx->stream>>>(P, cutp2, ctx->npad, ctx->nbr, ctx->nnbr, ctx->spos,
-         ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp, ctx->jbl, ctx->jbn, ctx->nbrc_l, ctx->nbrp_l);
+      k_list_filter<false><<<ctx->npad / 8, 256, 0, ctx->stream>>>(P, cutp2, ctx->npad, ctx->nbr, ctx->nnbr,
+         ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos, ctx->stag, O);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
 }
 
-// lanes per atom of the three field kernels (8, 16 or 32; t9gb_pair_lanes)
+static TensorList field_list(const Context* ctx) { return {ctx->nbrc, ctx->nnbrc, ctx->cfu, ctx->spu}; }
+static TensorList precond_list(const Context* ctx) { return {ctx->nbrp, ctx->nnbrp, ctx->cfp, ctx->spp}; }
+static Partners partners(const Context* ctx) { return {ctx->sp_start, ctx->sp_j}; }
+
+// lanes per atom of the three field kernels (4, 8, 16 or 32; t9gb_pair_lanes)
 #define T9_LANES_DISPATCH(KERNEL, ...)                                                                                 \
    do {                                                                                                                \
       const int g_ = ctx->pair_lanes;                                                                                  \
@@ -1062,6 +1047,10 @@ int pair_staging_setup()
          cudaSuccess ||
       cudaFuncSetAttribute(k_precond_dots_stg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
       return T9GB_CUDA_ERR;
+   // the block bitmap and its prefix counts: 8 bytes per 1,024 slots
+   if (cudaFuncSetAttribute(k_list_filter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) !=
+      cudaSuccess)
+      return T9GB_CUDA_ERR;
    return T9GB_OK;
 }
 
@@ -1071,9 +1060,8 @@ int launch_ufield_real(Context* ctx, const float* u6, const float* base6, float*
    prof_begin(ctx, P_UFIELD_REAL);
    if (staged_lanes(ctx)) {
       auto k = ctx->pair_lanes == 8 ? k_ufield_stg<8> : k_ufield_stg<4>;
-      T9_CUDA(launch_k(use_pdl(ctx), k, ctx->npad / 32, 32 * ctx->pair_lanes, STAGE_SMEM, ctx->stream, P, ctx->nbrc,
-         ctx->nbrc_l, ctx->nnbrc, ctx->jbl, ctx->jbn, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos, u6, base6, out6,
-         ctx->copy_err));
+      T9_CUDA(launch_k(use_pdl(ctx), k, ctx->npad / 32, 32 * ctx->pair_lanes, STAGE_SMEM, ctx->stream, P,
+         field_list(ctx), partners(ctx), ctx->nbrc_l, ctx->jbl, ctx->jbn, ctx->spos, u6, base6, out6, ctx->copy_err));
       prof_end(ctx);
       return T9GB_OK;
    }
@@ -1081,8 +1069,8 @@ int launch_ufield_real(Context* ctx, const float* u6, const float* base6, float*
    const int nb = grid_for((long long)ctx->npad * g, PAIR_THREADS);
    auto k = g == 4 ? k_ufield_real<4, false> : g == 8 ? k_ufield_real<8, false> : g == 32 ? k_ufield_real<32, false>
                                                                                     : k_ufield_real<16, false>;
-   T9_CUDA(launch_k(use_pdl(ctx), k, nb, PAIR_THREADS, 0, ctx->stream, P, ctx->npad, ctx->nbrc, ctx->nnbrc,
-      ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos, u6, nullptr, nullptr, base6, out6));
+   T9_CUDA(launch_k(use_pdl(ctx), k, nb, PAIR_THREADS, 0, ctx->stream, P, ctx->npad, field_list(ctx),
+      partners(ctx), ctx->spos, u6, nullptr, nullptr, base6, out6));
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
@@ -1092,8 +1080,8 @@ int launch_ufield_real_dir(Context* ctx, const float* p6, const float* z6, const
 {
    PairParams P = make_params(ctx, ctx->cfg.cutoff);
    prof_begin(ctx, P_UFIELD_REAL);
-   T9_LANES_DISPATCH2(k_ufield_real, true, P, ctx->npad, ctx->nbrc, ctx->nnbrc, ctx->sp_start, ctx->sp_j, ctx->sp_sc,
-      ctx->spos, p6, z6, scal, nullptr, out6);
+   T9_LANES_DISPATCH2(k_ufield_real, true, P, ctx->npad, field_list(ctx), partners(ctx), ctx->spos, p6, z6, scal,
+      nullptr, out6);
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
@@ -1103,7 +1091,7 @@ int launch_dfield_real(Context* ctx, const float* base6, float* out6)
 {
    PairParams P = make_params(ctx, ctx->cfg.cutoff);
    prof_begin(ctx, P_DFIELD_REAL);
-   T9_LANES_DISPATCH(k_dfield_real, P, ctx->npad, ctx->nbrc, ctx->nnbrc, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos,
+   T9_LANES_DISPATCH(k_dfield_real, P, ctx->npad, field_list(ctx), ctx->cfd, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos,
       ctx->srpole, base6, ctx->exfld, out6);
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
@@ -1122,15 +1110,15 @@ int launch_precond_sparse_dots(Context* ctx, const float* r6, float* z6, const P
       const int nblk = ctx->npad / 32;
       auto ks = g == 8 ? k_precond_dots_stg<8> : k_precond_dots_stg<4>;
       T9_CUDA(launch_k(use_pdl(ctx), ks, std::min(RED_MAX, nblk), 32 * g, STAGE_SMEM, ctx->stream, P, nblk,
-         (float)ctx->cfg.udiag, ctx->nbrp, ctx->nbrp_l, ctx->nnbrp, ctx->jbl, ctx->jbn, ctx->sp_start, ctx->sp_j,
-         ctx->sp_sc, ctx->spos, r6, z6, D, ctx->copy_err));
+         (float)ctx->cfg.udiag, precond_list(ctx), partners(ctx), ctx->nbrp_l, ctx->jbl, ctx->jbn, ctx->spos, r6, z6, D,
+         ctx->copy_err));
       prof_end(ctx);
       return T9GB_OK;
    }
    auto k = g == 4 ? k_precond_sparse_dots<4> : g == 8 ? k_precond_sparse_dots<8> : g == 32
          ? k_precond_sparse_dots<32> : k_precond_sparse_dots<16>;
-   T9_CUDA(launch_k(use_pdl(ctx), k, nb, PAIR_THREADS, 0, ctx->stream, P, ctx->npad, (float)ctx->cfg.udiag, ctx->nbrp,
-      ctx->nnbrp, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos, r6, z6, D));
+   T9_CUDA(launch_k(use_pdl(ctx), k, nb, PAIR_THREADS, 0, ctx->stream, P, ctx->npad, (float)ctx->cfg.udiag, precond_list(ctx),
+      partners(ctx), ctx->spos, r6, z6, D));
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
@@ -1141,8 +1129,8 @@ int launch_precond_sparse(Context* ctx, const float* r6, float* z6)
    PairParams P = make_params(ctx, ctx->cfg.usolve_cutoff + ctx->cfg.pbuffer);
    P.ewald = 0;
    prof_begin(ctx, P_PRECOND);
-   T9_LANES_DISPATCH(k_precond_sparse, P, ctx->npad, (float)ctx->cfg.udiag, ctx->nbrp, ctx->nnbrp, ctx->sp_start,
-      ctx->sp_j, ctx->sp_sc, ctx->spos, r6, z6);
+   T9_LANES_DISPATCH(k_precond_sparse, P, ctx->npad, (float)ctx->cfg.udiag, precond_list(ctx), partners(ctx),
+      ctx->spos, r6, z6);
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
@@ -1155,7 +1143,7 @@ int launch_empole_real(Context* ctx, double* e_atom)
 {
    PairParams P = make_params(ctx, ctx->cfg.cutoff);
    k_empole_real<GROUP><<<grid_for((long long)ctx->npad * GROUP, PAIR_THREADS), PAIR_THREADS, 0, ctx->stream>>>(P,
-      ctx->npad, (float)ctx->cfg.electric, ctx->nbrc, ctx->nnbrc, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos,
+      ctx->npad, (float)ctx->cfg.electric, nbrc_view(ctx), ctx->nnbrc, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos,
       ctx->srpole, e_atom);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
@@ -1261,7 +1249,7 @@ __device__ __forceinline__ void to_local(const float* F, const float* v, float* 
 }
 
 template <int G>
-__global__ void __launch_bounds__(256) k_learn_features(PairParams P, int npad, const int* __restrict__ nbr,
+__global__ void __launch_bounds__(256) k_learn_features(PairParams P, int npad, ListView nbr,
    const int* __restrict__ nnbr, const int* __restrict__ sp_start, const int* __restrict__ sp_j,
    const float4* __restrict__ sp_sc, const float4* __restrict__ spos, const float* __restrict__ srpole,
    const float* __restrict__ sframe, const float* __restrict__ e8, const float* __restrict__ u8,
@@ -1281,10 +1269,9 @@ __global__ void __launch_bounds__(256) k_learn_features(PairParams P, int npad, 
    if (i < P.n) {
       const float4 pi = spos[i];
       const float pti = u8[8 * i + 6];
-      const int* row = nbr + (size_t)i * P.cap;
       const int cnt = nnbr[i];
       for (int k = g; k < cnt; k += G) {
-         const int j = row[k];
+         const int j = nbr(i, k);
          const float4 pk = spos[j];
          const float3 d = sep(P, pi, pk);
          const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
@@ -1373,7 +1360,7 @@ int launch_learn_features(Context* ctx, const float* e8, const float* u8, float*
 {
    PairParams P = make_params(ctx, DESC_CUT);
    k_learn_features<GROUP><<<grid_for((long long)ctx->npad * GROUP, PAIR_THREADS), PAIR_THREADS, 0, ctx->stream>>>(P,
-      ctx->npad, ctx->cfg.cutoff >= DESC_CUT ? ctx->nbrc : ctx->nbr, ctx->cfg.cutoff >= DESC_CUT ? ctx->nnbrc : ctx->nnbr,
+      ctx->npad, ctx->cfg.cutoff >= DESC_CUT ? nbrc_view(ctx) : nbr_view(ctx), ctx->cfg.cutoff >= DESC_CUT ? ctx->nnbrc : ctx->nnbr,
       ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos, ctx->srpole, ctx->sframe, e8, u8, xf, ctx->spolar, fstat,
       ctx->status, xn);
    T9_CUDA(cudaGetLastError());

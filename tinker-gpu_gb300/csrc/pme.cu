@@ -314,49 +314,6 @@ __global__ void k_conv(size_t ng, const float* __restrict__ infl, float2* __rest
    }
 }
 
-// Sums of N values over the 32 lanes of a warp, value k ending in the lanes
-// where sum_slot<N>(lane) == k: each step halves the values a lane carries
-// (it sends the half it does not keep), so N values take about N + 3
-// shuffles where N separate trees take 5 N.  The order of the additions is
-// fixed.  Lanes with sum_slot < 0 hold nothing.
-template <int N, int O = 16>
-__device__ __forceinline__ float warp_sums(float* v, int lane)
-{
-   constexpr int H = (N + 1) / 2;
-   const bool up = lane & O;
-   if constexpr (N > 1) {
-#pragma unroll
-      for (int k = 0; k < H; ++k) {
-         const float hi = k + H < N ? v[k + H] : 0.f;
-         const float keep = up ? hi : v[k], send = up ? v[k] : hi;
-         v[k] = keep + __shfl_xor_sync(0xffffffffu, send, O);
-      }
-   } else {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
-   }
-   if constexpr (O > 1)
-      return warp_sums<H, O / 2>(v, lane);
-   else
-      return v[0];
-}
-
-template <int N, int O = 16>
-__device__ __forceinline__ int sum_slot(int lane)
-{
-   if constexpr (N <= 1) {
-      return (lane & (2 * O - 1)) == 0 ? 0 : -1;  // the other lanes hold copies
-   } else {
-      constexpr int H = (N + 1) / 2;
-      const bool up = lane & O;
-      int r;
-      if constexpr (O > 1)
-         r = sum_slot<H, O / 2>(lane);
-      else
-         r = 0;
-      return r < 0 || (up && r + H >= N) ? -1 : r + (up ? H : 0);
-   }
-}
-
 // Gather of the first potential derivatives fused with the recip + self
 // field, one warp per atom.  The points are loaded as lane (ix, jy) < 25
 // taking a column of five z points, so that each of a warp's five loads
