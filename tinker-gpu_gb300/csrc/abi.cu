@@ -43,6 +43,7 @@ static int alloc_all(Context* ctx)
    T9_CUDA(cudaMemset(ctx->exfld, 0, sizeof(float) * 4));
    T9_CUDA(cudaMalloc(&ctx->nnbr, sizeof(int) * npad));
    T9_CUDA(cudaMemset(ctx->nnbr, 0, sizeof(int) * npad));
+   T9_CUDA(cudaMalloc(&ctx->nnbre, sizeof(int) * npad));
    T9_CUDA(cudaMalloc(&ctx->nnbrc, sizeof(int) * npad));
    T9_CUDA(cudaMemset(ctx->nnbrc, 0, sizeof(int) * npad));
    T9_CUDA(cudaMalloc(&ctx->nnbrp, sizeof(int) * npad));
@@ -102,7 +103,7 @@ static void free_all(Context* ctx)
 {
    void* dev[] = {ctx->frames, ctx->pole, ctx->xyz, ctx->perm, ctx->iperm, ctx->spos, ctx->spolar, ctx->spolinv,
       ctx->sdamp, ctx->srpole, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->nbr, ctx->nnbr, ctx->nbr_over, ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp,
-      ctx->stag, ctx->cfu, ctx->cfd, ctx->cfp, ctx->spu, ctx->spp,
+      ctx->stag, ctx->sp_i, ctx->nbre, ctx->nnbre, ctx->cfu, ctx->cfd, ctx->cfp, ctx->spu, ctx->spp,
       ctx->jbl, ctx->jbn, ctx->nbrc_l, ctx->nbrp_l, ctx->copy_err,
       ctx->cell_count, ctx->cell_start, ctx->cell_atoms, ctx->atom_cell, ctx->rcp6, ctx->fld6, ctx->udir,
       ctx->efield, ctx->uind, ctx->rsd, ctx->zrsd, ctx->conj, ctx->vec, ctx->tmp6, ctx->e_atom, ctx->sframe, ctx->hout,

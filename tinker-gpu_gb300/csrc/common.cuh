@@ -282,6 +282,7 @@ struct Context {
    // scaled partners of every slot, both directions (CSR over slots)
    int* sp_start = nullptr;  // [npad + 1]
    int* sp_j = nullptr;      // partner slot
+   int* sp_i = nullptr;      // own slot
    float4* sp_sc = nullptr;  // m, d, p, u
    int nsp = 0;
 
@@ -290,6 +291,8 @@ struct Context {
    int nbr_cap = 0;
    int* nbr = nullptr;       // [npad][nbr_cap]
    int* nnbr = nullptr;      // [npad]
+   int* nbre = nullptr;      // [npad][nbr_cap] the rows' part that the filter needs, or null: all of it
+   int* nnbre = nullptr;     // [npad]
    // per-step sub-lists of nbr (same order): pairs within the cutoff and
    // within the preconditioner cutoff
    int* nbrc = nullptr;

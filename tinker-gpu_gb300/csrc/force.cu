@@ -358,8 +358,10 @@ __global__ void __launch_bounds__(128) k_elec_real(PairParams P, int npad, float
          load8(u8, i, ui);
       const float pti = rp[12 * i + 10];
       const int cnt = nnbr[i];
+      const int* row = nbr.p + nbr.at(i, 0);
+      const int sg = nbr.sg, gm = (1 << sg) - 1;
       for (int k = g; k < cnt; k += G) {
-         const int j = nbr(i, k);
+         const int j = row[((k >> sg) << 5) + (k & gm)];
          const float4 pk = spos[j];
          const float3 d = sep(P, pi, pk);
          const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;

@@ -53,6 +53,15 @@ static double list_cutoff(const Context* ctx)
    return r + std::max(0.0, c.list_buffer);
 }
 
+// The radius that the per-step filter needs from the stored list: 0 where the
+// stored list is no longer than that (no van der Waals term)
+static double inner_cutoff(const Context* ctx)
+{
+   const t9gb_config& c = ctx->cfg;
+   const double r = std::max(c.cutoff, c.usolve_cutoff + c.pbuffer) + std::max(0.0, c.list_buffer) + 0.01;
+   return r < list_cutoff(ctx) ? r : 0.0;
+}
+
 // Host: Morton order of the current coordinates, per-slot parameters, the
 // scaled-partner table and the neighbour-list storage.
 // the list and its two per-step sub-lists, all with row capacity cap
@@ -63,6 +72,10 @@ int alloc_lists(Context* ctx, int cap)
       *p = nullptr;
       T9_CUDA(cudaMalloc(p, sizeof(int) * (size_t)ctx->npad * cap));
    }
+   cudaFree(ctx->nbre);
+   ctx->nbre = nullptr;
+   if (inner_cutoff(ctx) > 0)
+      T9_CUDA(cudaMalloc(&ctx->nbre, sizeof(int) * (size_t)ctx->npad * cap));
    for (float2** p : {&ctx->cfu, &ctx->cfd, &ctx->cfp}) {
       cudaFree(*p);
       *p = nullptr;
@@ -169,7 +182,7 @@ int order_build(Context* ctx)
       part[si].push_back({sk, pr.second.e, pr.second.v});
       part[sk].push_back({si, pr.second.e, pr.second.v});
    }
-   std::vector<int> sp_start(npad + 1, 0), sp_j;
+   std::vector<int> sp_start(npad + 1, 0), sp_j, sp_i;
    std::vector<float4> sp_sc;
    std::vector<float> sp_v;
    for (int s = 0; s < npad; ++s) {
@@ -178,6 +191,7 @@ int order_build(Context* ctx)
       sp_start[s + 1] = sp_start[s] + (int)v.size();
       for (auto& e : v) {
          sp_j.push_back(e.k);
+         sp_i.push_back(s);
          sp_sc.push_back(e.sc);
          sp_v.push_back(e.v);
       }
@@ -230,6 +244,7 @@ int order_build(Context* ctx)
    cudaFree(ctx->iperm);
    cudaFree(ctx->sp_start);
    cudaFree(ctx->sp_j);
+   cudaFree(ctx->sp_i);
    cudaFree(ctx->sp_sc);
    cudaFree(ctx->sp_v);
    cudaFree(ctx->spu);
@@ -238,12 +253,13 @@ int order_build(Context* ctx)
    ctx->spu = ctx->spp = nullptr;
    cudaFree(ctx->cell_count);
    cudaFree(ctx->cell_start);
-   ctx->perm = ctx->iperm = ctx->sp_start = ctx->sp_j = ctx->cell_count = ctx->cell_start = nullptr;
+   ctx->perm = ctx->iperm = ctx->sp_start = ctx->sp_j = ctx->sp_i = ctx->cell_count = ctx->cell_start = nullptr;
    ctx->sp_sc = nullptr;
    T9_CUDA(cudaMalloc(&ctx->perm, sizeof(int) * npad));
    T9_CUDA(cudaMalloc(&ctx->iperm, sizeof(int) * n));
    T9_CUDA(cudaMalloc(&ctx->sp_start, sizeof(int) * (npad + 1)));
    T9_CUDA(cudaMalloc(&ctx->sp_j, sizeof(int) * std::max(1, ctx->nsp)));
+   T9_CUDA(cudaMalloc(&ctx->sp_i, sizeof(int) * std::max(1, ctx->nsp)));
    T9_CUDA(cudaMalloc(&ctx->sp_sc, sizeof(float4) * std::max(1, ctx->nsp)));
    T9_CUDA(cudaMalloc(&ctx->sp_v, sizeof(float) * std::max(1, ctx->nsp)));
    T9_CUDA(cudaMalloc(&ctx->spu, sizeof(float2) * std::max(1, ctx->nsp)));
@@ -253,6 +269,7 @@ int order_build(Context* ctx)
    T9_CUDA(cudaMemcpy(ctx->sp_start, sp_start.data(), sizeof(int) * (npad + 1), cudaMemcpyHostToDevice));
    if (ctx->nsp) {
       T9_CUDA(cudaMemcpy(ctx->sp_j, sp_j.data(), sizeof(int) * ctx->nsp, cudaMemcpyHostToDevice));
+      T9_CUDA(cudaMemcpy(ctx->sp_i, sp_i.data(), sizeof(int) * ctx->nsp, cudaMemcpyHostToDevice));
       T9_CUDA(cudaMemcpy(ctx->sp_sc, sp_sc.data(), sizeof(float4) * ctx->nsp, cudaMemcpyHostToDevice));
       T9_CUDA(cudaMemcpy(ctx->sp_v, sp_v.data(), sizeof(float) * ctx->nsp, cudaMemcpyHostToDevice));
    }
@@ -266,7 +283,7 @@ int order_build(Context* ctx)
       T9_CUDA(cudaMalloc(&ctx->cell_count, sizeof(int) * ctx->ncell));
       T9_CUDA(cudaMalloc(&ctx->cell_start, sizeof(int) * (ctx->ncell + 1)));
    }
-   if (cap != ctx->nbr_cap)
+   if (cap != ctx->nbr_cap || (inner_cutoff(ctx) > 0) != (ctx->nbre != nullptr))
       T9_CHECK(alloc_lists(ctx, cap));
    // legacy-stream copies above finish before the stream's kernels
    T9_CUDA(cudaDeviceSynchronize());
@@ -574,6 +591,38 @@ __global__ void __launch_bounds__(256) k_nbr_all(CellParams C, const float4* __r
    }
 }
 
+// The part of every row within r2, in the row's order (one warp per row): with
+// the van der Waals term the stored rows are twice as long as the per-step
+// filter needs, and it runs every step while this runs at list builds only.
+__global__ void __launch_bounds__(256) k_nbr_inner(CellParams C, float r2, const float4* __restrict__ spos,
+   const int* __restrict__ nbr, const int* __restrict__ nnbr, int* __restrict__ nbre, int* __restrict__ nnbre)
+{
+   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+   const int lane = threadIdx.x & 31;
+   if (i >= C.npad)
+      return;
+   const float4 pi = spos[i];
+   const size_t at = (size_t)i * C.cap;
+   const int cnt = nnbr[i];
+   const unsigned lt = (1u << lane) - 1u;
+   int out = 0;
+   for (int k0 = 0; k0 < cnt; k0 += 32) {
+      const int k = k0 + lane;
+      const int j = k < cnt ? nbr[at + k] : i;
+      const float4 pj = spos[j];
+      const float dx = image1(pj.x - pi.x, C.lx, C.ilx);
+      const float dy = image1(pj.y - pi.y, C.ly, C.ily);
+      const float dz = image1(pj.z - pi.z, C.lz, C.ilz);
+      const bool acc = k < cnt && dx * dx + dy * dy + dz * dz <= r2;
+      const unsigned m = __ballot_sync(0xffffffffu, acc);
+      if (acc)
+         nbre[at + out + __popc(m & lt)] = j;
+      out += __popc(m);
+   }
+   if (lane == 0)
+      nnbre[i] = out;
+}
+
 int list_update(Context* ctx)
 {
    const t9gb_config& cfg = ctx->cfg;
@@ -607,6 +656,11 @@ int list_update(Context* ctx)
    } else {
       k_nbr_all<<<grid_for((long long)ctx->npad * 32, 256), 256, 0, ctx->stream>>>(C, ctx->spos, ctx->sp_start,
          ctx->sp_j, ctx->nbr, ctx->nnbr, ctx->nbr_over);
+   }
+   if (ctx->nbre) {
+      const double re = inner_cutoff(ctx);
+      k_nbr_inner<<<grid_for((long long)ctx->npad * 32, 256), 256, 0, ctx->stream>>>(C, (float)(re * re), ctx->spos,
+         ctx->nbr, ctx->nnbr, ctx->nbre, ctx->nnbre);
    }
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());

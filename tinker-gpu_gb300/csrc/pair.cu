@@ -169,37 +169,40 @@ struct GlobalRows {
    }
 };
 
-// the row sum of one atom's lane g of G: two entries per trip, both sets of
-// loads in flight together, the next trip's indices loaded ahead.  ip, cp:
-// the lane's first index and factors; is: index stride from one entry of the
-// lane to the next (factors: 32)
-template <int G, class IDX, class R>
+// the row sum of one atom's lane g of G: U entries per trip, their loads in
+// flight together and added in order, the next trip's indices loaded ahead.
+// ip, cp: the lane's first index and factors; is: index stride from one entry
+// of the lane to the next (factors: 32).
+template <int G, int U, class IDX, class R>
 __device__ __forceinline__ void tensor_row(const PairParams& P, const IDX* __restrict__ ip, int is,
    const float2* __restrict__ cp, int cnt, int g, float4 pi, const R& rows, float* f)
 {
-   int k = g;
-   int j0 = k < cnt ? stream_index(ip) : 0;
-   int j1 = k + G < cnt ? stream_index(ip + is) : 0;
-   while (k + G < cnt) {
-      const float2 c0 = stream_coef(cp), c1 = stream_coef(cp + 32);
-      float4 p0, p1;
-      float u0[8], u1[8];
-      rows.get(j0, p0, u0);
-      rows.get(j1, p1, u1);
-      k += 2 * G;
-      ip += 2 * is;
-      cp += 64;
-      j0 = k < cnt ? stream_index(ip) : 0;
-      j1 = k + G < cnt ? stream_index(ip + is) : 0;
-      tensor_add(sep(P, pi, p0), c0, u0, f);
-      tensor_add(sep(P, pi, p1), c1, u1, f);
-   }
-   if (k < cnt) {
-      const float2 c0 = stream_coef(cp);
-      float4 p0;
-      float u0[8];
-      rows.get(j0, p0, u0);
-      tensor_add(sep(P, pi, p0), c0, u0, f);
+   int j[U];
+#pragma unroll
+   for (int q = 0; q < U; ++q)
+      j[q] = g + q * G < cnt ? stream_index(ip + q * is) : -1;
+   for (int k = g; k < cnt; k += U * G) {
+      float2 c[U];
+      float4 p[U];
+      float u[U][8];
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+         if (q == 0 || j[q] >= 0) {
+            c[q] = stream_coef(cp + 32 * q);
+            rows.get(j[q], p[q], u[q]);
+         }
+      ip += U * is;
+      cp += 32 * U;
+      int n[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q)
+         n[q] = k + (U + q) * G < cnt ? stream_index(ip + q * is) : -1;
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+         if (q == 0 || j[q] >= 0)
+            tensor_add(sep(P, pi, p[q]), c[q], u[q], f);
+         j[q] = n[q];
+      }
    }
 }
 
@@ -219,17 +222,17 @@ __device__ __forceinline__ void tensor_partners(const PairParams& P, const Partn
 }
 
 // both, from global memory
-template <int G, class R>
+template <int G, int U, class R>
 __device__ __forceinline__ void tensor_sum(const PairParams& P, const TensorList& T, const Partners& S, int i, int g,
    const float4* __restrict__ spos, const R& rows, float* f)
 {
    const float4 pi = spos[i];
    const size_t at = tile_at<G>(P.cap, i) + g;
-   tensor_row<G>(P, T.nbr + at, 32, T.coef + at, T.cnt[i], g, pi, rows, f);
+   tensor_row<G, U>(P, T.nbr + at, 32, T.coef + at, T.cnt[i], g, pi, rows, f);
    tensor_partners<G>(P, S, T.spc, i, g, pi, rows, f);
 }
 
-template <int G, bool DIR>
+template <int G, bool DIR, int U = 2>
 __global__ void __launch_bounds__(256) k_ufield_real(PairParams P, int npad, TensorList T, Partners S,
    const float4* __restrict__ spos, const float* __restrict__ u8, const float* __restrict__ z8,
    const double* __restrict__ scal, const float* __restrict__ base8, float* __restrict__ out8)
@@ -246,7 +249,7 @@ __global__ void __launch_bounds__(256) k_ufield_real(PairParams P, int npad, Ten
          rows.bd = (float)scal[S_B_D];
          rows.bp = (float)scal[S_B_P];
       }
-      tensor_sum<G>(P, T, S, i, g, spos, rows, f);
+      tensor_sum<G, U>(P, T, S, i, g, spos, rows, f);
    }
    pdl_trigger();
    for_own6<G>(f, [&](int c, float v) { out8[8 * i + c] = base8 && i < P.n ? v + base8[8 * i + c] : v; });
@@ -413,7 +416,7 @@ __global__ void __launch_bounds__(256) k_precond_sparse(PairParams P, int npad, 
       return;
    float f[6] = {0, 0, 0, 0, 0, 0};
    if (i < P.n)
-      tensor_sum<G>(P, T, S, i, g, spos, GlobalRows<false>{spos, r8, nullptr, 0.f, 0.f}, f);
+      tensor_sum<G, 2>(P, T, S, i, g, spos, GlobalRows<false>{spos, r8, nullptr, 0.f, 0.f}, f);
    const float poli = r8[8 * i + 7];
    for_own6<G>(f, [&](int c, float v) { z8[8 * i + c] = udiag * poli * r8[8 * i + c] + v; });
 }
@@ -444,8 +447,8 @@ __device__ __forceinline__ void precond_store(int i, float udiag, float* f, cons
 // block, the CG scalars.  Slots are visited block-strided, 256 / G per
 // block per trip (npad is a multiple of 32, so every lane of a block makes
 // the same trips); at most RED_MAX blocks.
-template <int G>
-__global__ void __launch_bounds__(256, 4) k_precond_sparse_dots(PairParams P, int npad, float udiag,
+template <int G, int U = 2>
+__global__ void __launch_bounds__(256, U > 2 ? 2 : 4) k_precond_sparse_dots(PairParams P, int npad, float udiag,
    TensorList T, Partners S, const float4* __restrict__ spos, const float* __restrict__ r8, float* __restrict__ z8,
    PcgDots D)
 {
@@ -458,7 +461,7 @@ __global__ void __launch_bounds__(256, 4) k_precond_sparse_dots(PairParams P, in
    for (int i = blockIdx.x * PER + threadIdx.x / G; i < npad; i += gridDim.x * PER) {
       float f[6] = {0, 0, 0, 0, 0, 0};
       if (i < P.n)
-         tensor_sum<G>(P, T, S, i, g, spos, rows, f);
+         tensor_sum<G, U>(P, T, S, i, g, spos, rows, f);
       precond_store<G>(i, udiag, f, r8, z8, D, dots);
    }
    pdl_trigger();
@@ -542,7 +545,7 @@ __device__ __forceinline__ void staged_sum(const PairParams& P, const TensorList
    const GlobalRows<false>& rows, float* f)
 {
    const float4 pi = spos[i];
-   tensor_row<G>(P, nbr_l + (size_t)i * P.cap + g, G, T.coef + tile_at<G>(P.cap, i) + g, T.cnt[i], g, pi, stg, f);
+   tensor_row<G, 2>(P, nbr_l + (size_t)i * P.cap + g, G, T.coef + tile_at<G>(P.cap, i) + g, T.cnt[i], g, pi, stg, f);
    tensor_partners<G>(P, S, T.spc, i, g, pi, rows, f);
 }
 
@@ -570,7 +573,7 @@ __global__ void __launch_bounds__(32 * G) k_ufield_stg(PairParams P, TensorList 
    if (i < P.n && staged)
       staged_sum<G>(P, T, S, nbr_l, i, g, spos, StagedRows{stg}, rows, f);
    else if (i < P.n)
-      tensor_sum<G>(P, T, S, i, g, spos, rows, f);
+      tensor_sum<G, 2>(P, T, S, i, g, spos, rows, f);
    pdl_trigger();
    for_own6<G>(f, [&](int c, float v) { out8[8 * i + c] = base8 && i < P.n ? base8[8 * i + c] + v : v; });
 }
@@ -610,7 +613,7 @@ __global__ void __launch_bounds__(32 * G) k_precond_dots_stg(PairParams P, int n
       if (i < P.n && staged)
          staged_sum<G>(P, T, S, nbr_l, i, g, spos, StagedRows{stg}, rows, f);
       else if (i < P.n)
-         tensor_sum<G>(P, T, S, i, g, spos, rows, f);
+         tensor_sum<G, 2>(P, T, S, i, g, spos, rows, f);
       precond_store<G>(i, udiag, f, r8, z8, D, dots);
    }
    pdl_trigger();
@@ -816,17 +819,36 @@ __device__ __forceinline__ void pair_factors(const PairParams& P, float r2, floa
    c = make_float2(us * s3 * polik * ir3, 3.f * us * s5 * polik * ir3 * invr * invr);
 }
 
+// The blocks past the rows' form the scaled partners' factors, a thread per
+// entry of the partner table (a warp per row had two lanes at work there).
 template <bool STAGE>
-__global__ void __launch_bounds__(STAGE ? 1024 : 256) k_list_filter(PairParams P, float cutp2, int npad,
-   const int* __restrict__ nbr, const int* __restrict__ nnbr, const int* __restrict__ sp_start,
-   const int* __restrict__ sp_j, const float4* __restrict__ sp_sc, const float4* __restrict__ spos,
-   const float2* __restrict__ stag, FilterOut O)
+__global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filter(PairParams P, float cutp2, int npad,
+   const int* __restrict__ nbr, const int* __restrict__ nnbr, const int* __restrict__ sp_j,
+   const int* __restrict__ sp_i, int nsp, const float4* __restrict__ sp_sc,
+   const float4* __restrict__ spos, const float2* __restrict__ stag, FilterOut O)
 {
    extern __shared__ unsigned bits_sm[];
    __shared__ int total_sm;
    constexpr int NW = STAGE ? 32 : 8;
    __shared__ float4 q_d[NW][64];  // separation, partner's pdamp
    __shared__ int q_j[NW][64];
+   const int blk = blockIdx.x;
+   if (blk >= npad / NW) {
+      const int q = (blk - npad / NW) * blockDim.x + threadIdx.x;
+      if (q >= nsp)
+         return;
+      const int ii = sp_i[q], js = sp_j[q];
+      const float4 pi = spos[ii], pk = spos[js];
+      const float2 ti = stag[ii], tk = stag[js];
+      const float3 d = sep(P, pi, pk);
+      const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+      float2 u, f, c;
+      pair_factors(P, r2, sp_sc[q].w, pi.w, pk.w, pair_gamma(P, ti.x, tk.x), ti.y * tk.y, u, f, c);
+      // zero factors beyond the cutoff
+      O.spu[q] = r2 <= P.cut2 ? u : make_float2(0.f, 0.f);
+      O.spp[q] = r2 <= cutp2 ? c : make_float2(0.f, 0.f);
+      return;
+   }
    const int words = (npad / 32 + 31) / 32;
    unsigned* bm = bits_sm;
    int* pre = reinterpret_cast<int*>(bits_sm + words);
@@ -835,7 +857,6 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256) k_list_filter(PairParams P
          bm[w] = 0u;
       __syncthreads();
    }
-   const int blk = blockIdx.x;
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    const int i = blk * NW + warp;
    const ListView V{nullptr, P.cap, O.lanes_log2};
@@ -847,28 +868,36 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256) k_list_filter(PairParams P
       const int cnt = nnbr[i];
       const float rmax2 = fmaxf(P.cut2, cutp2);
       const unsigned lt = (1u << lane) - 1u;
+      // the row's place in the tiled lists, and an entry's from it
+      const size_t base = V.at(i, 0);
+      int* nc = O.nbrc + base;
+      float2* cu = O.cu + base;
+      float2* cd = O.cd + base;
+      int* np = O.nbrp + base;
+      float2* cp = O.cp + base;
+      const int sg = O.lanes_log2, gm = (1 << sg) - 1;
       int qn = 0;
       // the first m (<= 32) queued entries into the sub-lists
       const auto drain = [&](int m) {
          const bool valid = lane < m;
          const int j = valid ? q_j[warp][lane] : i;
+         const float2 tk = stag[j];
          const float4 dk = valid ? q_d[warp][lane] : make_float4(1.f, 0.f, 0.f, 1.f);
          const float r2 = dk.x * dk.x + dk.y * dk.y + dk.z * dk.z;
          const bool inc = valid && r2 <= P.cut2, inp = valid && r2 <= cutp2;
          const unsigned mc = __ballot_sync(0xffffffffu, inc), mp = __ballot_sync(0xffffffffu, inp);
-         const float2 tk = stag[j];
          float2 u, f, c;
          pair_factors(P, r2, 1.f, pi.w, dk.w, pair_gamma(P, ti.x, tk.x), ti.y * tk.y, u, f, c);
          if (inc) {
-            const size_t at = V.at(i, oc + __popc(mc & lt));
-            O.nbrc[at] = j;
-            O.cu[at] = u;
-            O.cd[at] = f;
+            const unsigned k = oc + __popc(mc & lt), at = ((k >> sg) << 5) + (k & gm);
+            nc[at] = j;
+            cu[at] = u;
+            cd[at] = f;
          }
          if (inp) {
-            const size_t at = V.at(i, op + __popc(mp & lt));
-            O.nbrp[at] = j;
-            O.cp[at] = c;
+            const unsigned k = op + __popc(mp & lt), at = ((k >> sg) << 5) + (k & gm);
+            np[at] = j;
+            cp[at] = c;
          }
          if (STAGE && (inc || inp))
             atomicOr(&bm[j >> 10], 1u << ((j >> 5) & 31));
@@ -904,19 +933,6 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256) k_list_filter(PairParams P
       }
       if (qn > 0)
          drain(qn);
-      // scaled partners: zero factors beyond the cutoff
-      const int pb = sp_start[i + 1];
-      for (int q = sp_start[i] + lane; q < pb; q += 32) {
-         const int js = sp_j[q];
-         const float4 pk = spos[js];
-         const float3 d = sep(P, pi, pk);
-         const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-         const float2 tk = stag[js];
-         float2 u, f, c;
-         pair_factors(P, r2, sp_sc[q].w, pi.w, pk.w, pair_gamma(P, ti.x, tk.x), ti.y * tk.y, u, f, c);
-         O.spu[q] = r2 <= P.cut2 ? u : make_float2(0.f, 0.f);
-         O.spp[q] = r2 <= cutp2 ? c : make_float2(0.f, 0.f);
-      }
    }
    if (lane == 0) {
       O.nnbrc[i] = oc;
@@ -985,18 +1001,27 @@ int launch_list_filter(Context* ctx)
    const int nblk = ctx->npad / 32;
    const int words = (nblk + 31) / 32;
    const size_t smem = sizeof(unsigned) * 2 * (size_t)words;
+   const int* nbr = ctx->nbre ? ctx->nbre : ctx->nbr;
+   const int* nnbr = ctx->nbre ? ctx->nnbre : ctx->nnbr;
    ctx->list_lanes = ctx->pair_lanes;
    FilterOut O{nbrc_view(ctx).sg, ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp, ctx->cfu, ctx->cfd, ctx->cfp, ctx->spu,
       ctx->spp, ctx->jbl, ctx->jbn, ctx->nbrc_l, ctx->nbrp_l};
    if (ctx->pair_staged)
-      k_list_filter<true><<<nblk, 1024, smem, ctx->stream>>>(P, cutp2, ctx->npad, ctx->nbr, ctx->nnbr, ctx->sp_start,
-         ctx->sp_j, ctx->sp_sc, ctx->spos, ctx->stag, O);
+      k_list_filter<true><<<nblk + grid_for(ctx->nsp, 1024), 1024, smem, ctx->stream>>>(P, cutp2, ctx->npad, nbr, nnbr,
+         ctx->sp_j, ctx->sp_i, ctx->nsp, ctx->sp_sc, ctx->spos, ctx->stag, O);
    else
-      k_list_filter<false><<<ctx->npad / 8, 256, 0, ctx->stream>>>(P, cutp2, ctx->npad, ctx->nbr, ctx->nnbr,
-         ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos, ctx->stag, O);
+      k_list_filter<false><<<ctx->npad / 8 + grid_for(ctx->nsp, 256), 256, 0, ctx->stream>>>(P, cutp2, ctx->npad, nbr,
+         nnbr, ctx->sp_j, ctx->sp_i, ctx->nsp, ctx->sp_sc, ctx->spos, ctx->stag, O);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
 }
+
+// Where the grid leaves an SM at most one block, a row's trips wait on their
+// own latency, not on the L1's line rate: four entries a trip (80-106
+// registers).  GB300, induce: droplet of 1,500 atoms (rows of 1,499) 749 ->
+// 660 us; periodic boxes of 648 and 3,000 atoms the same either way; at
+// 12,288 atoms two entries are better (414 against 436 us).
+static bool few_blocks(int nb) { return nb <= 152; }
 
 static TensorList field_list(const Context* ctx) { return {ctx->nbrc, ctx->nnbrc, ctx->cfu, ctx->spu}; }
 static TensorList precond_list(const Context* ctx) { return {ctx->nbrp, ctx->nnbrp, ctx->cfp, ctx->spp}; }
@@ -1069,6 +1094,8 @@ int launch_ufield_real(Context* ctx, const float* u6, const float* base6, float*
    const int nb = grid_for((long long)ctx->npad * g, PAIR_THREADS);
    auto k = g == 4 ? k_ufield_real<4, false> : g == 8 ? k_ufield_real<8, false> : g == 32 ? k_ufield_real<32, false>
                                                                                     : k_ufield_real<16, false>;
+   if (g == 8 && few_blocks(nb))
+      k = k_ufield_real<8, false, 4>;
    T9_CUDA(launch_k(use_pdl(ctx), k, nb, PAIR_THREADS, 0, ctx->stream, P, ctx->npad, field_list(ctx),
       partners(ctx), ctx->spos, u6, nullptr, nullptr, base6, out6));
    prof_end(ctx);
@@ -1117,6 +1144,8 @@ int launch_precond_sparse_dots(Context* ctx, const float* r6, float* z6, const P
    }
    auto k = g == 4 ? k_precond_sparse_dots<4> : g == 8 ? k_precond_sparse_dots<8> : g == 32
          ? k_precond_sparse_dots<32> : k_precond_sparse_dots<16>;
+   if (g == 8 && few_blocks(nb))
+      k = k_precond_sparse_dots<8, 4>;
    T9_CUDA(launch_k(use_pdl(ctx), k, nb, PAIR_THREADS, 0, ctx->stream, P, ctx->npad, (float)ctx->cfg.udiag, precond_list(ctx),
       partners(ctx), ctx->spos, r6, z6, D));
    prof_end(ctx);
