@@ -360,8 +360,10 @@ __global__ void __launch_bounds__(128) k_elec_real(PairParams P, int npad, float
       const int cnt = nnbr[i];
       const int* row = nbr.p + nbr.at(i, 0);
       const int sg = nbr.sg, gm = (1 << sg) - 1;
+      int jn = g < cnt ? row[((g >> sg) << 5) + (g & gm)] : i;
       for (int k = g; k < cnt; k += G) {
-         const int j = row[((k >> sg) << 5) + (k & gm)];
+         const int j = jn, kn = k + G;
+         jn = kn < cnt ? row[((kn >> sg) << 5) + (kn & gm)] : i;
          const float4 pk = spos[j];
          const float3 d = sep(P, pi, pk);
          const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
