@@ -87,6 +87,7 @@ static int alloc_all(Context* ctx)
    T9_CUDA(cudaMallocHost(&ctx->h_stage, ctx->h_stage_bytes));
    T9_CUDA(cudaMallocHost(&ctx->h_in, sizeof(float) * 3 * (size_t)npad));
    T9_CUDA(cudaEventCreateWithFlags(&ctx->ev_in, cudaEventDisableTiming));
+   T9_CUDA(cudaEventCreateWithFlags(&ctx->ev_guess, cudaEventDisableTiming));
    T9_CUDA(cudaEventCreateWithFlags(&ctx->ev_solved, cudaEventDisableTiming));
    for (int k = 0; k < 4; ++k) {
       T9_CUDA(cudaStreamCreateWithFlags(&ctx->side_stream[k], cudaStreamNonBlocking));
@@ -143,6 +144,8 @@ static void free_all(Context* ctx)
       if (ctx->ev_join[k])
          cudaEventDestroy(ctx->ev_join[k]);
    }
+   if (ctx->ev_guess)
+      cudaEventDestroy(ctx->ev_guess);
    if (ctx->ev_solved)
       cudaEventDestroy(ctx->ev_solved);
    if (ctx->lx_stream)
@@ -412,10 +415,10 @@ int t9gb_set_xyz_device(t9gb_context* h, const float* xyz_device)
    if (!h || !xyz_device)
       return T9GB_BAD_ARG;
    Context* ctx = &h->c;
-   T9_CUDA(cudaMemcpyAsync(ctx->xyz, xyz_device, sizeof(float) * 3 * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
    ctx->have_xyz = true;
    if (ctx->have_order)
-      T9_CHECK(scatter_positions(ctx));
+      return scatter_positions(ctx, xyz_device);
+   T9_CUDA(cudaMemcpyAsync(ctx->xyz, xyz_device, sizeof(float) * 3 * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
    return T9GB_OK;
 }
 

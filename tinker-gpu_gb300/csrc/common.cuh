@@ -261,6 +261,7 @@ struct Context {
    std::vector<double> h_xyz;  // host copy for the ordering, refreshed by t9gb_nblist_build
    float* h_in = nullptr;      // pinned staging of host coordinates
    cudaEvent_t ev_in = nullptr; // its last copy to the device
+   cudaEvent_t ev_guess = nullptr;   // the predicted guess is there (pcg.cu)
    cudaEvent_t ev_solved = nullptr;  // the induce graph and its status copies (work queued after it runs on)
    bool ev_in_pending = false;
    bool have_xyz = false;
@@ -624,7 +625,8 @@ int launch_ufield_recip_gather_dir(Context* ctx, float* out6, const PcgAp& P);
 // the same on the second grid (and FFT plan)
 int launch_ufield_recip_grid_alt(Context* ctx, const float* u6);
 int launch_ufield_recip_gather_alt(Context* ctx, const float* u6, float* out6);
-int scatter_positions(Context* ctx);
+// sorted positions of ctx->xyz, or of src, which is then copied there too
+int scatter_positions(Context* ctx, const float* src = nullptr);
 // t9gb_emplar(grad) with `beside` called once the dipoles are solved and the
 // list is current, before the electrostatic forces are launched
 int emplar_grad_beside(Context* ctx, float* grad, const std::function<int()>& beside,

@@ -682,8 +682,9 @@ struct SplineParams {
    float *lo, *hi;     // [npad][SPL_ROW]
 };
 
+// copy (may be null): the coordinates in the caller's order as well.
 __global__ void k_scatter_pos(int npad, const int* __restrict__ perm, const float* __restrict__ xyz,
-   const float2* __restrict__ sdamp, float4* __restrict__ spos, SplineParams S)
+   float* __restrict__ copy, const float2* __restrict__ sdamp, float4* __restrict__ spos, SplineParams S)
 {
    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 3 * npad; e += gridDim.x * blockDim.x) {
       const int s = e / 3, d = e - 3 * s;
@@ -694,6 +695,8 @@ __global__ void k_scatter_pos(int npad, const int* __restrict__ perm, const floa
          continue;
       }
       const float x = xyz[3 * a + d];
+      if (copy)
+         copy[3 * a + d] = x;
       if (d == 0)
          spos[s] = make_float4(x, xyz[3 * a + 1], xyz[3 * a + 2], sdamp[s].x);
       if (S.nfft[0]) {
@@ -705,7 +708,7 @@ __global__ void k_scatter_pos(int npad, const int* __restrict__ perm, const floa
    }
 }
 
-int scatter_positions(Context* ctx)
+int scatter_positions(Context* ctx, const float* src)
 {
    const t9gb_config& c = ctx->cfg;
    SplineParams S = {};
@@ -718,8 +721,8 @@ int scatter_positions(Context* ctx)
       S.lo = ctx->pme.spl_lo;
       S.hi = ctx->pme.spl_hi;
    }
-   k_scatter_pos<<<grid_for(3 * (long long)ctx->npad, 256), 256, 0, ctx->stream>>>(ctx->npad, ctx->perm, ctx->xyz,
-      ctx->sdamp, ctx->spos, S);
+   k_scatter_pos<<<grid_for(3 * (long long)ctx->npad, 256), 256, 0, ctx->stream>>>(ctx->npad, ctx->perm,
+      src ? src : ctx->xyz, src && src != ctx->xyz ? ctx->xyz : nullptr, ctx->sdamp, ctx->spos, S);
    T9_CUDA(cudaGetLastError());
    ctx->list_stale = true;
    return T9GB_OK;

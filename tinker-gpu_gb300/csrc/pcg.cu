@@ -63,13 +63,11 @@ __device__ __forceinline__ float ring_coef(int predictor, int j, const float* __
 
 __global__ void k_init_guess(VecArgs A, const float* __restrict__ fld, float* __restrict__ efield,
    float* __restrict__ udir, float* __restrict__ uind, int pcgguess, int predictor, const float* __restrict__ hist,
-   const int* __restrict__ state, int set_uind, const float* __restrict__ lcoef)
+   const int* __restrict__ state, const float* __restrict__ lcoef)
 {
    const int nualt = state[ST_NUALT];
    const int depth = predictor == 1 ? 16 : predictor == 2 ? 6 : 0;
-   // set_uind 0: the guess is k_predict's, and the ring (64 bytes per element
-   // with ASPC) is not read again: 18.7 -> 6 us at 98,304 atoms
-   const bool predict = set_uind && depth > 0 && nualt >= depth;
+   const bool predict = depth > 0 && nualt >= depth;
    float coef[16];
    if (predict)
       for (int k = 0; k < depth; ++k) {
@@ -93,8 +91,7 @@ __global__ void k_init_guess(VecArgs A, const float* __restrict__ fld, float* __
       } else if (pcgguess) {
          u = ud;
       }
-      if (set_uind)
-         uind[x] = u;
+      uind[x] = u;
    }
 }
 
@@ -123,6 +120,22 @@ __global__ void k_predict(VecArgs A, int predictor, const float* __restrict__ hi
          u = v;
       }
       uind[x] = u;
+   }
+}
+
+// k_init_guess and k_init_rsd in one pass, where the guess and its field fld2
+// are there before the permanent field fld
+__global__ void k_init_predicted(VecArgs A, const float* __restrict__ fld, const float* __restrict__ fld2,
+   const float* __restrict__ uind, float* __restrict__ efield, float* __restrict__ udir, float* __restrict__ rsd)
+{
+   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < A.ne; e += gridDim.x * blockDim.x) {
+      const int s = e / 6, x = e + 2 * s;  // row s, component e - 6 s of [npad][8]
+      const float pol = A.polar[s], f = fld[x];
+      const float ud = __fmul_rn(pol, f);
+      efield[x] = f;
+      udir[x] = ud;
+      const float r = (ud - uind[x]) * A.polinv[s] + fld2[x];
+      rsd[x] = pol == 0.f ? 0.f : r;
    }
 }
 
@@ -194,34 +207,38 @@ __global__ void k_pcg_p1(VecArgs A, const float* __restrict__ fld, const float* 
 {
    pdl_wait();
    __shared__ double sh[64];
-   float dd = 0.f, dp = 0.f;
    float bd = 0.f, bp = 0.f;
    if (DIR) {
       bd = (float)scal[S_B_D];
       bp = (float)scal[S_B_P];
    }
-   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < A.ne; e += gridDim.x * blockDim.x) {
-      const int s = e / 6, x = e + 2 * s;  // row s, component e - 6 s of [npad][8]
-      float p = conj[x];
-      if (DIR) {
-         p = __fmaf_rn(e - 6 * s < 3 ? bd : bp, p, zrsd[x]);
-         conj[x] = p;
+   // a block forms the partials of up to four of the A.nb element blocks in
+   // turn: 2,048 tickets at one address cost more than the sums themselves
+   for (int vb = blockIdx.x; vb < A.nb; vb += gridDim.x) {
+      float dd = 0.f, dp = 0.f;
+      for (int e = vb * blockDim.x + threadIdx.x; e < A.ne; e += A.nb * blockDim.x) {
+         const int s = e / 6, x = e + 2 * s;  // row s, component e - 6 s of [npad][8]
+         float p = conj[x];
+         if (DIR) {
+            p = __fmaf_rn(e - 6 * s < 3 ? bd : bp, p, zrsd[x]);
+            conj[x] = p;
+         }
+         const float f = fld2 ? fld[x] + fld2[x] : fld[x];
+         const float v = A.polinv[s] * p - f;
+         vec[x] = v;
+         if (e - 6 * s < 3)
+            dd += p * v;
+         else
+            dp += p * v;
       }
-      const float f = fld2 ? fld[x] + fld2[x] : fld[x];
-      const float v = A.polinv[s] * p - f;
-      vec[x] = v;
-      if (e - 6 * s < 3)
-         dd += p * v;
-      else
-         dp += p * v;
+      const float pv[2] = {dd, dp};
+      store_partials_f<2>(red, R_PAP_D, pv, sh, vb);
    }
-   const float pv[2] = {dd, dp};
    pdl_trigger();
-   store_partials_f<2>(red, R_PAP_D, pv, sh);
    if (!last_block(state + ST_TICKET1))
       return;
    double tot[2];
-   sum_slots(red, R_PAP_D, 2, gridDim.x, sh, tot);
+   sum_slots(red, R_PAP_D, 2, A.nb, sh, tot);
    const double pap_d = tot[0], pap_p = tot[1];
    if (threadIdx.x == 0) {  // the step lengths in FP32 (used as FP32)
       scal[S_A_D] = pap_d == 0 ? 0.0 : (double)((float)scal[S_SUM_D] / (float)pap_d);
@@ -276,12 +293,27 @@ __global__ void k_pcg_peek_save(VecArgs A, float* __restrict__ uind, const float
    }
 }
 
-__global__ void k_bump_nualt(int* state, int depth)
+// End of a solve: the ring count, then the status words, the scalars and the
+// list's largest row into the host's pinned mirrors (one kernel where a bump
+// and three copies took four steps of the graph).
+__global__ void k_finish(int* state, int depth, const double* __restrict__ scal, const int* __restrict__ over,
+   int* __restrict__ h_status, double* __restrict__ h_scal, int* __restrict__ h_over)
 {
-   int v = state[ST_NUALT] + 1;
-   if (v > 2 * depth)
-      v -= depth;
-   state[ST_NUALT] = v;
+   const int t = threadIdx.x;
+   if (t < ST_NSTAT) {
+      int v = state[t];
+      if (t == ST_NUALT && depth > 0) {
+         v += 1;
+         if (v > 2 * depth)
+            v -= depth;
+         state[t] = v;
+      }
+      h_status[t] = v;
+   }
+   if (t < S_NSCAL)
+      h_scal[t] = scal[t];
+   if (t == 0)
+      *h_over = *over;
 }
 
 // ---------------------------------------------------------------------------
@@ -670,9 +702,8 @@ static int list_refresh_graph(Context* ctx)
    if (cudaStreamEndCapture(ctx->cap_stream, &tmp) != cudaSuccess && rc == T9GB_OK)
       rc = T9GB_CUDA_ERR;
    T9_CHECK(rc);
-   T9_CHECK(launch_list_filter(ctx));
-   T9_CUDA(cudaMemcpyAsync(ctx->h_over, ctx->nbr_over, sizeof(int), cudaMemcpyDeviceToHost, s0));
-   return T9GB_OK;
+   // the largest row reaches the host with the solve's status (k_finish)
+   return launch_list_filter(ctx);
 }
 
 // after a synchronisation: grow the list if an atom had more neighbours than
@@ -755,6 +786,9 @@ static int dfield6(Context* ctx, float* out6)
    return launch_dfield_recip_gather(ctx, out6, true);
 }
 
+// blocks of the Ap kernel: four per SM of 152
+static int p1_blocks(const VecArgs& A) { return std::min(A.nb, 608); }
+
 // z = M r with r.z, r.r and the CG scalars: one fused kernel for the sparse
 // preconditioner, else the preconditioner and the dot kernel
 static int precond_dots(Context* ctx, const VecArgs& A, int init, cudaGraphConditionalHandle handle,
@@ -799,7 +833,7 @@ static int pcg_body(Context* ctx, const VecArgs& A, cudaGraphConditionalHandle h
          T9_CHECK(launch_ufield_recip_gather_ap(ctx, ctx->fld6, P));
       } else {
          T9_CHECK(launch_ufield_recip_gather_dir(ctx, ctx->fld6, P));
-         k_pcg_p1<true><<<A.nb, VB, 0, ctx->stream>>>(A, ctx->fld6, nullptr, ctx->conj, ctx->zrsd, ctx->vec,
+         k_pcg_p1<true><<<p1_blocks(A), VB, 0, ctx->stream>>>(A, ctx->fld6, nullptr, ctx->conj, ctx->zrsd, ctx->vec,
             ctx->red, ctx->scal, ctx->status);
       }
    } else {
@@ -843,7 +877,7 @@ static int pcg_body(Context* ctx, const VecArgs& A, cudaGraphConditionalHandle h
          T9_CHECK(ufield6(ctx, ctx->conj, ctx->fld6));
       }
       prof_begin(ctx, P_VECTOR);
-      T9_CUDA(launch_k(pdl, k_pcg_p1<false>, A.nb, VB, 0, ctx->stream, A, ctx->fld6, rcp, ctx->conj, nullptr,
+      T9_CUDA(launch_k(pdl, k_pcg_p1<false>, p1_blocks(A), VB, 0, ctx->stream, A, ctx->fld6, rcp, ctx->conj, nullptr,
          ctx->vec, ctx->red, ctx->scal, ctx->status));
       prof_end(ctx);
    }
@@ -870,11 +904,9 @@ enum { V_PLAIN = 0, V_LEARNED = 1, V_COMPARE = 2, V_PREDICT = 3 };
 static int pcg_start_predict(Context* ctx, const VecArgs& A, bool graph)
 {
    const t9gb_config& c = ctx->cfg;
-   k_predict<<<A.nb, VB, 0, ctx->stream>>>(A, c.predictor, ctx->aspc_hist, ctx->status, ctx->uind, ctx->lx_coef);
-   T9_CUDA(cudaGetLastError());
    // the two reciprocal grids need no neighbour list: they start first and
    // run beside the list refresh (side 0: the permanent grid; side 3: the
-   // guess's grid on the second grid pair)
+   // guess and its grid on the second grid pair)
    T9_CHECK(recip_fork(ctx, 0));
    T9_CHECK(recip_fork(ctx, 3));
    cudaStream_t main = ctx->stream;
@@ -882,7 +914,11 @@ static int pcg_start_predict(Context* ctx, const VecArgs& A, bool graph)
    int rc = launch_dfield_recip_grid(ctx);
    if (rc == T9GB_OK) {
       ctx->stream = ctx->side_stream[3];
-      rc = launch_ufield_recip_grid_alt(ctx, ctx->uind);
+      k_predict<<<A.nb, VB, 0, ctx->stream>>>(A, c.predictor, ctx->aspc_hist, ctx->status, ctx->uind, ctx->lx_coef);
+      if (cudaGetLastError() != cudaSuccess || cudaEventRecord(ctx->ev_guess, ctx->stream) != cudaSuccess)
+         rc = T9GB_CUDA_ERR;
+      else
+         rc = launch_ufield_recip_grid_alt(ctx, ctx->uind);
    }
    ctx->stream = main;
    T9_CHECK(rc);
@@ -891,7 +927,9 @@ static int pcg_start_predict(Context* ctx, const VecArgs& A, bool graph)
    // grid), the permanent one here (then its gather)
    T9_CHECK(recip_fork(ctx, 2));
    ctx->stream = ctx->side_stream[2];
-   rc = launch_ufield_real(ctx, ctx->uind, nullptr, ctx->tmp6);
+   rc = cudaStreamWaitEvent(ctx->stream, ctx->ev_guess, 0) == cudaSuccess ? T9GB_OK : T9GB_CUDA_ERR;
+   if (rc == T9GB_OK)
+      rc = launch_ufield_real(ctx, ctx->uind, nullptr, ctx->tmp6);
    if (rc == T9GB_OK && cudaEventRecord(ctx->ev_join[3], ctx->side_stream[3]) == cudaSuccess &&
       cudaStreamWaitEvent(ctx->side_stream[2], ctx->ev_join[3], 0) == cudaSuccess)
       rc = launch_ufield_recip_gather_alt(ctx, ctx->uind, ctx->tmp6);
@@ -903,12 +941,11 @@ static int pcg_start_predict(Context* ctx, const VecArgs& A, bool graph)
    T9_CHECK(recip_join(ctx, 0));
    T9_CHECK(launch_dfield_recip_gather(ctx, ctx->fld6, true));
    T9_CHECK(recip_join(ctx, 2));
-   k_init_guess<<<A.nb, VB, 0, ctx->stream>>>(A, ctx->fld6, ctx->efield, ctx->udir, ctx->uind, c.pcgguess,
-      c.predictor, ctx->aspc_hist, ctx->status, 0, ctx->lx_coef);
+   k_init_predicted<<<A.nb, VB, 0, ctx->stream>>>(A, ctx->fld6, ctx->tmp6, ctx->uind, ctx->efield, ctx->udir,
+      ctx->rsd);
+   T9_CUDA(cudaGetLastError());
    if (ctx->learn_mode & 1)
       T9_CHECK(learn_forward(ctx, false));
-   k_init_rsd<<<A.nb, VB, 0, ctx->stream>>>(A, ctx->tmp6, ctx->efield, ctx->udir, ctx->uind, ctx->rsd, 0);
-   T9_CUDA(cudaGetLastError());
    return precond_dots(ctx, A, 1, 0, 0);
 }
 
@@ -935,7 +972,7 @@ static int pcg_start(Context* ctx, const VecArgs& A, bool graph, int variant)
       T9_CHECK(dfield6(ctx, ctx->fld6));
    }
    k_init_guess<<<A.nb, VB, 0, ctx->stream>>>(A, ctx->fld6, ctx->efield, ctx->udir, ctx->uind, c.pcgguess,
-      c.predictor, ctx->aspc_hist, ctx->status, 1, ctx->lx_coef);
+      c.predictor, ctx->aspc_hist, ctx->status, ctx->lx_coef);
    // the network runs when its guess is used or when this solve trains it
    if ((ctx->learn_mode & 1) || variant != V_PLAIN)
       T9_CHECK(learn_forward(ctx, variant != V_PLAIN));
@@ -968,12 +1005,10 @@ static int pcg_finish(Context* ctx, const VecArgs& A)
          ctx->aspc_hist, ctx->status);
       T9_CUDA(cudaGetLastError());
    }
-   if (depth > 0)
-      k_bump_nualt<<<1, 1, 0, ctx->stream>>>(ctx->status, depth);
    if (ctx->learn_mode & 1)
       T9_CHECK(learn_train(ctx));
-   T9_CUDA(cudaMemcpyAsync(ctx->h_status, ctx->status, sizeof(int) * ST_NSTAT, cudaMemcpyDeviceToHost, ctx->stream));
-   T9_CUDA(cudaMemcpyAsync(ctx->h_scal, ctx->scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, ctx->stream));
+   k_finish<<<1, 32, 0, ctx->stream>>>(ctx->status, depth, ctx->scal, ctx->nbr_over, ctx->h_status, ctx->h_scal,
+      ctx->h_over);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
 }

@@ -164,9 +164,14 @@ static __device__ __forceinline__ void store_partials(double* red, int first, co
 // FP64 pipe of this GPU issues a warp instruction in tens of cycles, so the
 // per-thread and per-warp sums avoid it), the block's eight warp sums and
 // everything after them in FP64; the same fixed order, so deterministic
+// slot: the block's place among the partials (its index, unless a block forms
+// the partials of several in turn)
 template <int N>
-static __device__ __forceinline__ void store_partials_f(double* red, int first, const float* v, double* sh)
+static __device__ __forceinline__ void store_partials_f(double* red, int first, const float* v, double* sh,
+   int slot = -1)
 {
+   if (slot < 0)
+      slot = blockIdx.x;
    float x[N];
 #pragma unroll
    for (int c = 0; c < N; ++c)
@@ -187,28 +192,29 @@ static __device__ __forceinline__ void store_partials_f(double* red, int first, 
       double r = 0.0;
       for (int k = 0; k < nw; ++k)
          r += sh[threadIdx.x * 8 + k];
-      red[(first + threadIdx.x) * RED_MAX + blockIdx.x] = r;
+      red[(first + threadIdx.x) * RED_MAX + slot] = r;
    }
    __syncthreads();
 }
 
 // true in the block that finishes last (threadfence + ticket); it resets the
-// ticket for the next launch
+// ticket for the next launch.  The barrier orders the block's writes before
+// thread 0's fence, and the fence is cumulative over them: one fence per block
+// and not one per warp, which each wait for all of the warp's stores.
 static __device__ __forceinline__ bool last_block(int* ticket)
 {
    __shared__ bool last;
-   __threadfence();
    __syncthreads();
    if (threadIdx.x == 0) {
+      __threadfence();
       unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(ticket), 1u);
       last = prev == gridDim.x - 1;
+      if (last) {
+         __threadfence();
+         *ticket = 0;
+      }
    }
    __syncthreads();
-   if (last) {
-      __threadfence();
-      if (threadIdx.x == 0)
-         *ticket = 0;
-   }
    return last;
 }
 
