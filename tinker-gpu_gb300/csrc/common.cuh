@@ -450,7 +450,7 @@ constexpr int STAGE_JB_CAP = 48;
 
 // energy / virial row sums: at most SUM_ROWS_MAX rows per launch, each
 // split over SUM_PARTS blocks
-constexpr int SUM_ROWS_MAX = 32, SUM_PARTS = 8;
+constexpr int SUM_ROWS_MAX = 32, SUM_PARTS = 32;
 constexpr int RED_MAX = 2048;
 constexpr int RED_SLOTS = 8;
 
@@ -699,6 +699,9 @@ void drop_graphs(Context* ctx);  // pcg.cu
 // <= 3 blocks of 9 FP32 virial rows, summed and symmetrised)
 int sum_rows_d(Context* ctx, const double* rows, int nrows, double* out);
 int sum_rows_virial(Context* ctx, const float* rows, int nblocks, double* virial);
+// the sums of rows of n entries, stride apart, into device memory
+int sum_rows_dev(Context* ctx, int nrows, int n, int stride, const double* rows, double* out);
+int sum_rows_dev(Context* ctx, int nrows, int n, int stride, const float* rows, double* out);
 // vdw.cu: reduced sites, pair kernel and per-atom gather (grad: dE/dx added
 // to or stored in grad when not null); energy rows in e_atom[2 npad ..)
 int vdw_forces(Context* ctx, float* grad, bool add, bool vir, double* energy);

@@ -683,17 +683,18 @@ struct SplineParams {
 };
 
 // copy (may be null): the coordinates in the caller's order as well.
-__global__ void k_scatter_pos(int npad, const int* __restrict__ perm, const float* __restrict__ xyz,
-   float* __restrict__ copy, const float2* __restrict__ sdamp, float4* __restrict__ spos, SplineParams S)
+constexpr int SCATTER_SLOTS = 64;  // per block of 192 threads
+
+__global__ void __launch_bounds__(3 * SCATTER_SLOTS) k_scatter_pos(int npad, const int* __restrict__ perm,
+   const float* __restrict__ xyz, float* __restrict__ copy, const float2* __restrict__ sdamp,
+   float4* __restrict__ spos, SplineParams S)
 {
-   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 3 * npad; e += gridDim.x * blockDim.x) {
-      const int s = e / 3, d = e - 3 * s;
-      const int a = perm[s];
-      if (a < 0) {
-         if (d == 0)
-            spos[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-         continue;
-      }
+   // the tables leave through shared memory: each thread's 10 words of a row
+   // would be written eight bytes at a time (21 -> 9 us at 98,304 atoms)
+   __shared__ float4 lo[SCATTER_SLOTS * SPL_ROW / 4], hi[SCATTER_SLOTS * SPL_ROW / 4];
+   const int q = threadIdx.x / 3, d = threadIdx.x - 3 * q, s0 = blockIdx.x * SCATTER_SLOTS, s = s0 + q;
+   const int a = s < npad ? perm[s] : -1;
+   if (a >= 0) {
       const float x = xyz[3 * a + d];
       if (copy)
          copy[3 * a + d] = x;
@@ -702,9 +703,21 @@ __global__ void k_scatter_pos(int npad, const int* __restrict__ perm, const floa
       if (S.nfft[0]) {
          const float rb = d == 0 ? S.r[0] : d == 1 ? S.r[1] : S.r[2];
          const int nf = d == 0 ? S.nfft[0] : d == 1 ? S.nfft[1] : S.nfft[2];
-         reinterpret_cast<int*>(S.org)[4 * s + d] =
-            spline_axis(x, rb, nf, d, S.lo + (size_t)SPL_ROW * s, S.hi + (size_t)SPL_ROW * s);
+         reinterpret_cast<int*>(S.org)[4 * s + d] = spline_axis(x, rb, nf, d,
+            reinterpret_cast<float*>(lo) + SPL_ROW * q, reinterpret_cast<float*>(hi) + SPL_ROW * q);
       }
+   } else if (s < npad && d == 0) {
+      spos[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+   }
+   if (!S.nfft[0])
+      return;
+   __syncthreads();
+   const int m = min(SCATTER_SLOTS, npad - s0) * (SPL_ROW / 4);
+   float4* glo = reinterpret_cast<float4*>(S.lo + (size_t)SPL_ROW * s0);
+   float4* ghi = reinterpret_cast<float4*>(S.hi + (size_t)SPL_ROW * s0);
+   for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      glo[k] = lo[k];
+      ghi[k] = hi[k];
    }
 }
 
@@ -721,7 +734,7 @@ int scatter_positions(Context* ctx, const float* src)
       S.lo = ctx->pme.spl_lo;
       S.hi = ctx->pme.spl_hi;
    }
-   k_scatter_pos<<<grid_for(3 * (long long)ctx->npad, 256), 256, 0, ctx->stream>>>(ctx->npad, ctx->perm,
+   k_scatter_pos<<<grid_for(ctx->npad, SCATTER_SLOTS), 3 * SCATTER_SLOTS, 0, ctx->stream>>>(ctx->npad, ctx->perm,
       src ? src : ctx->xyz, src && src != ctx->xyz ? ctx->xyz : nullptr, ctx->sdamp, ctx->spos, S);
    T9_CUDA(cudaGetLastError());
    ctx->list_stale = true;

@@ -207,38 +207,34 @@ __global__ void k_pcg_p1(VecArgs A, const float* __restrict__ fld, const float* 
 {
    pdl_wait();
    __shared__ double sh[64];
+   float dd = 0.f, dp = 0.f;
    float bd = 0.f, bp = 0.f;
    if (DIR) {
       bd = (float)scal[S_B_D];
       bp = (float)scal[S_B_P];
    }
-   // a block forms the partials of up to four of the A.nb element blocks in
-   // turn: 2,048 tickets at one address cost more than the sums themselves
-   for (int vb = blockIdx.x; vb < A.nb; vb += gridDim.x) {
-      float dd = 0.f, dp = 0.f;
-      for (int e = vb * blockDim.x + threadIdx.x; e < A.ne; e += A.nb * blockDim.x) {
-         const int s = e / 6, x = e + 2 * s;  // row s, component e - 6 s of [npad][8]
-         float p = conj[x];
-         if (DIR) {
-            p = __fmaf_rn(e - 6 * s < 3 ? bd : bp, p, zrsd[x]);
-            conj[x] = p;
-         }
-         const float f = fld2 ? fld[x] + fld2[x] : fld[x];
-         const float v = A.polinv[s] * p - f;
-         vec[x] = v;
-         if (e - 6 * s < 3)
-            dd += p * v;
-         else
-            dp += p * v;
+   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < A.ne; e += gridDim.x * blockDim.x) {
+      const int s = e / 6, x = e + 2 * s;  // row s, component e - 6 s of [npad][8]
+      float p = conj[x];
+      if (DIR) {
+         p = __fmaf_rn(e - 6 * s < 3 ? bd : bp, p, zrsd[x]);
+         conj[x] = p;
       }
-      const float pv[2] = {dd, dp};
-      store_partials_f<2>(red, R_PAP_D, pv, sh, vb);
+      const float f = fld2 ? fld[x] + fld2[x] : fld[x];
+      const float v = A.polinv[s] * p - f;
+      vec[x] = v;
+      if (e - 6 * s < 3)
+         dd += p * v;
+      else
+         dp += p * v;
    }
+   const float pv[2] = {dd, dp};
    pdl_trigger();
+   store_partials_f<2>(red, R_PAP_D, pv, sh);
    if (!last_block(state + ST_TICKET1))
       return;
    double tot[2];
-   sum_slots(red, R_PAP_D, 2, A.nb, sh, tot);
+   sum_slots(red, R_PAP_D, 2, gridDim.x, sh, tot);
    const double pap_d = tot[0], pap_p = tot[1];
    if (threadIdx.x == 0) {  // the step lengths in FP32 (used as FP32)
       scal[S_A_D] = pap_d == 0 ? 0.0 : (double)((float)scal[S_SUM_D] / (float)pap_d);
@@ -786,9 +782,6 @@ static int dfield6(Context* ctx, float* out6)
    return launch_dfield_recip_gather(ctx, out6, true);
 }
 
-// blocks of the Ap kernel: four per SM of 152
-static int p1_blocks(const VecArgs& A) { return std::min(A.nb, 608); }
-
 // z = M r with r.z, r.r and the CG scalars: one fused kernel for the sparse
 // preconditioner, else the preconditioner and the dot kernel
 static int precond_dots(Context* ctx, const VecArgs& A, int init, cudaGraphConditionalHandle handle,
@@ -833,7 +826,7 @@ static int pcg_body(Context* ctx, const VecArgs& A, cudaGraphConditionalHandle h
          T9_CHECK(launch_ufield_recip_gather_ap(ctx, ctx->fld6, P));
       } else {
          T9_CHECK(launch_ufield_recip_gather_dir(ctx, ctx->fld6, P));
-         k_pcg_p1<true><<<p1_blocks(A), VB, 0, ctx->stream>>>(A, ctx->fld6, nullptr, ctx->conj, ctx->zrsd, ctx->vec,
+         k_pcg_p1<true><<<A.nb, VB, 0, ctx->stream>>>(A, ctx->fld6, nullptr, ctx->conj, ctx->zrsd, ctx->vec,
             ctx->red, ctx->scal, ctx->status);
       }
    } else {
@@ -877,7 +870,7 @@ static int pcg_body(Context* ctx, const VecArgs& A, cudaGraphConditionalHandle h
          T9_CHECK(ufield6(ctx, ctx->conj, ctx->fld6));
       }
       prof_begin(ctx, P_VECTOR);
-      T9_CUDA(launch_k(pdl, k_pcg_p1<false>, p1_blocks(A), VB, 0, ctx->stream, A, ctx->fld6, rcp, ctx->conj, nullptr,
+      T9_CUDA(launch_k(pdl, k_pcg_p1<false>, A.nb, VB, 0, ctx->stream, A, ctx->fld6, rcp, ctx->conj, nullptr,
          ctx->vec, ctx->red, ctx->scal, ctx->status));
       prof_end(ctx);
    }

@@ -164,14 +164,9 @@ static __device__ __forceinline__ void store_partials(double* red, int first, co
 // FP64 pipe of this GPU issues a warp instruction in tens of cycles, so the
 // per-thread and per-warp sums avoid it), the block's eight warp sums and
 // everything after them in FP64; the same fixed order, so deterministic
-// slot: the block's place among the partials (its index, unless a block forms
-// the partials of several in turn)
 template <int N>
-static __device__ __forceinline__ void store_partials_f(double* red, int first, const float* v, double* sh,
-   int slot = -1)
+static __device__ __forceinline__ void store_partials_f(double* red, int first, const float* v, double* sh)
 {
-   if (slot < 0)
-      slot = blockIdx.x;
    float x[N];
 #pragma unroll
    for (int c = 0; c < N; ++c)
@@ -192,7 +187,7 @@ static __device__ __forceinline__ void store_partials_f(double* red, int first, 
       double r = 0.0;
       for (int k = 0; k < nw; ++k)
          r += sh[threadIdx.x * 8 + k];
-      red[(first + threadIdx.x) * RED_MAX + slot] = r;
+      red[(first + threadIdx.x) * RED_MAX + blockIdx.x] = r;
    }
    __syncthreads();
 }

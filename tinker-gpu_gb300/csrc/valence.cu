@@ -128,25 +128,6 @@ __global__ void k_valence_gather(int n, const int* __restrict__ start, const int
    }
 }
 
-// block b sums rows[b][0..m) (FP64 out[b]); one block per row
-__global__ void k_rows_sum(int m, const float* __restrict__ rows, const double* __restrict__ drow,
-   double* __restrict__ out)
-{
-   __shared__ double sh[256];
-   double v = 0;
-   for (int i = threadIdx.x; i < m; i += blockDim.x)
-      v += drow ? drow[i] : (double)rows[(size_t)blockIdx.x * m + i];
-   sh[threadIdx.x] = v;
-   __syncthreads();
-   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-      if (threadIdx.x < o)
-         sh[threadIdx.x] += sh[threadIdx.x + o];
-      __syncthreads();
-   }
-   if (threadIdx.x == 0)
-      out[blockIdx.x] = sh[0];
-}
-
 static void val_free(Context* ctx)
 {
    void* p[] = {ctx->val_idx, ctx->val_par, ctx->val_g, ctx->val_e, ctx->val_w, ctx->val_start, ctx->val_ent,
@@ -218,10 +199,9 @@ int valence_sums(Context* ctx, double* energy, double* virial)
             virial[c] = 0;
       return T9GB_OK;
    }
-   k_rows_sum<<<1, 256, 0, ctx->stream>>>(ctx->nval, nullptr, ctx->val_e, ctx->val_sum);
+   T9_CHECK(sum_rows_dev(ctx, 1, ctx->nval, ctx->nval, ctx->val_e, ctx->val_sum));
    if (virial)
-      k_rows_sum<<<9, 256, 0, ctx->stream>>>(ctx->nval, ctx->val_w, nullptr, ctx->val_sum + 1);
-   T9_CUDA(cudaGetLastError());
+      T9_CHECK(sum_rows_dev(ctx, 9, ctx->nval, ctx->nval, ctx->val_w, ctx->val_sum + 1));
    double h[10];
    T9_CUDA(cudaMemcpyAsync(h, ctx->val_sum, sizeof(double) * 10, cudaMemcpyDeviceToHost, ctx->stream));
    T9_CUDA(cudaStreamSynchronize(ctx->stream));
