@@ -1112,38 +1112,6 @@ __global__ void k_conv_virial(int n1, int n2, int n3, float L1, float L2, float 
 // force/torque parts of empoleEwaldRecipGeneric_cu (src/cu/hippo/empole.cu)
 // and epolarEwaldRecipSelf_cu1 (src/cu/epolarrecip.cu:414-511).
 
-__device__ __forceinline__ void row_sums20(const float2* __restrict__ g, const GridParams& G, int i1, size_t row,
-   const float (*t1)[4], bool imag, float* t)
-{
-   t[0] = t[1] = t[2] = t[3] = 0.f;
-#pragma unroll
-   for (int ix = 0; ix < 5; ++ix) {
-      int xb = i1 + ix;
-      xb -= (xb >= G.n1 ? G.n1 : 0);
-      const float2 qv = g[row + xb];
-      const float q = imag ? qv.y : qv.x;
-#pragma unroll
-      for (int l = 0; l < 4; ++l)
-         t[l] += q * t1[ix][l];
-   }
-}
-
-// row idx of a [5][L] weight table without dynamic indexing (keeps the
-// table in registers)
-template <int L>
-__device__ __forceinline__ void pick_row(const float (*t)[L], int idx, float* out)
-{
-#pragma unroll
-   for (int l = 0; l < L; ++l)
-      out[l] = t[0][l];
-#pragma unroll
-   for (int j = 1; j < 5; ++j)
-      if (idx == j)
-#pragma unroll
-         for (int l = 0; l < L; ++l)
-            out[l] = t[j][l];
-}
-
 __device__ __forceinline__ void fphi20(const float* t, const float* u, const float* v, float* phi)
 {
    phi[0] = t[0] * u[0] * v[0];
@@ -1237,52 +1205,114 @@ __device__ __forceinline__ void mpole_force(const float* m, const float* c, floa
    }
 }
 
+// The 20 sums of one atom over its 125 points (IMAG: of both parts), value k
+// left in out[k] (out[20 + k] the imaginary part's), shared memory.  The points
+// are loaded and exchanged as in gather_atom; lane (jy, kz) then sums its row
+// with the four x levels, forms its 20 products and the halving tree adds the
+// rows in the order of an xor tree (23 shuffles where 20 trees take 100).
+template <bool IMAG>
+__device__ __forceinline__ void force_sums(int s, int lane, const GridParams& G, const Sites& S,
+   const float2* __restrict__ g, float2* xch, float* out)
+{
+   const int4 o = S.org[s];
+   const float* lo = S.lo + (size_t)SPL_ROW * s;
+   const float* hi = S.hi + (size_t)SPL_ROW * s;
+   const int q5 = lane % 5, d5 = lane / 5;  // (ix, jy) loading, (jy, kz) summing
+   float* xr = reinterpret_cast<float*>(xch);
+   if (lane < 25) {
+      const unsigned plane = plane_bytes(G);
+      const char* col = reinterpret_cast<const char*>(g) + column_bytes(G, o, q5, d5);
+      float2 q[5];
+#pragma unroll
+      for (int kz = 0; kz < 5; ++kz) {
+         int zb = o.z + kz;
+         zb -= (zb >= G.n3 ? G.n3 : 0);
+         const float2* p = reinterpret_cast<const float2*>(col + (size_t)(unsigned)zb * plane);
+         if (IMAG)
+            q[kz] = *p;
+         else
+            q[kz].x = p->x;
+      }
+#pragma unroll
+      for (int kz = 0; kz < 5; ++kz)
+         if (IMAG)
+            xch[25 * kz + lane] = q[kz];
+         else
+            xr[25 * kz + lane] = q[kz].x;
+   }
+   __syncwarp();
+   float phi[20], psi[20];
+#pragma unroll
+   for (int c = 0; c < 20; ++c)
+      phi[c] = psi[c] = 0.f;
+   if (lane < 25) {
+      float t[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int ix = 0; ix < 5; ++ix) {
+         const float2 a = spl(lo, 0, ix), b = spl(hi, 0, ix);
+         float2 qv;
+         if (IMAG)
+            qv = xch[5 * lane + ix];
+         else
+            qv.x = xr[5 * lane + ix];
+         t[0] += qv.x * a.x;
+         t[1] += qv.x * a.y;
+         t[2] += qv.x * b.x;
+         t[3] += qv.x * b.y;
+         if (IMAG) {
+            w[0] += qv.y * a.x;
+            w[1] += qv.y * a.y;
+            w[2] += qv.y * b.x;
+            w[3] += qv.y * b.y;
+         }
+      }
+      const float2 ua = spl(lo, 1, q5), ub = spl(hi, 1, q5), va = spl(lo, 2, d5), vb = spl(hi, 2, d5);
+      const float u[4] = {ua.x, ua.y, ub.x, ub.y}, v[4] = {va.x, va.y, vb.x, vb.y};
+      fphi20(t, u, v, phi);
+      if (IMAG)
+         fphi20(w, u, v, psi);
+   }
+   const float a = warp_sums<20>(phi, lane);
+   const int c = sum_slot<20>(lane);
+   if (c >= 0)
+      out[c] = a;
+   if (IMAG) {
+      const float b = warp_sums<20>(psi, lane);
+      if (c >= 0)
+         out[20 + c] = b;
+   }
+   __syncwarp();
+}
+
+// Each warp sums FA consecutive atoms, then its first FA lanes finish one atom
+// each (one lane finishing each atom as it is summed takes 300 to 400 warp
+// instructions an atom).
+constexpr int FORCE_WARPS = 8;
+
 // permanent grid: multipole forces, torque field and energies (MPOLE), the
 // polarization force on the dipoles in the permanent field gradient and the
 // Ewald self torque (POLAR)
 // wout (may be null): the fractional-transform part of the virial per slot,
 // [9][npad]; the dipole-grid gather adds to the same rows
-template <bool MPOLE, bool POLAR>
-__global__ void __launch_bounds__(256) k_gather_force_perm(int n, int npad, GridParams G, float f, float aewald,
-   const float4* __restrict__ spos, const float2* __restrict__ g, const float* __restrict__ rp,
+template <bool MPOLE, bool POLAR, int FA>
+__global__ void __launch_bounds__(32 * FORCE_WARPS) k_gather_force_perm(int n, int npad, GridParams G, float f,
+   float aewald, Sites S, const float2* __restrict__ g, const float* __restrict__ rp,
    const float* __restrict__ u8, float* __restrict__ fout, float* __restrict__ tout, double* __restrict__ e_atom,
    double* __restrict__ e_self, float* __restrict__ wout)
 {
-   const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-   const int lane = threadIdx.x & 31;
-   if (s >= n)
+   __shared__ float2 xch[FORCE_WARPS][125];
+   __shared__ float sums[FORCE_WARPS][FA][21];
+   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+   const int s0 = (blockIdx.x * FORCE_WARPS + w) * FA;
+   for (int a = 0; a < FA && s0 + a < n; ++a)
+      force_sums<false>(s0 + a, lane, G, S, g, xch[w], sums[w][a]);
+   const int s = s0 + lane;
+   if (lane >= FA || s >= n)
       return;
-   int i1, i2, i3;
-   float w1, w2, w3;
-   site(G, spos[s], i1, i2, i3, w1, w2, w3);
    float phi[20];
 #pragma unroll
    for (int c = 0; c < 20; ++c)
-      phi[c] = 0.f;
-   if (lane < 25) {
-      float t1[5][4], t2[5][4], t3[5][4];
-      bspline5<4>(w1, t1);
-      bspline5<4>(w2, t2);
-      bspline5<4>(w3, t3);
-      const int jy = lane % 5, kz = lane / 5;
-      int zb = i3 + kz;
-      zb -= (zb >= G.n3 ? G.n3 : 0);
-      int yb = i2 + jy;
-      yb -= (yb >= G.n2 ? G.n2 : 0);
-      const size_t row = ((size_t)zb * G.n2 + yb) * G.n1;
-      float t[4], uy[4], vz[4];
-      pick_row<4>(t2, jy, uy);
-      pick_row<4>(t3, kz, vz);
-      row_sums20(g, G, i1, row, t1, false, t);
-      fphi20(t, uy, vz, phi);
-   }
-#pragma unroll
-   for (int c = 0; c < 20; ++c)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-         phi[c] += __shfl_xor_sync(0xffffffffu, phi[c], o);
-   if (lane != 0)
-      return;
+      phi[c] = sums[w][lane][c];
    to_cart20(G, phi);
    const float* m = rp + 12 * s;
    float F[3] = {0.f, 0.f, 0.f}, T[10];
@@ -1361,49 +1391,26 @@ __global__ void __launch_bounds__(256) k_gather_force_perm(int n, int npad, Grid
 
 // induced-dipole grid (d real, p imaginary): force on the multipoles in the
 // dipoles' potential, the mutual dipole force and the torque field
-__global__ void __launch_bounds__(256) k_gather_force_uind(int n, int npad, GridParams G, float f,
-   const float4* __restrict__ spos, const float2* __restrict__ g, const float* __restrict__ rp,
+template <int FA>
+__global__ void __launch_bounds__(32 * FORCE_WARPS) k_gather_force_uind(int n, int npad, GridParams G, float f,
+   Sites S, const float2* __restrict__ g, const float* __restrict__ rp,
    const float* __restrict__ u8, float* __restrict__ fout, float* __restrict__ tout, float* __restrict__ wout)
 {
-   const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-   const int lane = threadIdx.x & 31;
-   if (s >= n)
+   __shared__ float2 xch[FORCE_WARPS][125];
+   __shared__ float sums[FORCE_WARPS][FA][41];
+   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+   const int s0 = (blockIdx.x * FORCE_WARPS + w) * FA;
+   for (int a = 0; a < FA && s0 + a < n; ++a)
+      force_sums<true>(s0 + a, lane, G, S, g, xch[w], sums[w][a]);
+   const int s = s0 + lane;
+   if (lane >= FA || s >= n)
       return;
-   int i1, i2, i3;
-   float w1, w2, w3;
-   site(G, spos[s], i1, i2, i3, w1, w2, w3);
    float pd[20], pp[20];
 #pragma unroll
-   for (int c = 0; c < 20; ++c)
-      pd[c] = pp[c] = 0.f;
-   if (lane < 25) {
-      float t1[5][4], t2[5][4], t3[5][4];
-      bspline5<4>(w1, t1);
-      bspline5<4>(w2, t2);
-      bspline5<4>(w3, t3);
-      const int jy = lane % 5, kz = lane / 5;
-      int zb = i3 + kz;
-      zb -= (zb >= G.n3 ? G.n3 : 0);
-      int yb = i2 + jy;
-      yb -= (yb >= G.n2 ? G.n2 : 0);
-      const size_t row = ((size_t)zb * G.n2 + yb) * G.n1;
-      float t[4], uy[4], vz[4];
-      pick_row<4>(t2, jy, uy);
-      pick_row<4>(t3, kz, vz);
-      row_sums20(g, G, i1, row, t1, false, t);
-      fphi20(t, uy, vz, pd);
-      row_sums20(g, G, i1, row, t1, true, t);
-      fphi20(t, uy, vz, pp);
+   for (int c = 0; c < 20; ++c) {
+      pd[c] = sums[w][lane][c];
+      pp[c] = sums[w][lane][20 + c];
    }
-#pragma unroll
-   for (int c = 0; c < 20; ++c)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-         pd[c] += __shfl_xor_sync(0xffffffffu, pd[c], o);
-         pp[c] += __shfl_xor_sync(0xffffffffu, pp[c], o);
-      }
-   if (lane != 0)
-      return;
    to_cart20(G, pd);
    to_cart20(G, pp);
    float ps[20];
@@ -1799,6 +1806,10 @@ int launch_empole_recip(Context* ctx, double* e_atom)
 }  // namespace t9gb
 
 namespace t9gb {
+// atoms per warp of the force gathers: eight where that still gives an SM 20
+// warps, four below
+static int force_atoms(int n) { return n > 24576 ? 8 : 4; }
+
 // reciprocal forces for elec_forces (force.cu), in two halves: the
 // permanent-multipole grid (forces and torque fields of the multipoles, the
 // induced dipoles' force in the permanent field) and the induced-dipole
@@ -1823,15 +1834,12 @@ int launch_force_recip_perm(Context* ctx, bool mpole, bool polar, float* wrec)
    T9_CHECK(fft_conv(ctx, vir ? 1 : 0, mpole ? 0.5f * f : 0.f, 0.f, vir && polar, ctx->scal + 40));
    double* er = ctx->e_atom + np;
    double* es = ctx->e_atom + 2 * np;
-   if (mpole && polar)
-      k_gather_force_perm<true, true><<<nb, 256, 0, ctx->stream>>>(ctx->n, np, G, f, a, ctx->spos, ctx->pme.qgrid,
-         ctx->srpole, ctx->uind, ctx->frecp, ctx->trecp, er, es, wrec);
-   else if (mpole)
-      k_gather_force_perm<true, false><<<nb, 256, 0, ctx->stream>>>(ctx->n, np, G, f, a, ctx->spos, ctx->pme.qgrid,
-         ctx->srpole, ctx->uind, ctx->frecp, ctx->trecp, er, es, wrec);
-   else
-      k_gather_force_perm<false, true><<<nb, 256, 0, ctx->stream>>>(ctx->n, np, G, f, a, ctx->spos, ctx->pme.qgrid,
-         ctx->srpole, ctx->uind, ctx->frecp, ctx->trecp, nullptr, nullptr, wrec);
+   const int fa = force_atoms(ctx->n), fb = grid_for(ctx->n, FORCE_WARPS * fa);
+   auto k = mpole && polar ? (fa == 8 ? k_gather_force_perm<true, true, 8> : k_gather_force_perm<true, true, 4>)
+      : mpole              ? (fa == 8 ? k_gather_force_perm<true, false, 8> : k_gather_force_perm<true, false, 4>)
+                           : (fa == 8 ? k_gather_force_perm<false, true, 8> : k_gather_force_perm<false, true, 4>);
+   k<<<fb, 32 * FORCE_WARPS, 0, ctx->stream>>>(ctx->n, np, G, f, a, sites(ctx), ctx->pme.qgrid, ctx->srpole, ctx->uind,
+      ctx->frecp, ctx->trecp, mpole ? er : nullptr, mpole ? es : nullptr, wrec);
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
 }
@@ -1857,8 +1865,10 @@ int launch_force_recip_uind(Context* ctx, float* wrec, bool alt)
    if (rc == T9GB_OK)
       rc = fft_conv(ctx, vir ? 2 : 0, 0.f, 0.5f * f, false, ctx->scal + 46);
    if (rc == T9GB_OK) {
-      k_gather_force_uind<<<nb, 256, 0, ctx->stream>>>(ctx->n, ctx->npad, G, f, ctx->spos, P.qgrid, ctx->srpole,
-         ctx->uind, ctx->frecu, ctx->trecu, wrec);
+      const int fa = force_atoms(ctx->n);
+      auto k = fa == 8 ? k_gather_force_uind<8> : k_gather_force_uind<4>;
+      k<<<grid_for(ctx->n, FORCE_WARPS * fa), 32 * FORCE_WARPS, 0, ctx->stream>>>(ctx->n, ctx->npad, G, f, sites(ctx),
+         P.qgrid, ctx->srpole, ctx->uind, ctx->frecu, ctx->trecu, wrec);
       if (cudaGetLastError() != cudaSuccess)
          rc = T9GB_CUDA_ERR;
    }
