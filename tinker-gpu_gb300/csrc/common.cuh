@@ -620,6 +620,8 @@ struct PcgAp {
 int launch_precond_sparse_dots(Context* ctx, const float* r6, float* z6, const PcgDots& D);
 int launch_ufield_real_dir(Context* ctx, const float* p6, const float* z6, const double* scal, float* out6);
 int launch_ufield_recip_grid_dir(Context* ctx, const float* p6, const float* z6, const double* scal);
+int launch_ufield_spread_dir(Context* ctx, float* p6, const float* z6, const double* scal);
+int launch_ufield_transform(Context* ctx);
 int launch_ufield_recip_gather_ap(Context* ctx, float* out6, const PcgAp& P);
 int launch_ufield_recip_gather_dir(Context* ctx, float* out6, const PcgAp& P);
 // the same on the second grid (and FFT plan)

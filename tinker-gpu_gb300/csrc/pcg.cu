@@ -26,6 +26,11 @@
 namespace t9gb {
 
 constexpr int VB = 256;  // vector-kernel block size
+// boxes up to this size form the CG direction in the spread: a launch less in
+// an iteration, the real-space field a spread later (GB300, induce, 648 /
+// 3,000 / 6,300 / 12,288 atoms: 412 / 293 / 350 / 408 us, with a kernel of its
+// own 420 / 297 / 342 / 400)
+constexpr int DIR_SPREAD_MAX = 4096;
 
 // ASPC extrapolation weights (Kolafa, J. Comput. Chem. 25, 335 (2004)); the
 // reference tabulates them in src/cu/upredict.cu:40-55.
@@ -831,11 +836,30 @@ static int pcg_body(Context* ctx, const VecArgs& A, cudaGraphConditionalHandle h
       }
    } else {
       const bool pdl = use_pdl(ctx);
-      prof_begin(ctx, P_VECTOR);
-      T9_CUDA(launch_k(pdl, k_pcg_dir, A.nb, VB, 0, ctx->stream, A, ctx->scal, ctx->conj, ctx->zrsd));
-      prof_end(ctx);
+      const bool chain = ctx->cfg.use_ewald && (ctx->pcg_fuse & 96) == 96 && !ctx->prof.on;
+      const bool dir_in_spread = chain && ctx->npad <= DIR_SPREAD_MAX;
+      if (!dir_in_spread) {
+         prof_begin(ctx, P_VECTOR);
+         T9_CUDA(launch_k(pdl, k_pcg_dir, A.nb, VB, 0, ctx->stream, A, ctx->scal, ctx->conj, ctx->zrsd));
+         prof_end(ctx);
+      }
       const float* rcp = nullptr;
-      if (ctx->cfg.use_ewald && (ctx->pcg_fuse & 96) == 96 && !ctx->prof.on) {
+      if (dir_in_spread) {
+         // the spread forms and stores p (each row by its own warp), the
+         // real-space field starts behind it
+         T9_CHECK(launch_ufield_spread_dir(ctx, ctx->conj, ctx->zrsd, ctx->scal));
+         const int k = side_index(ctx);
+         T9_CHECK(recip_fork(ctx, k));
+         cudaStream_t main = ctx->stream;
+         ctx->stream = ctx->side_stream[k];
+         int rc = launch_ufield_real(ctx, ctx->conj, nullptr, ctx->fld6);
+         ctx->stream = main;
+         T9_CHECK(rc);
+         T9_CHECK(launch_ufield_transform(ctx));
+         T9_CHECK(launch_ufield_recip_gather(ctx, ctx->conj, ctx->rcp6, false));
+         T9_CHECK(recip_join(ctx, k));
+         rcp = ctx->rcp6;
+      } else if (chain) {
          // the reciprocal chain (spread, transform passes, gather into rcp6)
          // stays on this stream as programmatic dependents of the direction
          // kernel; the real-space field runs on the side stream

@@ -211,10 +211,12 @@ __device__ __forceinline__ float dot2(float a, float b, float c, float d)
 // part; MODE 1 spreads fractional d dipoles into the real and p dipoles into
 // the imaginary part.  rp rows are 12 floats (q, d, quadrupole, ...), u rows
 // 8.  DIR (MODE 1): the dipoles are the CG search direction p = z + b p_old
-// (src = p_old, z8 = z, b from scal), formed as each row is read.
+// (src = p_old, z8 = z, b from scal), formed as each row is read; dir8 (may
+// be null, else = src): p is stored there, each row by the one warp that
+// reads it.
 template <int MODE, bool DIR = false>
-__global__ void __launch_bounds__(256) k_spread(int n, GridParams G, Sites S, const float* __restrict__ src,
-   const float* __restrict__ z8, const double* __restrict__ scal, unsigned long long* __restrict__ q)
+__global__ void __launch_bounds__(256) k_spread(int n, GridParams G, Sites S, const float* src,
+   const float* __restrict__ z8, const double* __restrict__ scal, unsigned long long* __restrict__ q, float* dir8)
 {
    // the sites do not depend on the programmatic predecessor: they are read
    // before the wait for it (no-op otherwise)
@@ -267,10 +269,21 @@ __global__ void __launch_bounds__(256) k_spread(int n, GridParams G, Sites S, co
       pdl_wait();
       pdl_trigger();
       float u[8];
-      if (DIR)
+      if (DIR) {
          dir_row(src, z8, s, (float)scal[S_B_D], (float)scal[S_B_P], u);
-      else
+         if (dir8) {
+            __syncwarp(0x1ffffff);  // every lane has read the row
+            float v = u[0];
+#pragma unroll
+            for (int c = 1; c < 6; ++c)
+               if (lane == c)
+                  v = u[c];
+            if (lane < 6)
+               dir8[8 * s + lane] = v;
+         }
+      } else {
          load8(src, s, u);
+      }
       const float dx = G.a1 * u[0], dy = G.a2 * u[1], dz = G.a3 * u[2];
       const float px = G.a1 * u[3], py = G.a2 * u[4], pz = G.a3 * u[5];
       bool ok = true;
@@ -1654,7 +1667,7 @@ int launch_dfield_recip_grid(Context* ctx)
    prof_begin(ctx, P_SPREAD_MPOLE);
    ctx->pme.packed = false;
    k_spread<0><<<grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->srpole,
-      nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx));
+      nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx), nullptr);
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return fft_conv(ctx);
@@ -1692,7 +1705,7 @@ int launch_ufield_recip_grid(Context* ctx, const float* u6)
    prof_begin(ctx, P_SPREAD_UIND);
    ctx->pme.packed = true;
    T9_CUDA(launch_k(use_pdl(ctx), k_spread<1, false>, grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream,
-      ctx->n, G, sites(ctx), u6, nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx)));
+      ctx->n, G, sites(ctx), u6, nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx), nullptr));
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return fft_conv(ctx);
@@ -1750,11 +1763,24 @@ int launch_ufield_recip_grid_dir(Context* ctx, const float* p6, const float* z6,
    prof_begin(ctx, P_SPREAD_UIND);
    ctx->pme.packed = true;
    T9_CUDA(launch_k(use_pdl(ctx), k_spread<1, true>, grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream,
-      ctx->n, G, sites(ctx), p6, z6, scal, reinterpret_cast<unsigned long long*>(ctx->pme.qfx)));
+      ctx->n, G, sites(ctx), p6, z6, scal, reinterpret_cast<unsigned long long*>(ctx->pme.qfx), nullptr));
    prof_end(ctx);
    T9_CUDA(cudaGetLastError());
    return fft_conv(ctx);
 }
+
+// the CG search direction p = z + b p_old formed, stored in p6 and spread; its
+// transform
+int launch_ufield_spread_dir(Context* ctx, float* p6, const float* z6, const double* scal)
+{
+   GridParams G = grid_params(ctx);
+   ctx->pme.packed = true;
+   T9_CUDA(launch_k(use_pdl(ctx), k_spread<1, true>, grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream,
+      ctx->n, G, sites(ctx), p6, z6, scal, reinterpret_cast<unsigned long long*>(ctx->pme.qfx), p6));
+   return T9GB_OK;
+}
+
+int launch_ufield_transform(Context* ctx) { return fft_conv(ctx); }
 
 // recip + self field of the search direction p = z + b p_old (P.conj =
 // p_old, P.zrsd = z, P.scal = b) added to the real-space field in out6
@@ -1794,7 +1820,7 @@ int launch_empole_recip(Context* ctx, double* e_atom)
    GridParams G = grid_params(ctx);
    ctx->pme.packed = false;
    k_spread<0><<<grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->srpole,
-      nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx));
+      nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx), nullptr);
    T9_CUDA(cudaGetLastError());
    T9_CHECK(fft_conv(ctx));
    k_empole_recip_self<<<grid_for((long long)ctx->n * 32, 256), 256, 0, ctx->stream>>>(ctx->n, G,
@@ -1829,7 +1855,7 @@ int launch_force_recip_perm(Context* ctx, bool mpole, bool polar, float* wrec)
    }
    ctx->pme.packed = false;
    k_spread<0><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->srpole,
-      nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx));
+      nullptr, nullptr, reinterpret_cast<unsigned long long*>(ctx->pme.qfx), nullptr);
    T9_CUDA(cudaGetLastError());
    T9_CHECK(fft_conv(ctx, vir ? 1 : 0, mpole ? 0.5f * f : 0.f, 0.f, vir && polar, ctx->scal + 40));
    double* er = ctx->e_atom + np;
@@ -1860,7 +1886,7 @@ int launch_force_recip_uind(Context* ctx, float* wrec, bool alt)
    const bool vir = wrec != nullptr;
    P.packed = true;
    k_spread<1><<<nb, 256, 0, ctx->stream>>>(ctx->n, G, sites(ctx), ctx->uind,
-      nullptr, nullptr, reinterpret_cast<unsigned long long*>(P.qfx));
+      nullptr, nullptr, reinterpret_cast<unsigned long long*>(P.qfx), nullptr);
    int rc = cudaGetLastError() == cudaSuccess ? T9GB_OK : T9GB_CUDA_ERR;
    if (rc == T9GB_OK)
       rc = fft_conv(ctx, vir ? 2 : 0, 0.f, 0.5f * f, false, ctx->scal + 46);

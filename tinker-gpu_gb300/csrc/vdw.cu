@@ -80,15 +80,13 @@ struct HalAcc {
    float e, g[3], w[9];
 };
 
+// one pair at separation d (within the cutoff) of types ta, tb, scale vs
 template <bool VIR>
-__device__ __forceinline__ void hal_add(const PairParams& P, float4 a, float4 b, float vs, const float2* vtab, int nvt,
-   float cut, float off2, float off, HalAcc& o)
+__device__ __forceinline__ void hal_accumulate(float3 d, int ta, int tb, float vs, const float2* vtab, int nvt,
+   float cut, float off, HalAcc& o)
 {
-   const float3 d = sep(P, a, b);
    const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-   if (r2 > off2 || vs == 0.f)
-      return;
-   const float2 t = vtab[__float_as_int(a.w) * nvt + __float_as_int(b.w)];
+   const float2 t = vtab[ta * nvt + tb];
    const float r = sqrtf(r2);
    float e, de;
    hal_pair(r, t.x, t.y * vs, cut, off, e, de);
@@ -107,6 +105,20 @@ __device__ __forceinline__ void hal_add(const PairParams& P, float4 a, float4 b,
    }
 }
 
+template <bool VIR>
+__device__ __forceinline__ void hal_add(const PairParams& P, float4 a, float4 b, float vs, const float2* vtab, int nvt,
+   float cut, float off2, float off, HalAcc& o)
+{
+   const float3 d = sep(P, a, b);
+   const float r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+   if (r2 > off2 || vs == 0.f)
+      return;
+   hal_accumulate<VIR>(d, __float_as_int(a.w), __float_as_int(b.w), vs, vtab, nvt, cut, off, o);
+}
+
+constexpr int HAL_CHUNK = 4;  // candidates a lane loads at once
+constexpr int HAL_QUEUE = 8;  // queued pairs of a lane
+
 // G lanes per site: e_atom[s] (FP64), fout[s] = dE/dx of site s, virial rows
 // wout[c][s] (may be null)
 template <int G, bool VIR>
@@ -115,6 +127,7 @@ __global__ void __launch_bounds__(256) k_ehal(PairParams P, int npad, float cut,
    const float* __restrict__ sp_v, const float4* __restrict__ vpos, const float2* __restrict__ vtab, int nvt,
    double* __restrict__ e_atom, float* __restrict__ fout, float* __restrict__ wout)
 {
+   __shared__ float4 hq[HAL_QUEUE][256];
    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
    const int i = tid / G, g = tid % G;
    if (i >= npad)
@@ -128,12 +141,54 @@ __global__ void __launch_bounds__(256) k_ehal(PairParams P, int npad, float cut,
    for (int c = 0; c < 9; ++c)
       o.w[c] = 0.f;
    const float off2 = off * off;
+   const unsigned grp = __ballot_sync(0xffffffffu, i < P.n);
    if (i < P.n) {
       const float4 a = vpos[i];
       const int* row = nbr + (size_t)i * P.cap;
       const int cnt = nnbr[i];
-      for (int k = g; k < cnt; k += G)
-         hal_add<VIR>(P, a, vpos[row[k]], 1.f, vtab, nvt, cut, off2, off, o);
+      // Half of the stored pairs lie beyond the cutoff, so a warp would
+      // evaluate nearly every one with half of its lanes.  Each lane queues
+      // its pairs within the cutoff (in its order, so its sums are the same)
+      // and the warp evaluates when every lane still at work has one: 26 of 32
+      // lanes at work instead of 16, for about 35 instructions more a candidate.
+      // GB300, 648 / 12,288 / 98,304 atoms: 30 -> 21, 50 -> 47, 288 -> 265 us.
+      const int ta = __float_as_int(a.w);
+      int head = 0, len = 0;
+      int jn[HAL_CHUNK];
+      float4 b[HAL_CHUNK];
+#pragma unroll
+      for (int q = 0; q < HAL_CHUNK; ++q)
+         jn[q] = g + q * G < cnt ? row[g + q * G] : -1;
+      for (int k = g; __any_sync(grp, k < cnt); k += HAL_CHUNK * G) {
+         int j[HAL_CHUNK];
+#pragma unroll
+         for (int q = 0; q < HAL_CHUNK; ++q) {
+            j[q] = jn[q];
+            if (j[q] >= 0)
+               b[q] = vpos[j[q]];
+         }
+#pragma unroll
+         for (int q = 0; q < HAL_CHUNK; ++q)
+            jn[q] = k + (HAL_CHUNK + q) * G < cnt ? row[k + (HAL_CHUNK + q) * G] : -1;
+#pragma unroll
+         for (int q = 0; q < HAL_CHUNK; ++q)
+            if (j[q] >= 0) {
+               const float3 d = sep(P, a, b[q]);
+               if (d.x * d.x + d.y * d.y + d.z * d.z <= off2) {
+                  hq[(head + len) & (HAL_QUEUE - 1)][threadIdx.x] = make_float4(d.x, d.y, d.z, b[q].w);
+                  ++len;
+               }
+            }
+         // until a lane that has more to come runs dry, or while one is full
+         while (__all_sync(grp, len > 0 || k + HAL_CHUNK * G >= cnt) ? __any_sync(grp, len > 0)
+                                                                     : __any_sync(grp, len > HAL_QUEUE - HAL_CHUNK))
+            if (len > 0) {
+               const float4 v = hq[head & (HAL_QUEUE - 1)][threadIdx.x];
+               ++head;
+               --len;
+               hal_accumulate<VIR>(make_float3(v.x, v.y, v.z), ta, __float_as_int(v.w), 1.f, vtab, nvt, cut, off, o);
+            }
+      }
       const int pa = sp_start[i], pb = sp_start[i + 1];
       for (int q = pa + g; q < pb; q += G)
          hal_add<VIR>(P, a, vpos[sp_j[q]], sp_v[q], vtab, nvt, cut, off2, off, o);
