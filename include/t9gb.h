@@ -414,17 +414,19 @@ int t9gb_nblist_stats(t9gb_context* ctx, int* capacity, long long* entries, int*
  * hosts that own every device allocation, code running inside a CUDA-graph
  * stream capture, real-time loops that forbid allocator calls after
  * start-up.  Inputs and outputs are the caller's device arrays (xyz, uind,
- * uinp, field, fieldp [n][3]; pdamp, thole [n]); the working memory is a
- * static device array inside the library sized for
- * T9GB_NOALLOC_MAX_ATOMS atoms (384 KiB, held by every GPU that loads the
- * library until the process exits).  It computes the damped (non-Ewald)
- * field -T u of pairs within `cutoff` (minimum image when box != NULL has
- * three positive edges), all mutual scales 1, like t9gb_ufield on a context
- * with use_ewald = 0.  n > T9GB_NOALLOC_MAX_ATOMS returns T9GB_TOO_LARGE.
- * The first call on each device looks up the array's address
+ * uinp, field, fieldp [n][3]; pdamp, thole [n]).  It computes the damped
+ * (non-Ewald) field -T u of pairs within `cutoff` (minimum image when
+ * box != NULL has three positive edges), all mutual scales 1, like
+ * t9gb_ufield on a context with use_ewald = 0.  All pairs are tested, so
+ * n > T9GB_NOALLOC_MAX_ATOMS returns T9GB_TOO_LARGE.
+ *
+ * Outputs may overlap inputs.  Only then a call has working memory: a static
+ * device array inside the library (352 KiB, held by every GPU that loads the
+ * library until the process exits) that takes a copy of the inputs.  The
+ * first such call on each device looks up the array's address
  * (cudaGetSymbolAddress) and should therefore happen before any stream
- * capture.  Every call reuses the same array: calls that can overlap on the
- * GPU (different streams, no ordering between them) race. */
+ * capture, and such calls must not overlap on the GPU (different streams, no
+ * ordering between them): they share the array. */
 #define T9GB_NOALLOC_MAX_ATOMS 8192
 int t9gb_ufield_noalloc(int n, const double* box, double cutoff, const float* xyz_device, const float* pdamp_device,
    const float* thole_device, const float* uind_device, const float* uinp_device, float* field_device,
