@@ -119,6 +119,8 @@ struct PmeGrid {
    bool probe = false;        // spreads of the learned guess's residual: their own range flag
    int fft_cl = 0;            // fused transform: CTAs per z plane (a thread-block cluster), 0: one CTA
    int* fft_err = nullptr;    // device flag: a staged slab copy of a plane pass did not complete in time
+   bool small_fft = false;    // small cubic grid: transform and convolution as one cluster's work
+   float2* small_tw = nullptr;  // its twiddles, e^{-2 pi i k / n1}
 };
 
 // Per-kernel event timing (tracing): categories of timed launches.

@@ -1045,6 +1045,326 @@ static void fft_own_inverse(const PmeGrid& P, cudaStream_t st, bool split, bool 
 }
 
 // ---------------------------------------------------------------------------
+// Small cubic grids: the conversion from fixed point, the 3-D FFT, the
+// convolution and the inverse FFT as one kernel, on one cluster of SG_CL CTAs
+// that keeps the grid in its shared memory.  CTA r has planes
+// [r N / SG_CL, ...) for the x and y passes; for the z passes it has columns
+// [r N^2 / SG_CL, ...), which it reads from its peers' planes and writes back
+// through distributed shared memory.  An edge is RA x RB, each 2 to 8, and a
+// pass two Stockham steps between two buffers: for the factor R after the
+// product S of the factors before it, butterfly j takes the elements
+// j + q N / R and writes (j / S) S R + j % S + q S.  The inverse transform is
+// the forward one with real and imaginary parts exchanged before and after.
+//
+// What bounds it: a chain of twelve steps with a barrier each (about 250
+// cycles at 24^3, where a step moves 14 KB through a CTA's shared memory in
+// 110 of them; at 40^3 it moves 64 KB and the shared memory bounds it), two
+// cluster barriers and one trip to global memory each way.  It takes the
+// place of eight launches of a few microseconds (cuFFT's six, conversion,
+// convolution): an induce solve of 648 atoms on 16 / 20 / 24 / 30 / 36 / 40
+// points an edge takes 288 / 283 / 287 / 302 / 331 / 345 us instead of
+// 382 / 401 / 396 / 405 / 395 / 405, and on 32 points 302 instead of the 316
+// of the plane kernels.  With 8 CTAs it is 294 / 332 / 383 us at 24 / 30 /
+// 40; 256 threads take 289 / 317 / 378.  Edges are known at compile time:
+// the same steps with factors and strides from a table took 17.7 us a
+// transform at 24^3 instead of 7.3.
+constexpr int SG_CL = 16;       // CTAs, the largest cluster
+constexpr int SG_THREADS = 512;
+
+template <int R>
+__device__ __forceinline__ void dft_small(float2* v)
+{
+   if constexpr (R == 2) {
+      const float2 a = v[0], b = v[1];
+      v[0] = make_float2(a.x + b.x, a.y + b.y);
+      v[1] = make_float2(a.x - b.x, a.y - b.y);
+   } else if constexpr (R == 3) {
+      const float s3 = 0.866025403784438647f;
+      const float2 t = make_float2(v[1].x + v[2].x, v[1].y + v[2].y);
+      const float2 d = make_float2(s3 * (v[1].x - v[2].x), s3 * (v[1].y - v[2].y));
+      const float2 m = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
+      v[0] = make_float2(v[0].x + t.x, v[0].y + t.y);
+      v[1] = make_float2(m.x + d.y, m.y - d.x);
+      v[2] = make_float2(m.x - d.y, m.y + d.x);
+   } else if constexpr (R == 4) {
+      const float2 a = make_float2(v[0].x + v[2].x, v[0].y + v[2].y), b = make_float2(v[0].x - v[2].x, v[0].y - v[2].y);
+      const float2 c = make_float2(v[1].x + v[3].x, v[1].y + v[3].y), d = make_float2(v[1].x - v[3].x, v[1].y - v[3].y);
+      v[0] = make_float2(a.x + c.x, a.y + c.y);
+      v[1] = make_float2(b.x + d.y, b.y - d.x);
+      v[2] = make_float2(a.x - c.x, a.y - c.y);
+      v[3] = make_float2(b.x - d.y, b.y + d.x);
+   } else if constexpr (R == 5) {
+      // cos and sin of 2 pi / 5 and 4 pi / 5
+      const float c1 = 0.309016994374947424f, c2 = -0.809016994374947424f;
+      const float s1 = 0.951056516295153572f, s2 = 0.587785252292473129f;
+      const float2 a = make_float2(v[1].x + v[4].x, v[1].y + v[4].y), b = make_float2(v[1].x - v[4].x, v[1].y - v[4].y);
+      const float2 c = make_float2(v[2].x + v[3].x, v[2].y + v[3].y), d = make_float2(v[2].x - v[3].x, v[2].y - v[3].y);
+      const float2 p = make_float2(v[0].x + c1 * a.x + c2 * c.x, v[0].y + c1 * a.y + c2 * c.y);
+      const float2 q = make_float2(v[0].x + c2 * a.x + c1 * c.x, v[0].y + c2 * a.y + c1 * c.y);
+      const float2 e = make_float2(s1 * b.x + s2 * d.x, s1 * b.y + s2 * d.y);
+      const float2 f = make_float2(s2 * b.x - s1 * d.x, s2 * b.y - s1 * d.y);
+      v[0] = make_float2(v[0].x + a.x + c.x, v[0].y + a.y + c.y);
+      v[1] = make_float2(p.x + e.y, p.y - e.x);
+      v[4] = make_float2(p.x - e.y, p.y + e.x);
+      v[2] = make_float2(q.x + f.y, q.y - f.x);
+      v[3] = make_float2(q.x - f.y, q.y + f.x);
+   } else {
+      // R = 6, 8: the halves of even and odd index
+      constexpr int H = R / 2;
+      float2 e[H], o[H];
+#pragma unroll
+      for (int k = 0; k < H; ++k) {
+         e[k] = v[2 * k];
+         o[k] = v[2 * k + 1];
+      }
+      dft_small<H>(e);
+      dft_small<H>(o);
+#pragma unroll
+      for (int k = 0; k < H; ++k) {
+         constexpr float h = 0.5f, s3 = 0.866025403784438647f, r2 = 0.707106781186547524f;
+         const float2 w = H == 3 ? (k == 0 ? make_float2(1.f, 0.f) : (k == 1 ? make_float2(h, -s3) : make_float2(-h, -s3)))
+                                 : (k == 0 ? make_float2(1.f, 0.f)
+                                           : (k == 1 ? make_float2(r2, -r2)
+                                                     : (k == 2 ? make_float2(0.f, -1.f) : make_float2(-r2, -r2))));
+         const float2 t = k == 0 ? o[0] : (H == 4 && k == 2 ? make_float2(o[2].y, -o[2].x) : cmulf(w, o[k]));
+         v[k] = make_float2(e[k].x + t.x, e[k].y + t.y);
+         v[k + H] = make_float2(e[k].x - t.x, e[k].y - t.y);
+      }
+   }
+}
+
+template <int N>
+struct SmallGrid {
+   static constexpr int P = N | 1;  // row pitch: odd, so that threads on consecutive rows meet different banks
+   static constexpr int NZ = (N + SG_CL - 1) / SG_CL;       // the most planes of a CTA
+   static constexpr int NC = (N * N + SG_CL - 1) / SG_CL;   // the most columns
+   static constexpr int BUF = NZ * N * P > NC * N ? NZ * N * P : NC * N;
+   static constexpr size_t SMEM = sizeof(float2) * (2 * BUF + NC * N + N);
+   __device__ __forceinline__ static int z_owner(int z) { return ((z + 1) * SG_CL - 1) / N; }
+   __device__ __forceinline__ static int z_first(int r) { return r * N / SG_CL; }
+};
+
+// one Stockham step of the first `lines` of at most LM lines; load(l, i) and
+// store(l, i, k, v) take element i of line l (k: the thread's count of stores)
+template <int N, int R, int S, int LM, class Load, class Store>
+__device__ __forceinline__ void sg_step(int lines, const float2* tw, Load load, Store store)
+{
+   constexpr int NJ = N / R, TASKS = (LM * NJ + SG_THREADS - 1) / SG_THREADS;
+#pragma unroll
+   for (int it = 0; it < TASKS; ++it) {
+      const int t = threadIdx.x + it * SG_THREADS, j = t / LM, l = t % LM;
+      if (j >= NJ || l >= lines)
+         continue;
+      const int jl = j % S, to = j / S * S * R + jl;
+      float2 v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+         v[q] = load(l, j + q * NJ);
+      if (S > 1)
+#pragma unroll
+         for (int q = 1; q < R; ++q)
+            v[q] = cmulf(v[q], tw[q * jl * (N / (S * R))]);
+      dft_small<R>(v);
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+         store(l, to + q * S, it * R + q, v[q]);
+   }
+}
+
+template <int N, int RA, int RB>
+__global__ void __launch_bounds__(SG_THREADS) k_fft_small(long long* __restrict__ qfx, float2* __restrict__ g,
+   const float* __restrict__ infl, const float2* __restrict__ twg, int packed, float inv, int* __restrict__ range)
+{
+   using G = SmallGrid<N>;
+   constexpr int P = G::P, NC = G::NC, LX = G::NZ * N;
+   constexpr int PER = (G::NZ * N * N + SG_THREADS - 1) / SG_THREADS;       // grid points a thread
+   constexpr int CT = (NC * RA + SG_THREADS - 1) / SG_THREADS;              // z tasks of the second step
+   extern __shared__ __align__(16) float2 sgm[];
+   float2* const b0 = sgm;  // planes, read and written by the peers
+   float2* const b1 = b0 + G::BUF;
+   float2* const b2 = b1 + G::BUF;
+   float2* const tw = b2 + NC * N;
+   unsigned rank;
+   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+   const int z0 = G::z_first((int)rank), nz = G::z_first((int)rank + 1) - z0;
+   const int c0 = (int)rank * N * N / SG_CL, nc = ((int)rank + 1) * N * N / SG_CL - c0;
+   const int tid = threadIdx.x;
+   if (tid < N)
+      tw[tid] = twg[tid];
+   // the influence function where this thread's second z step will need it
+   float fn[CT * RB];
+#pragma unroll
+   for (int it = 0; it < CT; ++it) {
+      const int t = tid + it * SG_THREADS, j = t / NC, l = t % NC;
+#pragma unroll
+      for (int q = 0; q < RB; ++q)
+         fn[it * RB + q] = j < RA && l < nc ? infl[(size_t)(j + q * RA) * N * N + c0 + l] : 0.f;
+   }
+   pdl_wait();
+   pdl_trigger();
+   bool big = false;
+   {
+      long long* q = qfx + (size_t)z0 * N * N;
+      long long w[PER];
+#pragma unroll
+      for (int k = 0; k < PER; ++k)
+         w[k] = tid + k * SG_THREADS < nz * N * N ? q[tid + k * SG_THREADS] : 0;
+#pragma unroll
+      for (int k = 0; k < PER; ++k) {
+         const int e = tid + k * SG_THREADS;
+         if (e >= nz * N * N)
+            continue;
+         q[e] = 0;
+         big |= grid_word_big(w[k], packed);
+         b0[e / N * P + e % N] = grid_word(w[k], packed, inv);
+      }
+   }
+   if (big)
+      atomicOr(range, 1);
+   __syncthreads();
+   // plane passes from b0 over b1 back to b0; element i of row l, of column
+   // (plane l / N, x l % N)
+   auto px = [](int l, int i) { return l * P + i; };
+   auto py = [](int l, int i) { return l / N * (N * P) + i * P + l % N; };
+   auto plane = [&](auto at) {
+      sg_step<N, RA, 1, LX>(nz * N, tw, [&](int l, int i) { return b0[at(l, i)]; },
+         [&](int l, int i, int, float2 v) { b1[at(l, i)] = v; });
+      __syncthreads();
+      sg_step<N, RB, RA, LX>(nz * N, tw, [&](int l, int i) { return b1[at(l, i)]; },
+         [&](int l, int i, int, float2 v) { b0[at(l, i)] = v; });
+   };
+   plane(px);
+   __syncthreads();
+   plane(py);
+   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+   // point (z, column c0 + l) in its owner's b0
+   const unsigned b0_s = (unsigned)__cvta_generic_to_shared(b0);
+   auto peer = [&](int l, int z) {
+      const int own = G::z_owner(z), c = c0 + l;
+      const unsigned at = b0_s + 8u * (unsigned)(((z - G::z_first(own)) * N + c / N) * P + c % N);
+      unsigned r;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(at), "r"((unsigned)own));
+      return r;
+   };
+   sg_step<N, RA, 1, NC>(nc, tw,
+      [&](int l, int z) {
+         float2 v;
+         // volatile keeps the loads after the barrier; no memory clobber, so they pipeline
+         asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(peer(l, z)));
+         return v;
+      },
+      [&](int l, int z, int, float2 v) { b1[z * NC + l] = v; });
+   __syncthreads();
+   // the convolution, and the exchange of real and imaginary parts
+   sg_step<N, RB, RA, NC>(nc, tw, [&](int l, int z) { return b1[z * NC + l]; },
+      [&](int l, int z, int k, float2 v) { b2[z * NC + l] = make_float2(v.y * fn[k], v.x * fn[k]); });
+   __syncthreads();
+   sg_step<N, RA, 1, NC>(nc, tw, [&](int l, int z) { return b2[z * NC + l]; },
+      [&](int l, int z, int, float2 v) { b1[z * NC + l] = v; });
+   __syncthreads();
+   // a column belongs to one CTA: no peer still reads what is written here
+   sg_step<N, RB, RA, NC>(nc, tw, [&](int l, int z) { return b1[z * NC + l]; },
+      [&](int l, int z, int, float2 v) {
+         asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(peer(l, z)), "f"(v.x), "f"(v.y) : "memory");
+      });
+   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+   plane(py);
+   __syncthreads();
+   plane(px);
+   __syncthreads();
+#pragma unroll
+   for (int k = 0; k < PER; ++k) {
+      const int e = tid + k * SG_THREADS;
+      if (e < nz * N * N) {
+         const float2 v = b0[e / N * P + e % N];
+         g[(size_t)z0 * N * N + e] = make_float2(v.y, v.x);
+      }
+   }
+}
+
+using SmallFft = void (*)(long long*, float2*, const float*, const float2*, int, float, int*);
+
+// The kernel of an edge and its shared memory; null: not a small grid.  Even
+// products of two factors, from 16 (the least edge of a box with a 7 A
+// cutoff) to 40: at 48 the gain is down to 8 % (384 for 419 us) and the
+// trajectories' sensitivity to rounding, which grows with the box, moves the
+// velocities of a restart by 1.6e-5 between the two transforms (1.2e-5 at
+// 40), so larger boxes keep the transform they had.
+static SmallFft small_fft_kernel(int n, size_t* smem)
+{
+   switch (n) {
+   case 16: *smem = SmallGrid<16>::SMEM; return k_fft_small<16, 4, 4>;
+   case 18: *smem = SmallGrid<18>::SMEM; return k_fft_small<18, 3, 6>;
+   case 20: *smem = SmallGrid<20>::SMEM; return k_fft_small<20, 4, 5>;
+   case 24: *smem = SmallGrid<24>::SMEM; return k_fft_small<24, 4, 6>;
+   case 30: *smem = SmallGrid<30>::SMEM; return k_fft_small<30, 5, 6>;
+   case 32: *smem = SmallGrid<32>::SMEM; return k_fft_small<32, 4, 8>;
+   case 36: *smem = SmallGrid<36>::SMEM; return k_fft_small<36, 6, 6>;
+   case 40: *smem = SmallGrid<40>::SMEM; return k_fft_small<40, 5, 8>;
+   }
+   return nullptr;
+}
+
+// the launch as one cluster; at: room for its attributes
+static cudaLaunchConfig_t small_fft_config(size_t smem, cudaLaunchAttribute* at)
+{
+   cudaLaunchConfig_t cfg = {};
+   cfg.gridDim = dim3(SG_CL);
+   cfg.blockDim = dim3(SG_THREADS);
+   cfg.dynamicSmemBytes = smem;
+   at[0].id = cudaLaunchAttributeClusterDimension;
+   at[0].val.clusterDim.x = SG_CL;
+   at[0].val.clusterDim.y = 1;
+   at[0].val.clusterDim.z = 1;
+   cfg.attrs = at;
+   cfg.numAttrs = 1;
+   return cfg;
+}
+
+static int launch_small_fft(Context* ctx, int* range)
+{
+   PmeGrid& P = ctx->pme;
+   size_t smem = 0;
+   const SmallFft k = small_fft_kernel(P.n1, &smem);
+   cudaLaunchAttribute at[2];
+   cudaLaunchConfig_t cfg = small_fft_config(smem, at);
+   cfg.stream = ctx->stream;
+   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+   at[1].val.programmaticStreamSerializationAllowed = 1;
+   cfg.numAttrs = use_pdl(ctx) ? 2 : 1;
+   T9_CUDA(cudaLaunchKernelEx(&cfg, k, P.qfx, P.qgrid, (const float*)P.infl, (const float2*)P.small_tw,
+      P.packed ? 1 : 0, 1.0f / (float)(1 << P.pack_shift), range));
+   return T9GB_OK;
+}
+
+static int small_fft_setup(Context* ctx)
+{
+   PmeGrid& P = ctx->pme;
+   size_t smem = 0;
+   const SmallFft k = P.n1 == P.n2 && P.n2 == P.n3 ? small_fft_kernel(P.n1, &smem) : nullptr;
+   if (!k)
+      return T9GB_OK;
+   std::vector<float2> tw(P.n1);
+   for (int i = 0; i < P.n1; ++i) {
+      const double x = 2 * 3.14159265358979323846 * i / P.n1;
+      tw[i] = make_float2((float)std::cos(x), (float)-std::sin(x));
+   }
+   T9_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+   T9_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+   cudaLaunchAttribute at;
+   cudaLaunchConfig_t cfg = small_fft_config(smem, &at);
+   int fit = 0;
+   if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess || fit < 1) {
+      cudaGetLastError();  // a device whose free SMs hold no such cluster keeps cuFFT or the planes
+      return T9GB_OK;
+   }
+   T9_CUDA(cudaMalloc(&P.small_tw, sizeof(float2) * tw.size()));
+   T9_CUDA(cudaMemcpy(P.small_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
+   P.small_fft = true;
+   return T9GB_OK;
+}
+
+// ---------------------------------------------------------------------------
 // k-space part of the reciprocal virial (the strain derivative of the
 // influence function), read-only on the forward-transformed grid:
 //   W_ab += sum_m w(m) G(m) [-delta_ab + 2 h_a h_b (1 + pi^2 h^2 / a^2) / h^2]
@@ -1525,6 +1845,7 @@ int pme_setup(Context* ctx)
    // default where it measured faster than cuFFT on GB300 (64^3: 0.627 vs
    // 0.634 ms per induce step in the graph); at 128^3 cuFFT is faster
    P.own_fft = P.own_fft_ok && P.n1 <= 64;
+   T9_CHECK(small_fft_setup(ctx));
    if (P.own_fft_ok) {
       if (P.n1 == 32)
          T9_CHECK(fft_setup_kernels<32>(ctx));
@@ -1558,6 +1879,7 @@ void pme_free(Context* ctx)
    cudaFree(P.spl_hi);
    cudaFree(P.qstash);
    cudaFree(P.fft_err);
+   cudaFree(P.small_tw);
    P = PmeGrid();
 }
 
@@ -1612,6 +1934,11 @@ static int fft_conv(Context* ctx, int vir = 0, float wE = 0.f, float wP = 0.f, b
    const int cb = (int)std::min<size_t>((ng + 255) / 256, 152 * 16);
    prof_begin(ctx, P_FFT_CONV);
    int* range = ctx->status + (P.probe ? ST_RANGE_L : ST_RANGE);
+   if (P.small_fft && !vir) {
+      T9_CHECK(launch_small_fft(ctx, range));
+      prof_end(ctx);
+      return T9GB_OK;
+   }
    if (P.own_fft) {
       cudaStream_t st = ctx->stream;
       const bool split = vir != 0;
