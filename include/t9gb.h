@@ -360,14 +360,14 @@ int t9gb_pair_staging(t9gb_context* ctx, int enable);
 int t9gb_copy_error(t9gb_context* ctx, int* flag);
 
 /* Lanes of a warp that share one atom's neighbour row in the real-space
- * field and preconditioner kernels: 4, 8, 16 or 32 (default 8 up to 32,768
- * atoms, 4 above).  A tuning knob; results are identical up to the order of
+ * field and preconditioner kernels: 4, 8, 16 or 32 (default 16 up to 768
+ * atoms, 8 up to 32,768, 4 above).  A tuning knob; results are identical up to the order of
  * the per-lane partial sums. */
 int t9gb_pair_lanes(t9gb_context* ctx, int lanes);
 
 /* Lanes of a warp that share one atom's neighbour row in the real-space
- * force kernel (empole / epolar / emplar gradients): 4 (default), 8 or
- * 16.  A tuning knob; results are identical up to the order of the
+ * force kernel (empole / epolar / emplar gradients): 4, 8 or 16 (default 16
+ * up to 2,304 atoms, 8 up to 3,072, 4 above).  A tuning knob; results are identical up to the order of the
  * per-lane partial sums.  Measured on GB300 (emplar gradient, 12,288 /
  * 98,304 atoms, ms): 1 lane 0.817 / 4.031, 2 0.781 / 4.051, 4 0.758 /
  * 4.071, 8 0.768 / 4.148, 16 0.797 / 4.355 (1 and 2 are not built). */

@@ -216,8 +216,16 @@ int t9gb_create(const t9gb_config* cfg, t9gb_context** out)
    ctx->npad = ((cfg->n + WARP - 1) / WARP) * WARP;
    // lanes per atom of the field kernels: 8 on small boxes, 4 where the box
    // fills the GPU (GB300 induce: 12,288 atoms 0.573 / 0.631 ms at 8 / 4
-   // lanes; 98,304 atoms 2.588 / 2.514 ms)
-   ctx->pair_lanes = ctx->npad > 32768 ? 4 : 8;
+   // lanes; 98,304 atoms 2.588 / 2.514 ms), 16 where even their eight lanes
+   // leave most of it idle (648 atoms 0.320 / 0.301 ms at 8 / 16 lanes, 1,029
+   // atoms 0.332 / 0.343)
+   ctx->pair_lanes = ctx->npad > 32768 ? 4 : (ctx->npad > 768 ? 8 : 16);
+   // and of the real-space force kernel, whose rows are a serial chain of
+   // long pair terms on a small box (10 MD steps at 4 / 8 / 16 lanes: 648
+   // atoms 3.44 / 3.12 / 3.04 ms, 1,200 3.17 / 3.06 / 3.01, 2,187 4.12 / 4.00
+   // / 3.78, 2,550 4.24 / 3.89 / 4.00, 3,000 4.49 / 4.28 / 4.41, 3,993 4.86 /
+   // 4.81 / 4.83)
+   ctx->force_lanes = ctx->npad > 3072 ? 4 : (ctx->npad > 2304 ? 8 : 16);
    cudaGetDevice(&ctx->dev);
    int rc = T9GB_OK;
    if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess)

@@ -1,6 +1,6 @@
 // Real-space pair kernels over the per-step neighbour list.
 //
-// G consecutive lanes own one atom i (t9gb_pair_lanes: 8 up to 32,768 atoms,
+// G consecutive lanes own one atom i (t9gb_pair_lanes: 16 up to 768 atoms, 8 up to 32,768,
 // 4 above): lane g walks the list entries g, g+G, g+2G, ... of atom i
 // (consecutive addresses per step, two entries in flight per trip), then the
 // scaled partners of i the same way; the partial fields are combined with a
