@@ -1019,8 +1019,9 @@ int launch_list_filter(Context* ctx)
 // Where the grid leaves an SM at most one block, a row's trips wait on their
 // own latency, not on the L1's line rate: four entries a trip (80-106
 // registers).  GB300, induce: droplet of 1,500 atoms (rows of 1,499) 749 ->
-// 660 us; periodic boxes of 648 and 3,000 atoms the same either way; at
-// 12,288 atoms two entries are better (414 against 436 us).
+// 660 us; periodic boxes of 648 and 3,000 atoms the same either way (10 MD
+// steps of 648 atoms at 16 lanes 3.10 -> 3.05 ms); at 12,288 atoms two entries
+// are better (414 against 436 us).
 static bool few_blocks(int nb) { return nb <= 152; }
 
 static TensorList field_list(const Context* ctx) { return {ctx->nbrc, ctx->nnbrc, ctx->cfu, ctx->spu}; }
@@ -1096,6 +1097,8 @@ int launch_ufield_real(Context* ctx, const float* u6, const float* base6, float*
                                                                                     : k_ufield_real<16, false>;
    if (g == 8 && few_blocks(nb))
       k = k_ufield_real<8, false, 4>;
+   else if (g == 16 && few_blocks(nb))
+      k = k_ufield_real<16, false, 4>;
    T9_CUDA(launch_k(use_pdl(ctx), k, nb, PAIR_THREADS, 0, ctx->stream, P, ctx->npad, field_list(ctx),
       partners(ctx), ctx->spos, u6, nullptr, nullptr, base6, out6));
    prof_end(ctx);
@@ -1146,6 +1149,8 @@ int launch_precond_sparse_dots(Context* ctx, const float* r6, float* z6, const P
          ? k_precond_sparse_dots<32> : k_precond_sparse_dots<16>;
    if (g == 8 && few_blocks(nb))
       k = k_precond_sparse_dots<8, 4>;
+   else if (g == 16 && few_blocks(nb))
+      k = k_precond_sparse_dots<16, 4>;
    T9_CUDA(launch_k(use_pdl(ctx), k, nb, PAIR_THREADS, 0, ctx->stream, P, ctx->npad, (float)ctx->cfg.udiag, precond_list(ctx),
       partners(ctx), ctx->spos, r6, z6, D));
    prof_end(ctx);
