@@ -17,7 +17,7 @@ def test_default_lanes(gpu_lib, tg, nside, sites):
     a, b = engine_for(s), engine_for(s)
     b.pair_lanes(8)
     b.force_lanes(4)
-    ga, gb = a.emplar(gpu_lib.CALC_GRAD)[1], b.emplar(gpu_lib.CALC_GRAD)[1]
+    ga, gb = (e.emplar(gpu_lib.CALC_ENERGY | gpu_lib.CALC_GRAD)[1] for e in (a, b))
     assert rel_err(cpu(ga), cpu(gb)) < RTOL
     assert a.stats()[0] == b.stats()[0]
     for x, y in zip(a.induce()[:2] + a.dfield(), b.induce()[:2] + b.dfield()):

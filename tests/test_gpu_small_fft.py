@@ -26,6 +26,6 @@ def test_small_grid_fields(gpu_lib, oracle, tg, n):
             assert rel_err(cpu(x), r) < FIELD_RTOL
     # the dipole grid beside the permanent one
     abi = gpu_lib
-    ga, gb = a.emplar(abi.CALC_GRAD)[1], b.emplar(abi.CALC_GRAD)[1]
+    ga, gb = a.emplar(abi.CALC_ENERGY | abi.CALC_GRAD)[1], b.emplar(abi.CALC_ENERGY | abi.CALC_GRAD)[1]
     assert rel_err(cpu(ga), cpu(gb)) < 1e-5
     assert a.stats()[0] == b.stats()[0]
