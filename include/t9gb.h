@@ -344,11 +344,12 @@ int t9gb_pme_fft_cluster(t9gb_context* ctx, int ctas);
  * needs into shared memory with bulk asynchronous copies and reads every
  * neighbour from there; enable = 0 (the default) reads each neighbour row
  * from global memory through L1.  Bit-identical fields either way (the same
- * pairs in the same order); used with 4 or 8 lanes per atom.  A tuning knob:
- * measured on GB300 the staged kernels are slower (mutual field 22.6 vs
- * 20.7 us at 12,288 atoms, 161 vs 101 us at 98,304), because a block stages
- * about 39 neighbouring blocks of 1.5 KB, three times the rows it reads,
- * while the global kernels hit L1 on 85% of their row sectors. */
+ * pairs in the same order); used with 4 or 8 lanes per atom (so up to 768
+ * atoms only after t9gb_pair_lanes).  A tuning knob: measured on GB300 the
+ * staged kernels are slower (induce 0.439 vs 0.402 ms at 12,288 atoms, 2.45
+ * vs 1.72 ms at 98,304), because a block stages about 39 neighbouring blocks
+ * of 1.5 KB, three times the rows it reads, while the global kernels hit L1
+ * on 85% of their row sectors. */
 int t9gb_pair_staging(t9gb_context* ctx, int enable);
 
 /* Device flags of the library's asynchronous copies, read after a
@@ -392,11 +393,12 @@ int t9gb_force_lanes(t9gb_context* ctx, int lanes);
  * 0.527 -> 0.514 ms at 12,288 atoms, 2.313 -> 2.293 ms at 98,304.  Bit 5
  * (PME, without bit 1): the search direction's gather runs right after the
  * transform on the reciprocal stream, as a programmatic dependent of its
- * last pass (the spread and the gather form their B-splines, which need
- * the positions only, before they wait), and stores recip + self apart; the
+ * last pass, and stores recip + self apart; the
  * Ap kernel adds it to the real-space field, the sum the gather would form.
  * Bit 6 (with bit 5): that chain stays on the main stream behind the
- * direction kernel and the real-space field runs on the side stream.  Bits
+ * direction kernel and the real-space field runs on the side stream; up to
+ * 4,096 atoms the spread then forms and stores the direction and the kernel
+ * falls away (648 atoms 0.420 -> 0.412 ms a solve, 6,300 0.342 -> 0.350).  Bits
  * 5-6 give the same bits as without them; GB300 (induce ms, 12,288 /
  * 98,304 atoms): mask 25 0.4925 / 2.344, 57 0.4829 / 2.297, 121 (the
  * default) 0.473 / 2.285.  A tuning knob: the same iteration, results equal
