@@ -743,11 +743,11 @@ def main():
     per_launch_s = kernels[dom]["ms_per_launch"] / 1000.0
     achieved = alg / per_launch_s / 1e9
     mean_it = float(np.mean(iters))
-    # own kernels per step (fused FFT, default CG fusion; programmatic launches count as launches): positions 1, rotpole 2, list 5, permanent
-    # field 6 (real, spread, 3 transform, gather), guess 1, field of the guess 6, r0 1, M r0 with the
-    # dots 1, peek + predictor save 1, predictor index 1, output 1; per PCG iteration: direction 1,
-    # field 6, Ap 1, update 1, M r with the dots 1
-    launches_per_step = 26 + 10 * mean_it
+    # own kernels per step (fused FFT, default CG fusion; programmatic launches count as launches): positions
+    # and spline tables 1, rotpole 1, list check and filter 2, permanent field 6 (real, spread, 3 transform,
+    # gather), guess 1, field of the guess 6, r0 1, M r0 with the dots 1, peek + predictor save 1, status and
+    # predictor index 1, output 1; per PCG iteration: direction 1, field 6, Ap 1, update 1, M r with the dots 1
+    launches_per_step = 22 + 10 * mean_it
 
     # ---- forces: emplar (induce + multipole and polarization energy, gradient, virial) ----
     forces = None
