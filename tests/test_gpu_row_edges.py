@@ -64,6 +64,26 @@ def test_direction_in_the_spread(gpu_lib, tg, sites):
     assert a.stats()[0] == b.stats()[0]
 
 
+# one cluster takes both vector steps up to 3,072 slots (1,024 molecules); bit
+# 1 of the mask has its own pair of kernels at every size
+@pytest.mark.parametrize("sites", [216, 227, 1024, 1025])
+def test_vector_steps(gpu_lib, tg, sites):
+    s = _box(tg, sites)
+    a, b = engine_for(s), engine_for(s)
+    b.lib.t9gb_set_pcg_fusion(b.h, 3)
+    for x, y in zip(a.induce()[:2], b.induce()[:2]):
+        assert rel_err(cpu(x), cpu(y)) < 1e-5
+    assert a.stats()[0] == b.stats()[0]
+
+
+@pytest.mark.parametrize("nmol", [1, 11, 40])
+def test_vector_steps_of_a_cluster(gpu_lib, oracle, tg, nmol):
+    s = water_cluster(tg, nmol)
+    got, ref = engine_for(s).induce()[:2], oracle.OracleSystem(s).induce()[:2]
+    for x, y in zip(got, ref):  # two solves to 1e-6 D rms
+        assert np.abs(cpu(x) - y).max() * tg.units.DEBYE < 2e-5
+
+
 # rows of 16 lanes below and of 8 above 32,768 atoms; queues that never fill
 # (a few pairs) and that stay part full
 @pytest.mark.parametrize("sites, vacuum", [(216, False), (227, False), (10923, False), (216, True)])

@@ -265,6 +265,118 @@ __global__ void k_pcg_p2(VecArgs A, const double* __restrict__ scal, float* __re
    }
 }
 
+// Both steps in one kernel for small boxes: one cluster, whose CTAs exchange
+// their partial p.Ap through distributed shared memory, keeps Ap in registers
+// between them.  What bounds it is latency, one trip to memory and one
+// cluster barrier; k_pcg_p1 needs a round of atomics and a second read of the
+// partials by its last block, and k_pcg_p2 a launch.  GB300, a solve of 648 /
+// 1,500 / 2,187 / 3,000 atoms: 300 / 339 / 400 / 437 -> 277 / 321 / 384 / 424
+// us.  The line lies where a thread holds five elements; the sum's order is
+// another one, and larger boxes, whose trajectories are the more sensitive to
+// it, keep theirs.
+constexpr int STEP_CL = 8, STEP_THREADS = 512;
+constexpr int STEP_MAX = 3072;  // slots
+constexpr int STEP_PER = (6 * STEP_MAX + STEP_CL * STEP_THREADS - 1) / (STEP_CL * STEP_THREADS);
+
+__global__ void __launch_bounds__(STEP_THREADS) k_pcg_step(VecArgs A, const float* __restrict__ fld,
+   const float* __restrict__ fld2, const float* __restrict__ conj, float* __restrict__ uind, float* __restrict__ rsd,
+   double* __restrict__ scal)
+{
+   pdl_wait();
+   pdl_trigger();  // the preconditioner may stage its blocks
+   __shared__ float wsum[2][STEP_THREADS / 32];
+   __shared__ double part[2][STEP_CL];
+   __shared__ float step[2];
+   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+   float p[STEP_PER], v[STEP_PER], u[STEP_PER], r[STEP_PER];
+   float dd = 0.f, dp = 0.f;
+#pragma unroll
+   for (int k = 0; k < STEP_PER; ++k) {
+      const int e = blockIdx.x * STEP_THREADS + threadIdx.x + k * STEP_CL * STEP_THREADS;
+      p[k] = v[k] = u[k] = r[k] = 0.f;
+      if (e >= A.ne)
+         continue;
+      const int s = e / 6, x = e + 2 * s;  // row s, component e - 6 s of [npad][8]
+      p[k] = conj[x];
+      u[k] = uind[x];
+      r[k] = rsd[x];
+      const float f = fld2 ? fld[x] + fld2[x] : fld[x];
+      v[k] = A.polinv[s] * p[k] - f;
+      if (e - 6 * s < 3)
+         dd += p[k] * v[k];
+      else
+         dp += p[k] * v[k];
+   }
+#pragma unroll
+   for (int o = 16; o > 0; o >>= 1) {
+      dd += __shfl_xor_sync(0xffffffffu, dd, o);
+      dp += __shfl_xor_sync(0xffffffffu, dp, o);
+   }
+   if (lane == 0) {
+      wsum[0][w] = dd;
+      wsum[1][w] = dp;
+   }
+   __syncthreads();
+   if (w == 0) {  // half-warp h sums system h over the warps, in FP64
+      double b = (double)wsum[lane >> 4][lane & 15];
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1)
+         b += __shfl_xor_sync(0xffffffffu, b, o);
+      if ((lane & 15) < STEP_CL) {
+         const unsigned at = (unsigned)__cvta_generic_to_shared(&part[lane >> 4][blockIdx.x]);
+         unsigned to;
+         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"((unsigned)(lane & 15)));
+         asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(b) : "memory");
+      }
+   }
+   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+   if (w == 0) {
+      double b = part[lane >> 4][lane & (STEP_CL - 1)];
+#pragma unroll
+      for (int o = STEP_CL / 2; o > 0; o >>= 1)
+         b += __shfl_xor_sync(0xffffffffu, b, o);
+      if ((lane & 15) == 0) {  // the step lengths in FP32 (used as FP32)
+         const int sys = lane >> 4;
+         const float a = b == 0 ? 0.f : (float)scal[sys ? S_SUM_P : S_SUM_D] / (float)b;
+         step[sys] = a;
+         if (blockIdx.x == 0)
+            scal[sys ? S_A_P : S_A_D] = (double)a;
+      }
+   }
+   __syncthreads();
+   const float ad = step[0], ap = step[1];
+#pragma unroll
+   for (int k = 0; k < STEP_PER; ++k) {
+      const int e = blockIdx.x * STEP_THREADS + threadIdx.x + k * STEP_CL * STEP_THREADS;
+      if (e >= A.ne)
+         continue;
+      const int s = e / 6, x = e + 2 * s;
+      const float g = e - 6 * s < 3 ? ad : ap;
+      uind[x] = u[k] + g * p[k];
+      rsd[x] = A.polar[s] == 0.f ? 0.f : r[k] - g * v[k];
+   }
+}
+
+static int launch_pcg_step(Context* ctx, const VecArgs& A, const float* fld2)
+{
+   cudaLaunchConfig_t cfg = {};
+   cfg.gridDim = dim3(STEP_CL);
+   cfg.blockDim = dim3(STEP_THREADS);
+   cfg.stream = ctx->stream;
+   cudaLaunchAttribute at[2];
+   at[0].id = cudaLaunchAttributeClusterDimension;
+   at[0].val.clusterDim.x = STEP_CL;
+   at[0].val.clusterDim.y = 1;
+   at[0].val.clusterDim.z = 1;
+   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+   at[1].val.programmaticStreamSerializationAllowed = 1;
+   cfg.attrs = at;
+   cfg.numAttrs = use_pdl(ctx) ? 2 : 1;
+   T9_CUDA(cudaLaunchKernelEx(&cfg, k_pcg_step, A, (const float*)ctx->fld6, fld2, (const float*)ctx->conj, ctx->uind,
+      ctx->rsd, ctx->scal));
+   return T9GB_OK;
+}
+
 // p = z + b p in place (the paths that do not form p where it is read)
 __global__ void k_pcg_dir(VecArgs A, const double* __restrict__ scal, float* __restrict__ conj,
    const float* __restrict__ zrsd)
@@ -892,6 +1004,12 @@ static int pcg_body(Context* ctx, const VecArgs& A, cudaGraphConditionalHandle h
          rcp = ctx->rcp6;
       } else {
          T9_CHECK(ufield6(ctx, ctx->conj, ctx->fld6));
+      }
+      if (ctx->npad <= STEP_MAX) {
+         prof_begin(ctx, P_VECTOR);
+         T9_CHECK(launch_pcg_step(ctx, A, rcp));
+         prof_end(ctx);
+         return precond_dots(ctx, A, 0, handle, use_handle);
       }
       prof_begin(ctx, P_VECTOR);
       T9_CUDA(launch_k(pdl, k_pcg_p1<false>, A.nb, VB, 0, ctx->stream, A, ctx->fld6, rcp, ctx->conj, nullptr,
