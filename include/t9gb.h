@@ -322,7 +322,8 @@ int t9gb_use_graph(t9gb_context* ctx, int enable);
  * measured on GB300: on cubic grids of 16, 18, 20, 24, 30, 32, 36 or 40
  * points per edge one kernel on one thread-block cluster for everything from
  * the fixed-point grid to the potential (but where a virial reads the
- * transformed grid: there as below); on 64^3 the fused transform; cuFFT on
+ * transformed grid, and while the learned guess trains, whose weights follow the
+ * rounding of the dipoles: there as below, 32^3 with the fused transform); on 64^3 the fused transform; cuFFT on
  * every other grid, 128^3 included.  Replaces fftfront/fftback +
  * pmeConv (src/cudart/fft.cpp:65-95, src/cu/pme.cu:908-1031).  Enabling on
  * an unsupported grid returns T9GB_BAD_ARG. */
@@ -362,7 +363,7 @@ int t9gb_copy_error(t9gb_context* ctx, int* flag);
 
 /* Lanes of a warp that share one atom's neighbour row in the real-space
  * field and preconditioner kernels: 4, 8, 16 or 32 (default 16 up to 768
- * atoms, 8 up to 32,768, 4 above).  A tuning knob; results are identical up to the order of
+ * atoms, where no learned guess trains, 8 up to 32,768, 4 above).  A tuning knob; results are identical up to the order of
  * the per-lane partial sums. */
 int t9gb_pair_lanes(t9gb_context* ctx, int lanes);
 

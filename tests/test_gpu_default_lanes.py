@@ -22,3 +22,17 @@ def test_default_lanes(gpu_lib, tg, nside, sites):
     assert a.stats()[0] == b.stats()[0]
     for x, y in zip(a.induce()[:2] + a.dfield(), b.induce()[:2] + b.dfield()):
         assert rel_err(cpu(x), cpu(y)) < RTOL
+
+
+def test_learning_keeps_its_route(gpu_lib, tg):
+    """While the learned guess trains, a small box solves as with the larger boxes' kernels, bit for bit."""
+    s = tg.systems.make_config("water648")
+    a, b = engine_for(s), engine_for(s)
+    b.pair_lanes(8)
+    b.pme_own_fft(False)
+    for e in (a, b):
+        e.learn_config(3)
+    for _ in range(2):
+        for x, y in zip(a.induce()[:2], b.induce()[:2]):
+            assert (x == y).all()
+    assert (a.learn_weights() == b.learn_weights()).all()

@@ -188,6 +188,17 @@ const char* t9gb_status_string(int status)
 
 const char* t9gb_last_error(const t9gb_context* h) { return h ? h->c.last_error.c_str() : "null context"; }
 
+// Lanes per atom of the field kernels: 8 on small boxes, 4 where the box
+// fills the GPU (GB300 induce: 12,288 atoms 0.573 / 0.631 ms at 8 / 4 lanes;
+// 98,304 atoms 2.588 / 2.514 ms), 16 where even their eight lanes leave most of
+// it idle (648 atoms 0.320 / 0.301 ms at 8 / 16 lanes, 1,029 atoms 0.332 /
+// 0.343).  8 there too while the learned guess trains: its weights follow
+// the order of the fields' sums (fft_conv).
+static int default_pair_lanes(const Context* ctx)
+{
+   return ctx->npad > 32768 ? 4 : (ctx->npad > 768 || (ctx->learn_mode & 1) ? 8 : 16);
+}
+
 int t9gb_create(const t9gb_config* cfg, t9gb_context** out)
 {
    if (!cfg || !out || cfg->n <= 0)
@@ -214,13 +225,8 @@ int t9gb_create(const t9gb_config* cfg, t9gb_context** out)
    ctx->cfg = *cfg;
    ctx->n = cfg->n;
    ctx->npad = ((cfg->n + WARP - 1) / WARP) * WARP;
-   // lanes per atom of the field kernels: 8 on small boxes, 4 where the box
-   // fills the GPU (GB300 induce: 12,288 atoms 0.573 / 0.631 ms at 8 / 4
-   // lanes; 98,304 atoms 2.588 / 2.514 ms), 16 where even their eight lanes
-   // leave most of it idle (648 atoms 0.320 / 0.301 ms at 8 / 16 lanes, 1,029
-   // atoms 0.332 / 0.343)
-   ctx->pair_lanes = ctx->npad > 32768 ? 4 : (ctx->npad > 768 ? 8 : 16);
-   // and of the real-space force kernel, whose rows are a serial chain of
+   ctx->pair_lanes = default_pair_lanes(ctx);
+   // lanes of the real-space force kernel, whose rows are a serial chain of
    // long pair terms on a small box (10 MD steps at 4 / 8 / 16 lanes: 648
    // atoms 3.44 / 3.12 / 3.04 ms, 1,200 3.17 / 3.06 / 3.01, 2,187 4.12 / 4.00
    // / 3.78, 2,550 4.24 / 3.89 / 4.00, 3,000 4.49 / 4.28 / 4.41, 3,993 4.86 /
@@ -605,6 +611,11 @@ int t9gb_learn_config(t9gb_context* h, int mode, double lr, double weight_decay)
    if ((mode & 2) && !(ctx->learn_mode & 2))
       ctx->learn_since_probe = 1 << 30;  // first solve compares both starts
    ctx->learn_mode = mode;
+   if (ctx->pair_lanes_auto && ctx->pair_lanes != default_pair_lanes(ctx)) {
+      drop_graphs(ctx);
+      ctx->list_stale = true;  // the sub-lists are tiled for the lane count
+      ctx->pair_lanes = default_pair_lanes(ctx);
+   }
    ctx->learn_lr = (float)lr;
    ctx->learn_wd = (float)weight_decay;
    return T9GB_OK;
@@ -619,6 +630,7 @@ int t9gb_pair_lanes(t9gb_context* h, int lanes)
       h->c.list_stale = true;  // the sub-lists are tiled for the lane count
    }
    h->c.pair_lanes = lanes;
+   h->c.pair_lanes_auto = false;
    return T9GB_OK;
 }
 

@@ -1934,7 +1934,11 @@ static int fft_conv(Context* ctx, int vir = 0, float wE = 0.f, float wP = 0.f, b
    const int cb = (int)std::min<size_t>((ng + 255) / 256, 152 * 16);
    prof_begin(ctx, P_FFT_CONV);
    int* range = ctx->status + (P.probe ? ST_RANGE_L : ST_RANGE);
-   if (P.small_fft && !vir) {
+   // while the learned guess trains, the transform that its weights were trained
+   // with: AdamW's first steps divide by the size of a gradient, so a weight
+   // of a small one follows the rounding of the dipoles (2.3e-5 of the weights
+   // of 954 atoms between the two transforms, the dipoles 5e-7)
+   if (P.small_fft && !vir && !(ctx->learn_mode & 1)) {
       T9_CHECK(launch_small_fft(ctx, range));
       prof_end(ctx);
       return T9GB_OK;
