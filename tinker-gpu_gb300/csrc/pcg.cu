@@ -282,6 +282,9 @@ __global__ void __launch_bounds__(STEP_THREADS) k_pcg_step(VecArgs A, const floa
    const float* __restrict__ fld2, const float* __restrict__ conj, float* __restrict__ uind, float* __restrict__ rsd,
    double* __restrict__ scal)
 {
+   // the peers' shared memory is written only once they have all started: the
+   // wait for it, before the stores, overlaps the loads
+   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
    pdl_wait();
    pdl_trigger();  // the preconditioner may stage its blocks
    __shared__ float wsum[2][STEP_THREADS / 32];
@@ -317,6 +320,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_pcg_step(VecArgs A, const floa
       wsum[1][w] = dp;
    }
    __syncthreads();
+   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
    if (w == 0) {  // half-warp h sums system h over the warps, in FP64
       double b = (double)wsum[lane >> 4][lane & 15];
 #pragma unroll
