@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256) k_ehal(PairParams P, int npad, float cut,
          for (int q = 0; q < HAL_CHUNK; ++q)
             if (j[q] >= 0) {
                const float3 d = sep(P, a, b[q]);
-               if (d.x * d.x + d.y * d.y + d.z * d.z <= off2) {
+               if (!(d.x * d.x + d.y * d.y + d.z * d.z > off2)) {  // a NaN is evaluated, as in hal_add
                   hq[(head + len) & (HAL_QUEUE - 1)][threadIdx.x] = make_float4(d.x, d.y, d.z, b[q].w);
                   ++len;
                }
