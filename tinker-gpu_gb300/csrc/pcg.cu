@@ -271,9 +271,9 @@ __global__ void k_pcg_p2(VecArgs A, const double* __restrict__ scal, float* __re
 // cluster barrier; k_pcg_p1 needs a round of atomics and a second read of the
 // partials by its last block, and k_pcg_p2 a launch.  GB300, a solve of 648 /
 // 1,500 / 2,187 / 3,000 atoms: 300 / 339 / 400 / 437 -> 277 / 321 / 384 / 424
-// us.  The line lies where a thread holds five elements; the sum's order is
-// another one, and larger boxes, whose trajectories are the more sensitive to
-// it, keep theirs.
+// us.  The line lies where a thread holds five elements.  The sum is
+// k_pcg_p1's up to the order of its FP64 additions: the products of 32
+// consecutive elements in FP32, everything above them in FP64.
 constexpr int STEP_CL = 8, STEP_THREADS = 512;
 constexpr int STEP_MAX = 3072;  // slots
 constexpr int STEP_PER = (6 * STEP_MAX + STEP_CL * STEP_THREADS - 1) / (STEP_CL * STEP_THREADS);
@@ -287,16 +287,17 @@ __global__ void __launch_bounds__(STEP_THREADS) k_pcg_step(VecArgs A, const floa
    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
    pdl_wait();
    pdl_trigger();  // the preconditioner may stage its blocks
-   __shared__ float wsum[2][STEP_THREADS / 32];
+   __shared__ float wsum[2 * STEP_PER][STEP_THREADS / 32];
    __shared__ double part[2][STEP_CL];
    __shared__ float step[2];
    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
    float p[STEP_PER], v[STEP_PER], u[STEP_PER], r[STEP_PER];
-   float dd = 0.f, dp = 0.f;
+   float d[2 * STEP_PER];  // product k of system h at [2 k + h]
 #pragma unroll
    for (int k = 0; k < STEP_PER; ++k) {
       const int e = blockIdx.x * STEP_THREADS + threadIdx.x + k * STEP_CL * STEP_THREADS;
       p[k] = v[k] = u[k] = r[k] = 0.f;
+      d[2 * k] = d[2 * k + 1] = 0.f;
       if (e >= A.ne)
          continue;
       const int s = e / 6, x = e + 2 * s;  // row s, component e - 6 s of [npad][8]
@@ -305,24 +306,22 @@ __global__ void __launch_bounds__(STEP_THREADS) k_pcg_step(VecArgs A, const floa
       r[k] = rsd[x];
       const float f = fld2 ? fld[x] + fld2[x] : fld[x];
       v[k] = A.polinv[s] * p[k] - f;
+      const float pv = p[k] * v[k];
       if (e - 6 * s < 3)
-         dd += p[k] * v[k];
+         d[2 * k] = pv;
       else
-         dp += p[k] * v[k];
+         d[2 * k + 1] = pv;
    }
-#pragma unroll
-   for (int o = 16; o > 0; o >>= 1) {
-      dd += __shfl_xor_sync(0xffffffffu, dd, o);
-      dp += __shfl_xor_sync(0xffffffffu, dp, o);
-   }
-   if (lane == 0) {
-      wsum[0][w] = dd;
-      wsum[1][w] = dp;
-   }
+   const float ws = warp_sums<2 * STEP_PER>(d, lane);
+   const int slot = sum_slot<2 * STEP_PER>(lane);
+   if (slot >= 0)
+      wsum[slot][w] = ws;
    __syncthreads();
    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
    if (w == 0) {  // half-warp h sums system h over the warps, in FP64
       double b = (double)wsum[lane >> 4][lane & 15];
+      for (int k = 1; k * STEP_CL * STEP_THREADS < A.ne; ++k)
+         b += (double)wsum[2 * k + (lane >> 4)][lane & 15];
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1)
          b += __shfl_xor_sync(0xffffffffu, b, o);
