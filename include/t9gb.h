@@ -318,24 +318,25 @@ int t9gb_use_graph(t9gb_context* ctx, int enable);
  * clears the fixed-point grid, a z-line pass that applies the influence
  * function between the forward and inverse transforms, and an inverse 2-D
  * plane pass) or cuFFT C2C plus separate conversion and convolution kernels
- * (enable = 0).  The default, where this is not called, is the fastest
- * measured on GB300: on cubic grids of 16, 18, 20, 24, 30, 32, 36 or 40
- * points per edge one kernel on one thread-block cluster for everything from
- * the fixed-point grid to the potential (but where a virial reads the
- * transformed grid, and while the learned guess trains, whose weights follow the
- * rounding of the dipoles: there as below, 32^3 with the fused transform); on 64^3 the fused transform; cuFFT on
- * every other grid, 128^3 included.  Replaces fftfront/fftback +
+ * (enable = 0).  The default (not called, or enable = -1, which takes an
+ * earlier choice back) is the fastest measured on GB300: on cubic grids of
+ * 16, 18, 20, 24, 30, 32, 36 or 40 points per edge one kernel on one
+ * thread-block cluster for everything from the fixed-point grid to the
+ * potential (but where a virial reads the transformed grid, and while the
+ * learned guess trains, whose weights follow the rounding of the dipoles:
+ * there as below, 32^3 with the fused transform); on 64^3 the fused
+ * transform; cuFFT on every other grid, 128^3 included.  Replaces fftfront/fftback +
  * pmeConv (src/cudart/fft.cpp:65-95, src/cu/pme.cu:908-1031).  Enabling on
  * an unsupported grid returns T9GB_BAD_ARG. */
 int t9gb_pme_own_fft(t9gb_context* ctx, int enable);
 
-/* Partition of the fused transform's two plane passes (which a call of this
- * selects on 32^3): ctas = 0 (the
+/* Partition of the fused transform's two plane passes: ctas = 0 (the
  * default) runs one CTA per z plane; 2, 4 or 8 (8 on grids of 64 points
  * per edge or more) spread each plane over a thread-block cluster of that
  * many CTAs, which stage their row slabs with bulk asynchronous copies and
- * exchange rows for columns through distributed shared memory.
- * Bit-identical results either way.  A tuning knob: on GB300 at 64^3 the
+ * exchange rows for columns through distributed shared memory (on 32^3 in
+ * place of the default's one kernel, until ctas = 0).
+ * Bit-identical results with 0, 2, 4 or 8.  A tuning knob: on GB300 at 64^3 the
  * clustered passes measured 22.8 / 24.2 / 25.0 us per transform +
  * convolution against 21.0 us for one CTA per plane. */
 int t9gb_pme_fft_cluster(t9gb_context* ctx, int ctas);

@@ -420,8 +420,8 @@ class Engine:
         return e.value
 
     def pme_own_fft(self, enable=True):
-        """Fused power-of-two FFT (default where supported) or cuFFT."""
-        self._check(self.lib.t9gb_pme_own_fft(self.h, 1 if enable else 0))
+        """Fused power-of-two FFT (True) or cuFFT (False); -1: the default of the grid."""
+        self._check(self.lib.t9gb_pme_own_fft(self.h, -1 if enable == -1 else 1 if enable else 0))
 
     def fft_cluster(self, ctas=4):
         """CTAs per z plane in the fused transform's plane passes (0: one)."""

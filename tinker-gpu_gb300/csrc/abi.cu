@@ -660,11 +660,8 @@ int t9gb_pme_fft_cluster(t9gb_context* h, int ctas)
    const int n = ctx->pme.n1;
    if (!(ctas == 0 || ((ctas == 2 || ctas == 4 || (ctas == 8 && n >= 64)) && ctx->pme.own_fft_ok)))
       return T9GB_BAD_ARG;
-   const bool small = ctx->pme.small_fft && !ctx->pme.own_fft_ok;
-   if (ctas != ctx->pme.fft_cl || small != ctx->pme.small_fft)
+   if (pme_choose(ctx->pme, ctx->pme.choice, ctas))
       drop_graphs(ctx);
-   ctx->pme.small_fft = small;
-   ctx->pme.fft_cl = ctas;
    return T9GB_OK;
 }
 
@@ -730,12 +727,10 @@ int t9gb_pme_own_fft(t9gb_context* h, int enable)
    if (!h)
       return T9GB_BAD_ARG;
    Context* ctx = &h->c;
-   if (enable && !ctx->pme.own_fft_ok)
+   if (enable > 0 && !ctx->pme.own_fft_ok)
       return T9GB_BAD_ARG;
-   if ((enable != 0) != ctx->pme.own_fft || ctx->pme.small_fft)
+   if (pme_choose(ctx->pme, enable < 0 ? -1 : enable != 0, ctx->pme.fft_cl))
       drop_graphs(ctx);
-   ctx->pme.own_fft = enable != 0;
-   ctx->pme.small_fft = false;
    return T9GB_OK;
 }
 

@@ -102,6 +102,7 @@ struct ListView {
 
 struct PmeGrid {
    int n1 = 0, n2 = 0, n3 = 0;
+   int choice = -1;           // t9gb_pme_own_fft: cuFFT (0), the fused path (1) or the default (-1)
    bool own_fft = false;      // power-of-two grid: the library's fused FFT path
    bool own_fft_ok = false;   // the grid qualifies
    cufftHandle plan = 0, plan2 = 0;
@@ -120,7 +121,7 @@ struct PmeGrid {
    int fft_cl = 0;            // fused transform: CTAs per z plane (a thread-block cluster), 0: one CTA
    int* fft_err = nullptr;    // device flag: a staged slab copy of a plane pass did not complete in time
    bool small_fft = false;    // small cubic grid: transform and convolution as one cluster's work
-   float2* small_tw = nullptr;  // its twiddles, e^{-2 pi i k / n1}
+   float2* small_tw = nullptr;  // its twiddles, e^{-2 pi i k / n1}; null: no such kernel for the grid
 };
 
 // Per-kernel event timing (tracing): categories of timed launches.
@@ -630,6 +631,8 @@ int launch_ufield_recip_gather_dir(Context* ctx, float* out6, const PcgAp& P);
 // the same on the second grid (and FFT plan)
 int launch_ufield_recip_grid_alt(Context* ctx, const float* u6);
 int launch_ufield_recip_gather_alt(Context* ctx, const float* u6, float* out6);
+// the transform for the caller's choices; true: another one than before
+bool pme_choose(PmeGrid& P, int choice, int fft_cl);
 // sorted positions of ctx->xyz, or of src, which is then copied there too
 int scatter_positions(Context* ctx, const float* src = nullptr);
 // t9gb_emplar(grad) with `beside` called once the dipoles are solved and the

@@ -1360,7 +1360,6 @@ static int small_fft_setup(Context* ctx)
    }
    T9_CUDA(cudaMalloc(&P.small_tw, sizeof(float2) * tw.size()));
    T9_CUDA(cudaMemcpy(P.small_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
-   P.small_fft = true;
    return T9GB_OK;
 }
 
@@ -1842,10 +1841,8 @@ int pme_setup(Context* ctx)
    }
    // the fused FFT: cubic grids of 32, 64 or 128 points per edge
    P.own_fft_ok = P.n1 == P.n2 && P.n2 == P.n3 && (P.n1 == 32 || P.n1 == 64 || P.n1 == 128);
-   // default where it measured faster than cuFFT on GB300 (64^3: 0.627 vs
-   // 0.634 ms per induce step in the graph); at 128^3 cuFFT is faster
-   P.own_fft = P.own_fft_ok && P.n1 <= 64;
    T9_CHECK(small_fft_setup(ctx));
+   pme_choose(P, -1, 0);
    if (P.own_fft_ok) {
       if (P.n1 == 32)
          T9_CHECK(fft_setup_kernels<32>(ctx));
@@ -1860,6 +1857,22 @@ int pme_setup(Context* ctx)
       T9_CUDA(cudaDeviceSynchronize());
    }
    return T9GB_OK;
+}
+
+// The fused transform is the default where it measured faster than cuFFT on
+// GB300 (64^3: 0.627 vs 0.634 ms per induce step in the graph; at 128^3 cuFFT
+// is faster); the one-cluster transform where it has a kernel and nothing else
+// was asked for.  Every choice can be taken back.
+bool pme_choose(PmeGrid& P, int choice, int fft_cl)
+{
+   const bool own = choice < 0 ? P.own_fft_ok && P.n1 <= 64 : choice != 0;
+   const bool small = P.small_tw && choice < 0 && fft_cl == 0;
+   const bool changed = own != P.own_fft || small != P.small_fft || fft_cl != P.fft_cl;
+   P.choice = choice;
+   P.fft_cl = fft_cl;
+   P.own_fft = own;
+   P.small_fft = small;
+   return changed;
 }
 
 void pme_free(Context* ctx)
