@@ -331,6 +331,8 @@ struct Context {
    int pcg_fuse = 121;            // t9gb_set_pcg_fusion (bit 4: programmatic dependent launch, bits 5-6: gather and stream layout)
    int force_lanes = 4;           // lanes per atom in the real-space force kernel
    bool list_stale = true;        // positions changed since the last list check
+   int list_have = 0;             // else: the parts of the sub-lists formed for them (LIST_...)
+   int list_used = 0;             // the parts that calls asked for at these positions, or those before
    bool list_need_build = true;   // no valid list for the current order / capacity
    float4* sref = nullptr;        // [npad] positions at the last list build
    int* lflag = nullptr;          // device: rebuild requested / an atom moved too far
@@ -589,7 +591,16 @@ inline ListView nbr_view(const Context* ctx) { return {ctx->nbr, ctx->nbr_cap, 5
 // ---- entry points implemented across the translation units ----
 int order_build(Context* ctx);  // host: spatial order, scaled partners
 int list_update(Context* ctx);  // device: exact neighbour list
-int ensure_list(Context* ctx);  // list_update when the coordinates changed
+// Parts of the per-step sub-lists: the cutoff one, the field factors of its
+// entries, and the preconditioner's with its factors.
+enum { LIST_CUT = 1, LIST_FIELD = 3, LIST_PRECOND = 4, LIST_ALL = 7 };
+// the stored list and the parts of the sub-lists a call needs, at the current
+// positions; list_ready: they are there
+int ensure_list(Context* ctx, int need);
+inline bool list_ready(const Context* ctx, int need)
+{
+   return !ctx->list_stale && !ctx->list_need_build && (need & ~ctx->list_have) == 0;
+}
 int check_list_overflow(Context* ctx, int* redo);
 int lx_config(Context* ctx, int order);   // pcg.cu
 int lx_state(Context* ctx, int* fits, int* rejected, float* coef16);  // pcg.cu
@@ -597,7 +608,7 @@ int lx_wait(Context* ctx);                // pcg.cu
 int alloc_lists(Context* ctx, int cap);          // nbr, nbrc, nbrp with row capacity cap
 int pair_staging_setup();                         // pair.cu: shared-memory limits of the staged kernels
 int mlp_tc_setup();                               // mlp.cu: shared-memory limit of the tcgen05 forward
-int launch_list_filter(Context* ctx);             // pair.cu  // after a sync; redo = 1: grown, repeat
+int launch_list_filter(Context* ctx, int parts);  // pair.cu  // after a sync; redo = 1: grown, repeat
 // The fused kernels of a CG iteration: the sparse preconditioner with the
 // r.z / r.r sums and the CG scalars (pair.cu), and the mutual-field gather
 // with Ap = p/alpha - field, p.Ap and the step length (pme.cu).

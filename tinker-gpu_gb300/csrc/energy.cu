@@ -99,7 +99,7 @@ extern "C" int t9gb_empole_energy(t9gb_context* h, double* energy, double* parts
    if (!ctx->have_order)
       return T9GB_NOT_READY;
    for (int attempt = 0; attempt < 2; ++attempt) {
-      T9_CHECK(ensure_list(ctx));
+      T9_CHECK(ensure_list(ctx, LIST_CUT));
       T9_CUDA(cudaMemsetAsync(ctx->e_atom, 0, sizeof(double) * 3 * ctx->npad, ctx->stream));
       T9_CHECK(launch_empole_real(ctx, ctx->e_atom));
       T9_CHECK(launch_empole_recip(ctx, ctx->e_atom + ctx->npad));
@@ -250,8 +250,8 @@ static int elec_terms(Context* ctx, bool mpole, bool polar, int vers, double* en
       // a list refreshed here needs its capacity checked; one already checked
       // (after the solve above, or an earlier call) does not, and the gradient
       // then stays in stream order without a synchronisation
-      const bool fresh = ctx->list_stale || ctx->list_need_build;
-      T9_CHECK(ensure_list(ctx));
+      const bool fresh = !list_ready(ctx, LIST_CUT);
+      T9_CHECK(ensure_list(ctx, LIST_CUT));
       // work that reads the list starts once the list is final: here when it
       // was current already, else after the capacity check below
       if (beside && !beside_done && !fresh) {
@@ -325,7 +325,7 @@ int emplar_grad_beside(Context* ctx, float* grad, const std::function<int()>& be
       return T9GB_OK;
    if (queued)
       T9_CHECK(reset());
-   T9_CHECK(ensure_list(ctx));
+   T9_CHECK(ensure_list(ctx, LIST_CUT));
    return forces();
 }
 

@@ -821,8 +821,15 @@ __device__ __forceinline__ void pair_factors(const PairParams& P, float r2, floa
 
 // The blocks past the rows' form the scaled partners' factors, a thread per
 // entry of the partner table (a warp per row had two lanes at work there).
-template <bool STAGE>
-__global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filter(PairParams P, float cutp2, int npad,
+// PARTS (LIST_...): what to form.  A solve and the fields take everything;
+// the energies and forces read the cutoff sub-list alone and the preconditioner
+// by itself its own, and would pay for factors that nothing reads (GB300,
+// 98,304 atoms, calls after a position update: preconditioner 361 -> 283 us,
+// multipole energy without Ewald sum 416 -> 330, van der Waals, which reads
+// the stored rows, 580 -> 365; the preconditioner's filter 142 us at five
+// blocks an SM, 129 at six, 138 at eight).
+template <bool STAGE, int PARTS>
+__global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : PARTS == LIST_PRECOND ? 6 : 5) k_list_filter(PairParams P, float cutp2, int npad,
    const int* __restrict__ nbr, const int* __restrict__ nnbr, const int* __restrict__ sp_j,
    const int* __restrict__ sp_i, int nsp, const float4* __restrict__ sp_sc,
    const float4* __restrict__ spos, const float2* __restrict__ stag, FilterOut O)
@@ -832,6 +839,7 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filt
    constexpr int NW = STAGE ? 32 : 8;
    __shared__ float4 q_d[NW][64];  // separation, partner's pdamp
    __shared__ int q_j[NW][64];
+   constexpr bool CUT = PARTS & LIST_CUT, PRE = PARTS & LIST_PRECOND, FIELD = (PARTS & LIST_FIELD) == LIST_FIELD;
    const int blk = blockIdx.x;
    if (blk >= npad / NW) {
       const int q = (blk - npad / NW) * blockDim.x + threadIdx.x;
@@ -845,8 +853,10 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filt
       float2 u, f, c;
       pair_factors(P, r2, sp_sc[q].w, pi.w, pk.w, pair_gamma(P, ti.x, tk.x), ti.y * tk.y, u, f, c);
       // zero factors beyond the cutoff
-      O.spu[q] = r2 <= P.cut2 ? u : make_float2(0.f, 0.f);
-      O.spp[q] = r2 <= cutp2 ? c : make_float2(0.f, 0.f);
+      if (FIELD)
+         O.spu[q] = r2 <= P.cut2 ? u : make_float2(0.f, 0.f);
+      if (PRE)
+         O.spp[q] = r2 <= cutp2 ? c : make_float2(0.f, 0.f);
       return;
    }
    const int words = (npad / 32 + 31) / 32;
@@ -866,7 +876,7 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filt
       const float2 ti = stag[i];  // thole or type, polarizability
       const int* row = nbr + (size_t)i * P.cap;
       const int cnt = nnbr[i];
-      const float rmax2 = fmaxf(P.cut2, cutp2);
+      const float rmax2 = CUT && PRE ? fmaxf(P.cut2, cutp2) : CUT ? P.cut2 : cutp2;
       const unsigned lt = (1u << lane) - 1u;
       // the row's place in the tiled lists, and an entry's from it
       const size_t base = V.at(i, 0);
@@ -884,15 +894,17 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filt
          const float2 tk = stag[j];
          const float4 dk = valid ? q_d[warp][lane] : make_float4(1.f, 0.f, 0.f, 1.f);
          const float r2 = dk.x * dk.x + dk.y * dk.y + dk.z * dk.z;
-         const bool inc = valid && r2 <= P.cut2, inp = valid && r2 <= cutp2;
+         const bool inc = CUT && valid && r2 <= P.cut2, inp = PRE && valid && r2 <= cutp2;
          const unsigned mc = __ballot_sync(0xffffffffu, inc), mp = __ballot_sync(0xffffffffu, inp);
          float2 u, f, c;
          pair_factors(P, r2, 1.f, pi.w, dk.w, pair_gamma(P, ti.x, tk.x), ti.y * tk.y, u, f, c);
          if (inc) {
             const unsigned k = oc + __popc(mc & lt), at = ((k >> sg) << 5) + (k & gm);
             nc[at] = j;
-            cu[at] = u;
-            cd[at] = f;
+            if (FIELD) {
+               cu[at] = u;
+               cd[at] = f;
+            }
          }
          if (inp) {
             const unsigned k = op + __popc(mp & lt), at = ((k >> sg) << 5) + (k & gm);
@@ -912,6 +924,14 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filt
          const float3 d = sep(P, pi, pk);
          const bool acc = in && d.x * d.x + d.y * d.y + d.z * d.z <= rmax2;
          const unsigned m = __ballot_sync(0xffffffffu, acc);
+         if (PARTS == LIST_CUT) {  // indices alone: nothing to queue for
+            const unsigned k = oc + __popc(m & lt);
+            if (acc)
+               nc[((k >> sg) << 5) + (k & gm)] = j;
+            oc += __popc(m);
+            j = jn;
+            continue;
+         }
          if (acc) {
             const int p = qn + __popc(m & lt);
             q_d[warp][p] = make_float4(d.x, d.y, d.z, pk.w);
@@ -935,8 +955,10 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filt
          drain(qn);
    }
    if (lane == 0) {
-      O.nnbrc[i] = oc;
-      O.nnbrp[i] = op;
+      if (CUT)
+         O.nnbrc[i] = oc;
+      if (PRE)
+         O.nnbrp[i] = op;
    }
    if (!STAGE)
       return;
@@ -993,8 +1015,9 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : 5) k_list_filt
    }
 }
 
-int launch_list_filter(Context* ctx)
+int launch_list_filter(Context* ctx, int parts)
 {
+   const bool cut = parts == LIST_CUT && !ctx->pair_staged, pre = parts == LIST_PRECOND && !ctx->pair_staged;
    PairParams P = make_params(ctx, ctx->cfg.cutoff);
    const double cp = ctx->cfg.usolve_cutoff + ctx->cfg.pbuffer;
    const float cutp2 = cp * cp > 3.0e38 ? 3.0e38f : (float)(cp * cp);
@@ -1007,11 +1030,15 @@ int launch_list_filter(Context* ctx)
    FilterOut O{nbrc_view(ctx).sg, ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp, ctx->cfu, ctx->cfd, ctx->cfp, ctx->spu,
       ctx->spp, ctx->jbl, ctx->jbn, ctx->nbrc_l, ctx->nbrp_l};
    if (ctx->pair_staged)
-      k_list_filter<true><<<nblk + grid_for(ctx->nsp, 1024), 1024, smem, ctx->stream>>>(P, cutp2, ctx->npad, nbr, nnbr,
-         ctx->sp_j, ctx->sp_i, ctx->nsp, ctx->sp_sc, ctx->spos, ctx->stag, O);
-   else
-      k_list_filter<false><<<ctx->npad / 8 + grid_for(ctx->nsp, 256), 256, 0, ctx->stream>>>(P, cutp2, ctx->npad, nbr,
+      k_list_filter<true, LIST_ALL><<<nblk + grid_for(ctx->nsp, 1024), 1024, smem, ctx->stream>>>(P, cutp2, ctx->npad,
+         nbr, nnbr, ctx->sp_j, ctx->sp_i, ctx->nsp, ctx->sp_sc, ctx->spos, ctx->stag, O);
+   else {
+      auto k = cut ? k_list_filter<false, LIST_CUT> : pre ? k_list_filter<false, LIST_PRECOND>
+                                                          : k_list_filter<false, LIST_ALL>;
+      k<<<ctx->npad / 8 + (cut ? 0 : grid_for(ctx->nsp, 256)), 256, 0, ctx->stream>>>(P, cutp2, ctx->npad, nbr,
          nnbr, ctx->sp_j, ctx->sp_i, ctx->nsp, ctx->sp_sc, ctx->spos, ctx->stag, O);
+   }
+   ctx->list_have = cut || pre ? parts : LIST_ALL;
    T9_CUDA(cudaGetLastError());
    return T9GB_OK;
 }
@@ -1074,7 +1101,7 @@ int pair_staging_setup()
       cudaFuncSetAttribute(k_precond_dots_stg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
       return T9GB_CUDA_ERR;
    // the block bitmap and its prefix counts: 8 bytes per 1,024 slots
-   if (cudaFuncSetAttribute(k_list_filter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) !=
+   if (cudaFuncSetAttribute(k_list_filter<true, LIST_ALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) !=
       cudaSuccess)
       return T9GB_CUDA_ERR;
    return T9GB_OK;

@@ -766,18 +766,33 @@ static int list_build_body(Context* ctx)
    return T9GB_OK;
 }
 
-// host-driven refresh (one synchronisation)
-int ensure_list(Context* ctx)
+// host-driven refresh (one synchronisation where the positions are new).  The
+// sub-lists get the parts that the call needs and, at new positions, those
+// that the calls at the positions before asked for: a program that makes the
+// same calls at every step filters once a step.
+int ensure_list(Context* ctx, int need)
 {
-   if (!ctx->list_stale && !ctx->list_need_build)
+   if (list_ready(ctx, need)) {
+      ctx->list_used |= need;
       return T9GB_OK;
-   T9_CHECK(list_request(ctx));
-   T9_CHECK(launch_disp_check(ctx, 0, 0));
-   T9_CUDA(cudaMemcpyAsync(ctx->h_lflag, ctx->lflag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-   T9_CUDA(cudaStreamSynchronize(ctx->stream));
-   if (*ctx->h_lflag)
-      T9_CHECK(list_build_body(ctx));
-   T9_CHECK(launch_list_filter(ctx));
+   }
+   int parts = need;
+   if (ctx->list_stale || ctx->list_need_build) {
+      T9_CHECK(list_request(ctx));
+      T9_CHECK(launch_disp_check(ctx, 0, 0));
+      T9_CUDA(cudaMemcpyAsync(ctx->h_lflag, ctx->lflag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      T9_CUDA(cudaStreamSynchronize(ctx->stream));
+      if (*ctx->h_lflag)
+         T9_CHECK(list_build_body(ctx));
+      parts |= ctx->list_used;
+      ctx->list_used = need;
+      ctx->list_have = 0;
+   } else {
+      parts |= ctx->list_have;
+      ctx->list_used |= need;
+   }
+   if (parts)
+      T9_CHECK(launch_list_filter(ctx, parts));
    T9_CUDA(cudaMemcpyAsync(ctx->h_over, ctx->nbr_over, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
    ctx->list_stale = false;
    return T9GB_OK;
@@ -819,7 +834,7 @@ static int list_refresh_graph(Context* ctx)
       rc = T9GB_CUDA_ERR;
    T9_CHECK(rc);
    // the largest row reaches the host with the solve's status (k_finish)
-   return launch_list_filter(ctx);
+   return launch_list_filter(ctx, LIST_ALL);
 }
 
 // after a synchronisation: grow the list if an atom had more neighbours than
@@ -1060,7 +1075,7 @@ static int pcg_start_predict(Context* ctx, const VecArgs& A, bool graph)
    }
    ctx->stream = main;
    T9_CHECK(rc);
-   T9_CHECK(graph ? list_refresh_graph(ctx) : ensure_list(ctx));
+   T9_CHECK(graph ? list_refresh_graph(ctx) : ensure_list(ctx, LIST_ALL));
    // the real-space fields: the guess's on side 2 (then its gather, after the
    // grid), the permanent one here (then its gather)
    T9_CHECK(recip_fork(ctx, 2));
@@ -1101,12 +1116,12 @@ static int pcg_start(Context* ctx, const VecArgs& A, bool graph, int variant)
       const int rc = launch_dfield_recip_grid(ctx);
       ctx->stream = main;
       T9_CHECK(rc);
-      T9_CHECK(graph ? list_refresh_graph(ctx) : ensure_list(ctx));
+      T9_CHECK(graph ? list_refresh_graph(ctx) : ensure_list(ctx, LIST_ALL));
       T9_CHECK(launch_dfield_real(ctx, nullptr, ctx->fld6));
       T9_CHECK(recip_join(ctx, 0));
       T9_CHECK(launch_dfield_recip_gather(ctx, ctx->fld6, true));
    } else {
-      T9_CHECK(graph ? list_refresh_graph(ctx) : ensure_list(ctx));
+      T9_CHECK(graph ? list_refresh_graph(ctx) : ensure_list(ctx, LIST_ALL));
       T9_CHECK(dfield6(ctx, ctx->fld6));
    }
    k_init_guess<<<A.nb, VB, 0, ctx->stream>>>(A, ctx->fld6, ctx->efield, ctx->udir, ctx->uind, c.pcgguess,
@@ -1266,6 +1281,7 @@ static int induce_graph(Context* ctx, int variant)
       T9_CUDA(cudaStreamSynchronize(ctx->stream));
    }
    ctx->list_stale = false;
+   ctx->list_have = LIST_ALL;
    return T9GB_OK;
 }
 
@@ -1469,10 +1485,10 @@ int reset_predictor(Context* ctx)
 // public field entry points (sorted internally, caller order at the boundary)
 
 template <class F>
-static int with_list(Context* ctx, F&& body)
+static int with_list(Context* ctx, int need, F&& body)
 {
    for (int attempt = 0; attempt < 3; ++attempt) {
-      T9_CHECK(ensure_list(ctx));
+      T9_CHECK(ensure_list(ctx, need));
       T9_CHECK(body());
       T9_CUDA(cudaStreamSynchronize(ctx->stream));
       int redo = 0;
@@ -1497,7 +1513,7 @@ static int with_list(Context* ctx, F&& body)
 
 int public_dfield(Context* ctx, float* field, float* fieldp)
 {
-   return with_list(ctx, [&]() {
+   return with_list(ctx, LIST_ALL, [&]() {
       T9_CHECK(dfield6(ctx, ctx->tmp6));
       return scatter_from_sorted3(ctx, ctx->tmp6, field, fieldp);
    });
@@ -1505,7 +1521,7 @@ int public_dfield(Context* ctx, float* field, float* fieldp)
 
 int public_ufield(Context* ctx, const float* uind, const float* uinp, float* field, float* fieldp)
 {
-   return with_list(ctx, [&]() {
+   return with_list(ctx, LIST_ALL, [&]() {
       T9_CHECK(gather_to_sorted3(ctx, uind, uinp, ctx->tmp6));
       T9_CHECK(ufield6(ctx, ctx->tmp6, ctx->vec));
       return scatter_from_sorted3(ctx, ctx->vec, field, fieldp);
@@ -1514,7 +1530,7 @@ int public_ufield(Context* ctx, const float* uind, const float* uinp, float* fie
 
 int public_precond(Context* ctx, const float* rsd, const float* rsdp, float* zrsd, float* zrsdp)
 {
-   return with_list(ctx, [&]() {
+   return with_list(ctx, LIST_PRECOND, [&]() {
       T9_CHECK(gather_to_sorted3(ctx, rsd, rsdp, ctx->tmp6));
       T9_CHECK(launch_precond_sparse(ctx, ctx->tmp6, ctx->vec));
       return scatter_from_sorted3(ctx, ctx->vec, zrsd, zrsdp);
