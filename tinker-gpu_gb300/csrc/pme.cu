@@ -2176,9 +2176,15 @@ int launch_empole_recip(Context* ctx, double* e_atom)
 }  // namespace t9gb
 
 namespace t9gb {
-// atoms per warp of the force gathers: eight where that still gives an SM 20
-// warps, four below
-static int force_atoms(int n) { return n > 24576 ? 8 : 4; }
+// Atoms per warp of the force gathers: eight where that still gives an SM 20
+// warps, four below, one where four leave most of the chip idle (both
+// kernels, us at one / four atoms: 648 atoms 15 / 23, 3,000 17 / 24, 5,184
+// 24 / 25, 8,232 29 / 26)
+static int force_atoms(int n) { return n > 24576 ? 8 : (n > 6144 ? 4 : 1); }
+
+// a kernel by that number
+#define T9_FORCE_ATOMS(FA, KERNEL, ...)                                                                                \
+   ((FA) == 8 ? KERNEL<__VA_ARGS__ 8> : (FA) == 4 ? KERNEL<__VA_ARGS__ 4> : KERNEL<__VA_ARGS__ 1>)
 
 // reciprocal forces for elec_forces (force.cu), in two halves: the
 // permanent-multipole grid (forces and torque fields of the multipoles, the
@@ -2205,9 +2211,9 @@ int launch_force_recip_perm(Context* ctx, bool mpole, bool polar, float* wrec)
    double* er = ctx->e_atom + np;
    double* es = ctx->e_atom + 2 * np;
    const int fa = force_atoms(ctx->n), fb = grid_for(ctx->n, FORCE_WARPS * fa);
-   auto k = mpole && polar ? (fa == 8 ? k_gather_force_perm<true, true, 8> : k_gather_force_perm<true, true, 4>)
-      : mpole              ? (fa == 8 ? k_gather_force_perm<true, false, 8> : k_gather_force_perm<true, false, 4>)
-                           : (fa == 8 ? k_gather_force_perm<false, true, 8> : k_gather_force_perm<false, true, 4>);
+   auto k = mpole && polar ? T9_FORCE_ATOMS(fa, k_gather_force_perm, true, true, )
+      : mpole              ? T9_FORCE_ATOMS(fa, k_gather_force_perm, true, false, )
+                           : T9_FORCE_ATOMS(fa, k_gather_force_perm, false, true, );
    k<<<fb, 32 * FORCE_WARPS, 0, ctx->stream>>>(ctx->n, np, G, f, a, sites(ctx), ctx->pme.qgrid, ctx->srpole, ctx->uind,
       ctx->frecp, ctx->trecp, mpole ? er : nullptr, mpole ? es : nullptr, wrec);
    T9_CUDA(cudaGetLastError());
@@ -2236,7 +2242,7 @@ int launch_force_recip_uind(Context* ctx, float* wrec, bool alt)
       rc = fft_conv(ctx, vir ? 2 : 0, 0.f, 0.5f * f, false, ctx->scal + 46);
    if (rc == T9GB_OK) {
       const int fa = force_atoms(ctx->n);
-      auto k = fa == 8 ? k_gather_force_uind<8> : k_gather_force_uind<4>;
+      auto k = T9_FORCE_ATOMS(fa, k_gather_force_uind);
       k<<<grid_for(ctx->n, FORCE_WARPS * fa), 32 * FORCE_WARPS, 0, ctx->stream>>>(ctx->n, ctx->npad, G, f, sites(ctx),
          P.qgrid, ctx->srpole, ctx->uind, ctx->frecu, ctx->trecu, wrec);
       if (cudaGetLastError() != cudaSuccess)
