@@ -48,12 +48,12 @@ static int alloc_all(Context* ctx)
    T9_CUDA(cudaMemset(ctx->nnbrc, 0, sizeof(int) * npad));
    T9_CUDA(cudaMalloc(&ctx->nnbrp, sizeof(int) * npad));
    T9_CUDA(cudaMemset(ctx->nnbrp, 0, sizeof(int) * npad));
-   T9_CUDA(cudaMalloc(&ctx->nbr_over, sizeof(int)));
-   T9_CUDA(cudaMemset(ctx->nbr_over, 0, sizeof(int)));
+   T9_CUDA(cudaMalloc(&ctx->nbr_over, sizeof(int) * LIST_CAPS));
+   T9_CUDA(cudaMemset(ctx->nbr_over, 0, sizeof(int) * LIST_CAPS));
    T9_CUDA(cudaMalloc(&ctx->copy_err, sizeof(int)));
    T9_CUDA(cudaMemset(ctx->copy_err, 0, sizeof(int)));
-   T9_CUDA(cudaMallocHost(&ctx->h_over, sizeof(int)));
-   *ctx->h_over = 0;
+   T9_CUDA(cudaMallocHost(&ctx->h_over, sizeof(int) * LIST_CAPS));
+   std::fill(ctx->h_over, ctx->h_over + LIST_CAPS, 0);
    T9_CUDA(cudaMalloc(&ctx->cell_atoms, sizeof(int) * npad));
    T9_CUDA(cudaMalloc(&ctx->atom_cell, sizeof(int) * npad));
    float** v6[] = {&ctx->rcp6, &ctx->fld6, &ctx->udir, &ctx->efield, &ctx->uind, &ctx->rsd, &ctx->zrsd,

@@ -292,7 +292,8 @@ struct Context {
 
    // per-step neighbour list (exact cutoff, scaled partners excluded)
    float list_cut = 0;
-   int nbr_cap = 0;
+   int nbr_cap = 0;          // row capacity of the stored list
+   int cut_cap = 0, pre_cap = 0;  // of the cutoff and the preconditioner sub-lists (at most nbr_cap)
    int* nbr = nullptr;       // [npad][nbr_cap]
    int* nnbr = nullptr;      // [npad]
    int* nbre = nullptr;      // [npad][nbr_cap] the rows' part that the filter needs, or null: all of it
@@ -307,8 +308,8 @@ struct Context {
    // radial factors of every sub-list entry, formed by the filter: (b1, b2)
    // of the mutual field and (b2, b3) of the permanent one (nbrc), (c1, c2)
    // of the preconditioner (nbrp); and those of the scaled partners
-   float2* cfu = nullptr;    // [npad][nbr_cap], tiled
-   float2* cfd = nullptr;
+   float2* cfu = nullptr;    // [npad][cut_cap], tiled
+   float2* cfd = nullptr;    // [npad][pre_cap] for cfp
    float2* cfp = nullptr;
    float2* spu = nullptr;    // [nsp] mutual field
    float2* spp = nullptr;    // [nsp] preconditioner
@@ -319,12 +320,12 @@ struct Context {
    // slot within the block)
    int* jbl = nullptr;               // [npad / 32][STAGE_JB_CAP]
    int* jbn = nullptr;               // [npad / 32]
-   unsigned short* nbrc_l = nullptr; // [npad][nbr_cap]
-   unsigned short* nbrp_l = nullptr; // [npad][nbr_cap]
+   unsigned short* nbrc_l = nullptr; // [npad][cut_cap]
+   unsigned short* nbrp_l = nullptr; // [npad][pre_cap]
    bool pair_staged = false;         // t9gb_pair_staging
    bool mlp_tc = true;               // learned guess: forward pass on tcgen05 (t9gb_learn_tensor_path)
    int* copy_err = nullptr;          // device flag: a staging copy did not complete in time
-   int* nbr_over = nullptr;  // device max count seen (overflow check)
+   int* nbr_over = nullptr;  // [LIST_CAPS] device: largest row beyond each capacity (overflow check)
    int* h_over = nullptr;    // pinned mirror
    int pair_lanes = 8;            // lanes per atom in the field kernels
    bool pair_lanes_auto = true;   // they are the default's
@@ -453,6 +454,10 @@ constexpr double VDW_SITE_MARGIN = 0.25;
 // three blocks per SM); water blocks need 39 on average, 45 at most at a
 // 7 A cutoff
 constexpr int STAGE_JB_CAP = 48;
+
+// list capacities with an overflow word each: stored rows, cutoff sub-list,
+// preconditioner sub-list
+constexpr int LIST_CAPS = 3;
 
 // energy / virial row sums: at most SUM_ROWS_MAX rows per launch, each
 // split over SUM_PARTS blocks
@@ -584,7 +589,7 @@ inline void prof_collect(Context* ctx)
 inline ListView nbrc_view(const Context* ctx)
 {
    const int g = ctx->list_lanes;
-   return {ctx->nbrc, ctx->nbr_cap, g == 4 ? 2 : g == 8 ? 3 : g == 16 ? 4 : 5};
+   return {ctx->nbrc, ctx->cut_cap, g == 4 ? 2 : g == 8 ? 3 : g == 16 ? 4 : 5};
 }
 inline ListView nbr_view(const Context* ctx) { return {ctx->nbr, ctx->nbr_cap, 5}; }
 
@@ -601,14 +606,20 @@ inline bool list_ready(const Context* ctx, int need)
 {
    return !ctx->list_stale && !ctx->list_need_build && (need & ~ctx->list_have) == 0;
 }
+// after a synchronisation: grow a list that had too few entries a row; redo = 1:
+// grown, repeat.  One overflow can hide the next (a sub-list of rows that were
+// cut short), and the dipole grid's range may ask for a pass of its own: at most
+// four passes in all.
 int check_list_overflow(Context* ctx, int* redo);
+constexpr int LIST_PASSES = 5;
 int lx_config(Context* ctx, int order);   // pcg.cu
 int lx_state(Context* ctx, int* fits, int* rejected, float* coef16);  // pcg.cu
 int lx_wait(Context* ctx);                // pcg.cu
-int alloc_lists(Context* ctx, int cap);          // nbr, nbrc, nbrp with row capacity cap
+// the lists with the row capacities of the stored rows and the two sub-lists
+int alloc_lists(Context* ctx, int cap, int cut, int pre);
 int pair_staging_setup();                         // pair.cu: shared-memory limits of the staged kernels
 int mlp_tc_setup();                               // mlp.cu: shared-memory limit of the tcgen05 forward
-int launch_list_filter(Context* ctx, int parts);  // pair.cu  // after a sync; redo = 1: grown, repeat
+int launch_list_filter(Context* ctx, int parts);  // pair.cu
 // The fused kernels of a CG iteration: the sparse preconditioner with the
 // r.z / r.r sums and the CG scalars (pair.cu), and the mutual-field gather
 // with Ap = p/alpha - field, p.Ap and the step length (pme.cu).

@@ -98,7 +98,7 @@ extern "C" int t9gb_empole_energy(t9gb_context* h, double* energy, double* parts
    Context* ctx = &h->c;
    if (!ctx->have_order)
       return T9GB_NOT_READY;
-   for (int attempt = 0; attempt < 2; ++attempt) {
+   for (int attempt = 0; attempt < LIST_PASSES; ++attempt) {
       T9_CHECK(ensure_list(ctx, LIST_CUT));
       T9_CUDA(cudaMemsetAsync(ctx->e_atom, 0, sizeof(double) * 3 * ctx->npad, ctx->stream));
       T9_CHECK(launch_empole_real(ctx, ctx->e_atom));
@@ -246,7 +246,7 @@ static int elec_terms(Context* ctx, bool mpole, bool polar, int vers, double* en
          return rc;
    }
    bool beside_done = false;
-   for (int attempt = 0; attempt < 2; ++attempt) {
+   for (int attempt = 0; attempt < LIST_PASSES; ++attempt) {
       // a list refreshed here needs its capacity checked; one already checked
       // (after the solve above, or an earlier call) does not, and the gradient
       // then stays in stream order without a synchronisation

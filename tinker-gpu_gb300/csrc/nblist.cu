@@ -64,27 +64,25 @@ static double inner_cutoff(const Context* ctx)
 
 // Host: Morton order of the current coordinates, per-slot parameters, the
 // scaled-partner table and the neighbour-list storage.
-// the list and its two per-step sub-lists, all with row capacity cap
-int alloc_lists(Context* ctx, int cap)
+// The list (4 bytes an entry, 8 with the van der Waals term) and its two
+// per-step sub-lists with their factors (22 and 14 bytes), which hold what lies
+// within the real-space and the preconditioner cutoff alone: with the stored
+// rows' capacity they would take three to six times the memory.
+int alloc_lists(Context* ctx, int cap, int cut, int pre)
 {
-   for (int** p : {&ctx->nbr, &ctx->nbrc, &ctx->nbrp}) {
+   const auto fresh = [&](auto** p, int row) {
       cudaFree(*p);
       *p = nullptr;
-      T9_CUDA(cudaMalloc(p, sizeof(int) * (size_t)ctx->npad * cap));
-   }
-   cudaFree(ctx->nbre);
-   ctx->nbre = nullptr;
-   if (inner_cutoff(ctx) > 0)
-      T9_CUDA(cudaMalloc(&ctx->nbre, sizeof(int) * (size_t)ctx->npad * cap));
-   for (float2** p : {&ctx->cfu, &ctx->cfd, &ctx->cfp}) {
-      cudaFree(*p);
-      *p = nullptr;
-      T9_CUDA(cudaMalloc(p, sizeof(float2) * (size_t)ctx->npad * cap));
-   }
-   for (unsigned short** p : {&ctx->nbrc_l, &ctx->nbrp_l}) {
-      cudaFree(*p);
-      *p = nullptr;
-      T9_CUDA(cudaMalloc(p, sizeof(unsigned short) * (size_t)ctx->npad * cap));
+      return row == 0 || cudaMalloc(p, sizeof(**p) * (size_t)ctx->npad * row) == cudaSuccess;
+   };
+   const bool ok = fresh(&ctx->nbr, cap) && fresh(&ctx->nbre, inner_cutoff(ctx) > 0 ? cap : 0) &&
+      fresh(&ctx->nbrc, cut) && fresh(&ctx->cfu, cut) && fresh(&ctx->cfd, cut) && fresh(&ctx->nbrc_l, cut) &&
+      fresh(&ctx->nbrp, pre) && fresh(&ctx->cfp, pre) && fresh(&ctx->nbrp_l, pre);
+   if (!ok) {
+      ctx->last_error = "no memory for the neighbour list";
+      ctx->nbr_cap = ctx->cut_cap = ctx->pre_cap = 0;  // nothing is there to be used
+      ctx->have_order = false;
+      return T9GB_CUDA_ERR;
    }
    if (!ctx->jbl) {
       const int nblk = ctx->npad / 32;
@@ -94,7 +92,19 @@ int alloc_lists(Context* ctx, int cap)
       T9_CUDA(cudaMemset(ctx->jbn, 0x7f, sizeof(int) * (size_t)nblk));
    }
    ctx->nbr_cap = cap;
+   ctx->cut_cap = cut;
+   ctx->pre_cap = pre;
    return T9GB_OK;
+}
+
+// The first capacity of a sub-list of radius r: half as many again as the mean
+// density gives (that of the atoms' extent without a box, of which a round
+// droplet fills a half), whole tiles, and never more than a stored row.  A
+// denser spot overflows it and the list is grown.
+static int sublist_cap(const Context* ctx, double r, double volume, bool pbc, int cap)
+{
+   const double expect = ctx->n / volume * 4.18879020478639 * r * r * r * (pbc ? 1.5 : 3.0) + 32;
+   return expect >= cap ? cap : ((int)expect + 31) / 32 * 32;
 }
 
 int order_build(Context* ctx)
@@ -239,6 +249,9 @@ int order_build(Context* ctx)
    }
    cap = ((cap + 31) / 32) * 32;
    cap = std::max(cap, ctx->nbr_cap);
+   const double vol = len[0] * len[1] * len[2];
+   const int cut = std::max(ctx->cut_cap, sublist_cap(ctx, cfg.cutoff, vol, pbc, cap));
+   const int pre = std::max(ctx->pre_cap, sublist_cap(ctx, cfg.usolve_cutoff + cfg.pbuffer, vol, pbc, cap));
 
    cudaFree(ctx->perm);
    cudaFree(ctx->iperm);
@@ -283,8 +296,9 @@ int order_build(Context* ctx)
       T9_CUDA(cudaMalloc(&ctx->cell_count, sizeof(int) * ctx->ncell));
       T9_CUDA(cudaMalloc(&ctx->cell_start, sizeof(int) * (ctx->ncell + 1)));
    }
-   if (cap != ctx->nbr_cap || (inner_cutoff(ctx) > 0) != (ctx->nbre != nullptr))
-      T9_CHECK(alloc_lists(ctx, cap));
+   if (cap != ctx->nbr_cap || cut != ctx->cut_cap || pre != ctx->pre_cap ||
+      (inner_cutoff(ctx) > 0) != (ctx->nbre != nullptr))
+      T9_CHECK(alloc_lists(ctx, cap, cut, pre));
    // legacy-stream copies above finish before the stream's kernels
    T9_CUDA(cudaDeviceSynchronize());
    T9_CHECK(fill_row_padding(ctx));

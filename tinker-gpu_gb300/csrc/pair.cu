@@ -771,6 +771,8 @@ static constexpr int PAIR_THREADS = 256;
 // the staged kernels find the row in shared memory.
 struct FilterOut {
    int lanes_log2;  // of the tiled layout (ListView)
+   int cut_cap, pre_cap;  // row capacities
+   int* over;       // [LIST_CAPS] largest rows beyond them
    int *nbrc, *nnbrc, *nbrp, *nnbrp;
    float2* cu;  // mutual field
    float2* cd;  // permanent field (b2, b3)
@@ -869,7 +871,7 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : PARTS == LIST_
    }
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    const int i = blk * NW + warp;
-   const ListView V{nullptr, P.cap, O.lanes_log2};
+   const ListView VC{nullptr, O.cut_cap, O.lanes_log2}, VP{nullptr, O.pre_cap, O.lanes_log2};
    int oc = 0, op = 0;
    if (i < P.n) {
       const float4 pi = spos[i];
@@ -879,12 +881,12 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : PARTS == LIST_
       const float rmax2 = CUT && PRE ? fmaxf(P.cut2, cutp2) : CUT ? P.cut2 : cutp2;
       const unsigned lt = (1u << lane) - 1u;
       // the row's place in the tiled lists, and an entry's from it
-      const size_t base = V.at(i, 0);
+      const size_t base = VC.at(i, 0), basep = VP.at(i, 0);
       int* nc = O.nbrc + base;
       float2* cu = O.cu + base;
       float2* cd = O.cd + base;
-      int* np = O.nbrp + base;
-      float2* cp = O.cp + base;
+      int* np = O.nbrp + basep;
+      float2* cp = O.cp + basep;
       const int sg = O.lanes_log2, gm = (1 << sg) - 1;
       int qn = 0;
       // the first m (<= 32) queued entries into the sub-lists
@@ -900,16 +902,20 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : PARTS == LIST_
          pair_factors(P, r2, 1.f, pi.w, dk.w, pair_gamma(P, ti.x, tk.x), ti.y * tk.y, u, f, c);
          if (inc) {
             const unsigned k = oc + __popc(mc & lt), at = ((k >> sg) << 5) + (k & gm);
-            nc[at] = j;
-            if (FIELD) {
-               cu[at] = u;
-               cd[at] = f;
+            if (k < (unsigned)O.cut_cap) {
+               nc[at] = j;
+               if (FIELD) {
+                  cu[at] = u;
+                  cd[at] = f;
+               }
             }
          }
          if (inp) {
             const unsigned k = op + __popc(mp & lt), at = ((k >> sg) << 5) + (k & gm);
-            np[at] = j;
-            cp[at] = c;
+            if (k < (unsigned)O.pre_cap) {
+               np[at] = j;
+               cp[at] = c;
+            }
          }
          if (STAGE && (inc || inp))
             atomicOr(&bm[j >> 10], 1u << ((j >> 5) & 31));
@@ -926,7 +932,7 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : PARTS == LIST_
          const unsigned m = __ballot_sync(0xffffffffu, acc);
          if (PARTS == LIST_CUT) {  // indices alone: nothing to queue for
             const unsigned k = oc + __popc(m & lt);
-            if (acc)
+            if (acc && k < (unsigned)O.cut_cap)
                nc[((k >> sg) << 5) + (k & gm)] = j;
             oc += __popc(m);
             j = jn;
@@ -954,6 +960,12 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : PARTS == LIST_
       if (qn > 0)
          drain(qn);
    }
+   if (lane == 0 && CUT && oc > O.cut_cap)
+      atomicMax(O.over + 1, oc);
+   if (lane == 0 && PRE && op > O.pre_cap)
+      atomicMax(O.over + 2, op);
+   oc = min(oc, O.cut_cap);
+   op = min(op, O.pre_cap);
    if (lane == 0) {
       if (CUT)
          O.nnbrc[i] = oc;
@@ -1000,15 +1012,15 @@ __global__ void __launch_bounds__(STAGE ? 1024 : 256, STAGE ? 1 : PARTS == LIST_
       }
    }
    if (i < P.n) {
-      unsigned short* lc = O.nbrc_l + (size_t)i * P.cap;
-      unsigned short* lp = O.nbrp_l + (size_t)i * P.cap;
+      unsigned short* lc = O.nbrc_l + (size_t)i * O.cut_cap;
+      unsigned short* lp = O.nbrp_l + (size_t)i * O.pre_cap;
       for (int k = lane; k < oc; k += 32) {
-         const int j = O.nbrc[V.at(i, k)], jb = j >> 5;
+         const int j = O.nbrc[VC.at(i, k)], jb = j >> 5;
          const int q = pre[jb >> 5] + __popc(bm[jb >> 5] & ((1u << (jb & 31)) - 1u));
          lc[k] = (unsigned short)(q * 32 + (j & 31));
       }
       for (int k = lane; k < op; k += 32) {
-         const int j = O.nbrp[V.at(i, k)], jb = j >> 5;
+         const int j = O.nbrp[VP.at(i, k)], jb = j >> 5;
          const int q = pre[jb >> 5] + __popc(bm[jb >> 5] & ((1u << (jb & 31)) - 1u));
          lp[k] = (unsigned short)(q * 32 + (j & 31));
       }
@@ -1027,7 +1039,7 @@ int launch_list_filter(Context* ctx, int parts)
    const int* nbr = ctx->nbre ? ctx->nbre : ctx->nbr;
    const int* nnbr = ctx->nbre ? ctx->nnbre : ctx->nnbr;
    ctx->list_lanes = ctx->pair_lanes;
-   FilterOut O{nbrc_view(ctx).sg, ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp, ctx->cfu, ctx->cfd, ctx->cfp, ctx->spu,
+   FilterOut O{nbrc_view(ctx).sg, ctx->cut_cap, ctx->pre_cap, ctx->nbr_over, ctx->nbrc, ctx->nnbrc, ctx->nbrp, ctx->nnbrp, ctx->cfu, ctx->cfd, ctx->cfp, ctx->spu,
       ctx->spp, ctx->jbl, ctx->jbn, ctx->nbrc_l, ctx->nbrp_l};
    if (ctx->pair_staged)
       k_list_filter<true, LIST_ALL><<<nblk + grid_for(ctx->nsp, 1024), 1024, smem, ctx->stream>>>(P, cutp2, ctx->npad,
@@ -1107,9 +1119,25 @@ int pair_staging_setup()
    return T9GB_OK;
 }
 
-int launch_ufield_real(Context* ctx, const float* u6, const float* base6, float* out6)
+// parameters of the kernels over the two sub-lists (cap: their row capacity)
+static PairParams field_params(const Context* ctx)
 {
    PairParams P = make_params(ctx, ctx->cfg.cutoff);
+   P.cap = ctx->cut_cap;
+   return P;
+}
+
+static PairParams precond_params(const Context* ctx)
+{
+   PairParams P = make_params(ctx, ctx->cfg.usolve_cutoff + ctx->cfg.pbuffer);
+   P.ewald = 0;
+   P.cap = ctx->pre_cap;
+   return P;
+}
+
+int launch_ufield_real(Context* ctx, const float* u6, const float* base6, float* out6)
+{
+   PairParams P = field_params(ctx);
    prof_begin(ctx, P_UFIELD_REAL);
    if (staged_lanes(ctx)) {
       auto k = ctx->pair_lanes == 8 ? k_ufield_stg<8> : k_ufield_stg<4>;
@@ -1135,7 +1163,7 @@ int launch_ufield_real(Context* ctx, const float* u6, const float* base6, float*
 
 int launch_ufield_real_dir(Context* ctx, const float* p6, const float* z6, const double* scal, float* out6)
 {
-   PairParams P = make_params(ctx, ctx->cfg.cutoff);
+   PairParams P = field_params(ctx);
    prof_begin(ctx, P_UFIELD_REAL);
    T9_LANES_DISPATCH2(k_ufield_real, true, P, ctx->npad, field_list(ctx), partners(ctx), ctx->spos, p6, z6, scal,
       nullptr, out6);
@@ -1146,7 +1174,7 @@ int launch_ufield_real_dir(Context* ctx, const float* p6, const float* z6, const
 
 int launch_dfield_real(Context* ctx, const float* base6, float* out6)
 {
-   PairParams P = make_params(ctx, ctx->cfg.cutoff);
+   PairParams P = field_params(ctx);
    prof_begin(ctx, P_DFIELD_REAL);
    T9_LANES_DISPATCH(k_dfield_real, P, ctx->npad, field_list(ctx), ctx->cfd, ctx->sp_start, ctx->sp_j, ctx->sp_sc, ctx->spos,
       ctx->srpole, base6, ctx->exfld, out6);
@@ -1157,8 +1185,7 @@ int launch_dfield_real(Context* ctx, const float* base6, float* out6)
 
 int launch_precond_sparse_dots(Context* ctx, const float* r6, float* z6, const PcgDots& D)
 {
-   PairParams P = make_params(ctx, ctx->cfg.usolve_cutoff + ctx->cfg.pbuffer);
-   P.ewald = 0;
+   PairParams P = precond_params(ctx);
    const int g = ctx->pair_lanes;
    const int per = PAIR_THREADS / g;
    const int nb = std::min(RED_MAX, (ctx->npad + per - 1) / per);
@@ -1187,8 +1214,7 @@ int launch_precond_sparse_dots(Context* ctx, const float* r6, float* z6, const P
 
 int launch_precond_sparse(Context* ctx, const float* r6, float* z6)
 {
-   PairParams P = make_params(ctx, ctx->cfg.usolve_cutoff + ctx->cfg.pbuffer);
-   P.ewald = 0;
+   PairParams P = precond_params(ctx);
    prof_begin(ctx, P_PRECOND);
    T9_LANES_DISPATCH(k_precond_sparse, P, ctx->npad, (float)ctx->cfg.udiag, precond_list(ctx), partners(ctx),
       ctx->spos, r6, z6);

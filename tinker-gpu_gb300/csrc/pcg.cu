@@ -428,8 +428,8 @@ __global__ void k_finish(int* state, int depth, const double* __restrict__ scal,
    }
    if (t < S_NSCAL)
       h_scal[t] = scal[t];
-   if (t == 0)
-      *h_over = *over;
+   if (t < LIST_CAPS)
+      h_over[t] = over[t];
 }
 
 // ---------------------------------------------------------------------------
@@ -793,7 +793,7 @@ int ensure_list(Context* ctx, int need)
    }
    if (parts)
       T9_CHECK(launch_list_filter(ctx, parts));
-   T9_CUDA(cudaMemcpyAsync(ctx->h_over, ctx->nbr_over, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+   T9_CUDA(cudaMemcpyAsync(ctx->h_over, ctx->nbr_over, sizeof(int) * LIST_CAPS, cudaMemcpyDeviceToHost, ctx->stream));
    ctx->list_stale = false;
    return T9GB_OK;
 }
@@ -837,17 +837,26 @@ static int list_refresh_graph(Context* ctx)
    return launch_list_filter(ctx, LIST_ALL);
 }
 
-// after a synchronisation: grow the list if an atom had more neighbours than
-// the row capacity; *redo = 1 when the caller must repeat its work
+// after a synchronisation: grow a list if an atom had more neighbours than
+// its row capacity; *redo = 1 when the caller must repeat its work.  The
+// sub-lists grow with the stored rows, whose overflow cut them short.
 int check_list_overflow(Context* ctx, int* redo)
 {
    *redo = 0;
-   if (*ctx->h_over <= ctx->nbr_cap)
+   const int* over = ctx->h_over;
+   if (over[0] <= ctx->nbr_cap && over[1] <= ctx->cut_cap && over[2] <= ctx->pre_cap)
       return T9GB_OK;
-   int cap = ((int)(*ctx->h_over * 1.25) + 31) / 32 * 32;
-   T9_CHECK(alloc_lists(ctx, cap));
-   *ctx->h_over = 0;
-   T9_CUDA(cudaMemsetAsync(ctx->nbr_over, 0, sizeof(int), ctx->stream));
+   const auto grown = [](int cap, int most) {
+      return most > cap ? ((int)(most * 1.25) + 31) / 32 * 32 : cap;
+   };
+   const int cap = grown(ctx->nbr_cap, over[0]);
+   const auto sub = [&](int c, int most) {
+      const int with = (int)(((long long)c * cap / ctx->nbr_cap + 31) / 32 * 32);
+      return std::min(cap, std::max(with, grown(c, most)));
+   };
+   T9_CHECK(alloc_lists(ctx, cap, sub(ctx->cut_cap, over[1]), sub(ctx->pre_cap, over[2])));
+   std::fill(ctx->h_over, ctx->h_over + LIST_CAPS, 0);
+   T9_CUDA(cudaMemsetAsync(ctx->nbr_over, 0, sizeof(int) * LIST_CAPS, ctx->stream));
    ctx->list_need_build = true;
    drop_graphs(ctx);
    *redo = 1;
@@ -1330,7 +1339,7 @@ int induce_sorted(Context* ctx)
    bool range_failed = false;
    ctx->induce_redone = false;
    T9_CHECK(lx_wait(ctx));
-   for (int attempt = 0; attempt < 3; ++attempt) {
+   for (int attempt = 0; attempt < LIST_PASSES; ++attempt) {
       if (attempt > 0)
          ctx->induce_redone = true;
       T9_CHECK(graph ? induce_graph(ctx, variant) : induce_stepwise(ctx, variant));
@@ -1487,7 +1496,7 @@ int reset_predictor(Context* ctx)
 template <class F>
 static int with_list(Context* ctx, int need, F&& body)
 {
-   for (int attempt = 0; attempt < 3; ++attempt) {
+   for (int attempt = 0; attempt < LIST_PASSES; ++attempt) {
       T9_CHECK(ensure_list(ctx, need));
       T9_CHECK(body());
       T9_CUDA(cudaStreamSynchronize(ctx->stream));

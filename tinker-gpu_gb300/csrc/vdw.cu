@@ -414,7 +414,7 @@ extern "C" int t9gb_ehal(t9gb_context* h, int vers, double* energy, float* grad,
    }
    const bool vir = (vers & T9GB_CALC_VIRIAL) != 0;
    T9_CHECK(force_setup(ctx));
-   for (int attempt = 0; attempt < 2; ++attempt) {
+   for (int attempt = 0; attempt < LIST_PASSES; ++attempt) {
       T9_CHECK(ensure_list(ctx, 0));  // the stored rows
       T9_CUDA(cudaMemsetAsync(ctx->e_atom, 0, sizeof(double) * 3 * ctx->npad, ctx->stream));
       T9_CHECK(vdw_forces(ctx, (vers & T9GB_CALC_GRAD) ? grad : nullptr, false, vir, nullptr));
