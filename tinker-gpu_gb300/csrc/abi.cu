@@ -424,15 +424,31 @@ int t9gb_set_xyz_host(t9gb_context* h, const double* xyz)
    return T9GB_OK;
 }
 
+// a kernel on this GPU may read p as floats
+static bool kernel_readable(const Context* ctx, const float* p)
+{
+   cudaPointerAttributes a = {};
+   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+   }
+   return a.type == cudaMemoryTypeDevice && a.device == ctx->dev && (uintptr_t)p % alignof(float) == 0;
+}
+
 int t9gb_set_xyz_device(t9gb_context* h, const float* xyz_device)
 {
    if (!h || !xyz_device)
       return T9GB_BAD_ARG;
    Context* ctx = &h->c;
+   // the scatter reads and copies memory of this GPU itself; for any other
+   // pointer the copy decides whether it is one, with an error where a kernel
+   // would fault
+   const bool direct = ctx->have_order && kernel_readable(ctx, xyz_device);
+   if (!direct)
+      T9_CUDA(cudaMemcpyAsync(ctx->xyz, xyz_device, sizeof(float) * 3 * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
    ctx->have_xyz = true;
    if (ctx->have_order)
-      return scatter_positions(ctx, xyz_device);
-   T9_CUDA(cudaMemcpyAsync(ctx->xyz, xyz_device, sizeof(float) * 3 * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
+      T9_CHECK(scatter_positions(ctx, direct ? xyz_device : nullptr));
    return T9GB_OK;
 }
 
