@@ -66,8 +66,8 @@ def parse():
     ap.add_argument("--no-large", action="store_true", help="skip the 98,304-atom leg")
     ap.add_argument("--large-config", default="water98304")
     ap.add_argument("--fft", choices=["auto", "own", "cufft"], default="auto",
-                    help="PME transform: the library's default (its fused transform on cubic 32/64 grids, cuFFT "
-                    "otherwise), the fused transform, or cuFFT")
+                    help="PME transform: the library's default (one cluster on small cubic grids, its fused transform "
+                    "on 64^3, cuFFT otherwise), the fused transform, or cuFFT")
     ap.add_argument("--lanes", type=int, default=0,
                     help="lanes per atom in the real-space field kernels (0: the library's choice by box size)")
     ap.add_argument("--no-flush", action="store_true",
@@ -156,17 +156,23 @@ def measured_peaks():
 
 
 # Algorithmic (compulsory) bytes per launch of each kernel: every input read
-# once, every output written once.  "entries" = neighbour-list entries.
+# once, every output written once.  "entries" = entries of the stored neighbour
+# list, within the cutoff and its buffer (9 A); the kernels read the
+# sub-lists within the cutoff (7 A) and the preconditioner's (6.5 A), whose
+# sizes follow at the boxes' uniform density, 4 bytes an index and 8 (the
+# permanent field 16) for the pair's stored factors.
 def algorithmic_bytes(kernel, n, entries, nfft):
     ng = nfft ** 3
+    in_cut, in_precond = int(entries * (7.0 / 9.0) ** 3), int(entries * (6.5 / 9.0) ** 3)
     if kernel == "ufield_real":
-        # pos 16 + dipoles 24 + damping 8 + recip field 24 in, field 24 out, list 4/entry
-        return n * (16 + 24 + 8 + 24 + 24) + 4 * entries
+        # pos 16 + dipoles 24 + recip field 24 in, field 24 out
+        return n * (16 + 24 + 24 + 24) + 12 * in_cut
     if kernel == "dfield_real":
-        # pos 16 + multipoles 40 + damping 8 + recip field 24 in, field 24 out
-        return n * (16 + 40 + 8 + 24 + 24) + 4 * entries
+        # pos 16 + multipoles 40 + recip field 24 in, field 24 out
+        return n * (16 + 40 + 24 + 24) + 20 * in_cut
     if kernel == "precond_sparse":
-        return n * (16 + 24 + 8 + 4 + 24) + 4 * entries
+        # pos 16 + residual 24 + polarizability 4 in, z 24 out
+        return n * (16 + 24 + 4 + 24) + 12 * in_precond
     if kernel == "spread_uind":
         # pos + dipoles in, fixed-point grid (one 8-byte word per point: d and p packed) written once
         return n * (16 + 24) + 8 * ng
@@ -832,9 +838,10 @@ def main():
             "config": {
                 "workload": args.config, "atoms": s.n, "pme_grid": list(s.settings["nfft"]), "cutoff_A": 7.0,
                 "poleps_debye": s.settings["poleps"], "predictor": args.predictor, "history_frames": args.history,
-                "fft": {"auto": "library default: fused transform on cubic 32/64 grids, cuFFT C2C otherwise",
+                "fft": {"auto": "library default: one cluster on cubic grids of 16 to 40, the fused transform on 64^3, "
+                                "cuFFT C2C otherwise",
                         "own": "fused power-of-two transform (library)", "cufft": "cuFFT C2C"}[args.fft],
-                "lanes_per_atom": args.lanes or "library default (8 up to 32,768 atoms, 4 above)",
+                "lanes_per_atom": args.lanes or "library default (16 up to 768 atoms, 8 up to 32,768, 4 above)",
                 "l2": "not flushed (profiling run)" if args.no_flush else "flushed (512 MB write) between timed steps",
                 "parallelism": f"replicas x{world}",
             },

@@ -400,7 +400,7 @@ int t9gb_force_lanes(t9gb_context* ctx, int lanes);
  * Bit 6 (with bit 5): that chain stays on the main stream behind the
  * direction kernel and the real-space field runs on the side stream; up to
  * 4,096 atoms the spread then forms and stores the direction and the kernel
- * falls away (648 atoms 0.420 -> 0.412 ms a solve, 6,300 0.342 -> 0.350).  Bits
+ * falls away (648 atoms 0.264 -> 0.258 ms a solve, 8,232 0.531 -> 0.543).  Bits
  * 5-6 give the same bits as without them; GB300 (induce ms, 12,288 /
  * 98,304 atoms): mask 25 0.4925 / 2.344, 57 0.4829 / 2.297, 121 (the
  * default) 0.473 / 2.285.  A tuning knob: the same iteration, results equal

@@ -189,10 +189,10 @@ const char* t9gb_status_string(int status)
 const char* t9gb_last_error(const t9gb_context* h) { return h ? h->c.last_error.c_str() : "null context"; }
 
 // Lanes per atom of the field kernels: 8 on small boxes, 4 where the box
-// fills the GPU (GB300 induce: 12,288 atoms 0.573 / 0.631 ms at 8 / 4 lanes;
-// 98,304 atoms 2.588 / 2.514 ms), 16 where even their eight lanes leave most of
-// it idle (648 atoms 0.320 / 0.301 ms at 8 / 16 lanes, 1,029 atoms 0.332 /
-// 0.343).  8 there too while the learned guess trains: its weights follow
+// fills the GPU (GB300, a solve from alpha E at 4 / 8 / 16 lanes: 12,288 atoms
+// 0.709 / 0.665 / 0.728 ms, 24,000 1.028 / 1.051 / 1.090, 98,304 2.681 / 2.772 /
+// 2.985), 16 where even eight lanes leave most of it idle (648 atoms 0.330 / 0.274
+// / 0.264, 768 0.309 / 0.284 / 0.295, 1,536 0.350 / 0.295 / 0.309).  8 there too while the learned guess trains: its weights follow
 // the order of the fields' sums (fft_conv).
 static int default_pair_lanes(const Context* ctx)
 {
@@ -227,10 +227,11 @@ int t9gb_create(const t9gb_config* cfg, t9gb_context** out)
    ctx->npad = ((cfg->n + WARP - 1) / WARP) * WARP;
    ctx->pair_lanes = default_pair_lanes(ctx);
    // lanes of the real-space force kernel, whose rows are a serial chain of
-   // long pair terms on a small box (10 MD steps at 4 / 8 / 16 lanes: 648
-   // atoms 3.44 / 3.12 / 3.04 ms, 1,200 3.17 / 3.06 / 3.01, 2,187 4.12 / 4.00
-   // / 3.78, 2,550 4.24 / 3.89 / 4.00, 3,000 4.49 / 4.28 / 4.41, 3,993 4.86 /
-   // 4.81 / 4.83)
+   // long pair terms on a small box (GB300, 10 MD steps from the lattice with
+   // no predictor at 4 / 8 / 16 lanes: 648 atoms 3.34 / 3.16 / 3.07 ms, 1,536 3.83 /
+   // 3.71 / 3.69, 2,187 4.40 / 4.18 / 4.09, 2,550 4.72 / 4.60 / 4.56, 3,000 5.02 /
+   // 4.82 / 4.80, 3,072 5.03 / 5.04 / 5.16, 3,993 5.63 / 5.58 / 5.55: beyond
+   // 3,072 atoms the three are within 2 %)
    ctx->force_lanes = ctx->npad > 3072 ? 4 : (ctx->npad > 2304 ? 8 : 16);
    cudaGetDevice(&ctx->dev);
    int rc = T9GB_OK;

@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(3 * SCATTER_SLOTS) k_scatter_pos(int npad, con
    float4* __restrict__ spos, SplineParams S)
 {
    // the tables leave through shared memory: each thread's 10 words of a row
-   // would be written eight bytes at a time (21 -> 9 us at 98,304 atoms)
+   // would be written eight bytes at a time (21 -> 10 us at 98,304 atoms)
    __shared__ float4 lo[SCATTER_SLOTS * SPL_ROW / 4], hi[SCATTER_SLOTS * SPL_ROW / 4];
    const int q = threadIdx.x / 3, d = threadIdx.x - 3 * q, s0 = blockIdx.x * SCATTER_SLOTS, s = s0 + q;
    const int a = s < npad ? perm[s] : -1;

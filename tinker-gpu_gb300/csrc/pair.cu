@@ -96,11 +96,12 @@ __device__ __forceinline__ void for_own6(float* f, F&& fn)
 // the transcendental chain).  The sub-lists and factors are stored by tiles of
 // 32 / G atoms (ListView), so that a warp's index load is one 128-byte line
 // and its factor load two; the neighbour's row is one 32-byte load.  What
-// bounds the rows is the L1's rate of one line per cycle (83% of it at 98,304
-// atoms, 4 lanes: 1 + 2 + 11 + 14 lines for 32 pairs, 47 before).  GB300, ncu,
-// 12,288 / 98,304 atoms: mutual field 20.6 -> 16.0 / 97 -> 76 us,
-// preconditioner 20.5 -> 15.8 / 82 -> 63, permanent field 26.3 -> 18.9 /
-// 120 -> 94, filter 23 -> 33 / 118 -> 211 (once per position update).
+// bounds the rows is the L1's rate of one line per cycle (1 + 2 + 11 + 14 lines
+// for 32 pairs, 47 before; from cold caches ncu has the L1 at 68 and 75 % for
+// the mutual field and the preconditioner of 98,304 atoms, 4 lanes).  GB300,
+// ncu, 12,288 / 98,304 atoms: mutual field 20.6 -> 16.2 / 97 -> 77 us,
+// preconditioner 20.5 -> 16.0 / 82 -> 63, permanent field 26.3 -> 19.1 /
+// 120 -> 96, filter 23 -> 31 / 118 -> 205 (once per position update).
 
 // a sub-list with its factors, tiled (ListView) for the kernels' lane count:
 // counts per slot, indices, factors, and the factors of the scaled partners
@@ -1057,10 +1058,10 @@ int launch_list_filter(Context* ctx, int parts)
 
 // Where the grid leaves an SM at most one block, a row's trips wait on their
 // own latency, not on the L1's line rate: four entries a trip (80-106
-// registers).  GB300, induce: droplet of 1,500 atoms (rows of 1,499) 749 ->
-// 660 us; periodic boxes of 648 and 3,000 atoms the same either way (10 MD
-// steps of 648 atoms at 16 lanes 3.10 -> 3.05 ms); at 12,288 atoms two entries
-// are better (414 against 436 us).
+// registers).  GB300, a solve from alpha E: droplets of 648 / 1,500 / 2,100 atoms
+// (rows of all atoms) 319 / 702 / 1,212 -> 297 / 623 / 863 us; periodic boxes of
+// 648 to 3,072 atoms the same either way; at 12,288 atoms two entries are better
+// (670 against 722).
 static bool few_blocks(int nb) { return nb <= 152; }
 
 static TensorList field_list(const Context* ctx) { return {ctx->nbrc, ctx->nnbrc, ctx->cfu, ctx->spu}; }

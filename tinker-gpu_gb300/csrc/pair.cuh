@@ -1,6 +1,5 @@
-// Shared pieces of the real-space pair kernels (pair.cu, force.cu): pair
-// parameters, minimum-image separation, fixed xor-tree group reductions and
-// the 32-byte row load.
+// Shared pieces of the real-space pair kernels (pair.cu, force.cu, vdw.cu): pair
+// parameters, minimum-image separation and fixed xor-tree group reductions.
 #pragma once
 #include "common.cuh"
 
@@ -14,7 +13,7 @@ struct PairParams {
    int ewald;
    float aewald;
    float ec1, ec2, ec3, ec4;  // (2a^2)^j / (sqrt(pi) a), j = 1..4
-   int cap;              // list row stride
+   int cap;              // row capacity of the list that the kernel walks
    const float* thl;     // per-type-pair Thole table [nthl][nthl], or null
    int nthl;
 };

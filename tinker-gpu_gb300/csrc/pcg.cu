@@ -26,10 +26,12 @@
 namespace t9gb {
 
 constexpr int VB = 256;  // vector-kernel block size
-// boxes up to this size form the CG direction in the spread: a launch less in
-// an iteration, the real-space field a spread later (GB300, induce, 648 /
-// 3,000 / 6,300 / 12,288 atoms: 412 / 293 / 350 / 408 us, with a kernel of its
-// own 420 / 297 / 342 / 400)
+// Boxes up to this size form the CG direction in the spread: a launch less in
+// an iteration, the real-space field a spread later.  GB300, a solve from alpha
+// E with coordinates on the device, 648 / 1,536 / 3,993 / 5,184 / 8,232 / 12,288
+// atoms: 258 / 294 / 444 / 469 / 543 / 679 us, with a kernel of its own
+// 264 / 302 / 457 / 498 / 531 / 670.  The gain has gone at 8,232; the line is on
+// its near side.
 constexpr int DIR_SPREAD_MAX = 4096;
 
 // ASPC extrapolation weights (Kolafa, J. Comput. Chem. 25, 335 (2004)); the
@@ -269,9 +271,11 @@ __global__ void k_pcg_p2(VecArgs A, const double* __restrict__ scal, float* __re
 // their partial p.Ap through distributed shared memory, keeps Ap in registers
 // between them.  What bounds it is latency, one trip to memory and one
 // cluster barrier; k_pcg_p1 needs a round of atomics and a second read of the
-// partials by its last block, and k_pcg_p2 a launch.  GB300, a solve of 648 /
-// 1,500 / 2,187 / 3,000 atoms: 300 / 339 / 400 / 437 -> 277 / 321 / 384 / 424
-// us.  The line lies where a thread holds five elements.  The sum is
+// partials by its last block, and k_pcg_p2 a launch.  GB300, a solve from alpha
+// E of 648 / 1,029 / 1,536 / 3,000 atoms: 278 / 308 / 336 / 403 -> 258 / 294 /
+// 294 / 403 us.  The line lies where a thread holds five elements and the gain
+// ends: with nine, 3,993 atoms take 444 instead of 447, 5,184 501 instead of
+// 491.  The sum is
 // k_pcg_p1's up to the order of its FP64 additions: the products of 32
 // consecutive elements in FP32, everything above them in FP64.
 constexpr int STEP_CL = 8, STEP_THREADS = 512;

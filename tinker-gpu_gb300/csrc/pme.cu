@@ -1061,11 +1061,11 @@ static void fft_own_inverse(const PmeGrid& P, cudaStream_t st, bool split, bool 
 // 110 of them; at 40^3 it moves 64 KB and the shared memory bounds it), two
 // cluster barriers and one trip to global memory each way.  It takes the
 // place of eight launches of a few microseconds (cuFFT's six, conversion,
-// convolution): an induce solve of 648 atoms on 16 / 20 / 24 / 30 / 36 / 40
-// points an edge takes 288 / 283 / 287 / 302 / 331 / 345 us instead of
-// 382 / 401 / 396 / 405 / 395 / 405, and on 32 points 302 instead of the 316
-// of the plane kernels.  With 8 CTAs it is 294 / 332 / 383 us at 24 / 30 /
-// 40; 256 threads take 289 / 317 / 378.  Edges are known at compile time:
+// convolution): a solve of 648 atoms from alpha E on 16 / 18 / 20 / 24 / 30 /
+// 36 / 40 points an edge takes 247 / 273 / 254 / 262 / 272 / 299 / 337 us instead
+// of 350 / 357 / 362 / 356 / 375 / 360 / 371, and on 32 points 268 instead of the
+// 282 of the plane kernels.  8 CTAs take 7 / 30 / 38 us more than 16 at 24 / 30 /
+// 40, 256 threads 2 / 15 / 33 more than 512.  Edges are known at compile time:
 // the same steps with factors and strides from a table took 17.7 us a
 // transform at 24^3 instead of 7.3.
 constexpr int SG_CL = 16;       // CTAs, the largest cluster

@@ -50,8 +50,8 @@ __device__ __forceinline__ void bspline5(float w, float th[5][LEVEL])
 }
 
 // Rows of the tables, 32 floats (128 bytes) per slot: point j of axis a at
-// [10 a + 2 j]: value and first derivative in SplineTable::lo, second and
-// third derivative in SplineTable::hi (entries 30 and 31 unused).
+// [10 a + 2 j]: value and first derivative in PmeGrid::spl_lo, second and
+// third derivative in PmeGrid::spl_hi (entries 30 and 31 unused).
 constexpr int SPL_ROW = 32;
 
 __device__ __forceinline__ float2 spl(const float* row, int axis, int j)
