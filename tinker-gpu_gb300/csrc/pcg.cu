@@ -1036,7 +1036,7 @@ static int pcg_body(Context* ctx, const VecArgs& A, cudaGraphConditionalHandle h
       } else {
          T9_CHECK(ufield6(ctx, ctx->conj, ctx->fld6));
       }
-      if (ctx->npad <= STEP_MAX && !(ctx->learn_mode & 1)) {  // training: as for the small transform (fft_conv)
+      if (ctx->npad <= STEP_MAX) {
          prof_begin(ctx, P_VECTOR);
          T9_CHECK(launch_pcg_step(ctx, A, rcp));
          prof_end(ctx);
