@@ -181,7 +181,9 @@ int t9gb_md_positions_device(t9gb_context* ctx, float* xyz_device);
 /* Steps integrated and PCG iterations spent in them since t9gb_md_init. */
 int t9gb_md_stats(t9gb_context* ctx, long long* steps, long long* pcg_iterations);
 
-/* Coordinates [n][3].  Replace copyPosToXyz (src/atom.cpp:161-166). */
+/* Coordinates [n][3].  Replace copyPosToXyz (src/atom.cpp:161-166).
+ * xyz_device: memory of the context's GPU, which is read where it is, in
+ * stream order; any other pointer is copied first, as device to device. */
 int t9gb_set_xyz_host(t9gb_context* ctx, const double* xyz);
 int t9gb_set_xyz_device(t9gb_context* ctx, const float* xyz_device);
 
@@ -414,7 +416,12 @@ int t9gb_set_pcg_fusion(t9gb_context* ctx, int mask);
 
 /* Neighbour-list sizes: row capacity, entries of the current list (both
  * directions) and scaled pairs (the reference's Spatial::nakpl/niak,
- * include/ff/spatial.h:15-140). */
+ * include/ff/spatial.h:15-140).  The rows stored take 4 bytes an entry of the
+ * capacity and atom (8 with the van der Waals term); the per-step sub-lists
+ * within the cutoff and the preconditioner's have shorter rows of 22 and 14
+ * bytes an entry.  Every capacity starts from the mean density and grows
+ * where a row needs more.  Without a cutoff (at most 16,384 atoms) rows hold
+ * every atom, 26 n^2 bytes in all. */
 int t9gb_nblist_stats(t9gb_context* ctx, int* capacity, long long* entries, int* nscaled);
 
 /* Mutual field without any allocation.  No counterpart in the reference: it
